@@ -4,11 +4,11 @@
 namespace dv {
 
 int decode_fwd_v64c32(const DecodeArgs& a, cudaStream_t st, int sms) {
-  return launch_decode_fwd<32, 64, 1, 128>(a, st, sms);
+  return launch_decode_fwd<32, 64, 1, 32, 16, 1>(a, st, sms);
 }
 
 int decode_bwd_v64c32(const DecodeArgs& a, cudaStream_t st, int sms) {
-  return launch_decode_bwd<32, 64, 1, 64>(a, st, sms);
+  return launch_decode_bwd<32, 64, 1, 16, true>(a, st, sms);
 }
 
 }  // namespace dv

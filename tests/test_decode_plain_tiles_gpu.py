@@ -1,0 +1,64 @@
+"""GPU: the plain FP32 decoder, forward and backward, at the edges of its
+16- and 32-segment warp tiles and of the backward's 128-segment steps, with
+rays that end inside tiles and segments on the grid's far faces, against the
+FP64 oracle.  Tolerances: forward 1e-5 abs, gradients 1e-4 relative L2, the
+plain form's stated ones."""
+import pytest
+import torch
+
+from oracle import torch_ref
+
+pytestmark = pytest.mark.gpu
+SIZES = [1, 15, 16, 17, 31, 32, 33, 127, 128, 129, 1000]
+
+
+def case(n, channels, kind, seed):
+    from diver_gb300.decoder import random_decoder
+
+    g = torch.Generator().manual_seed(seed)
+    dims = torch.tensor([9, 7, 5])
+    vox = torch.randn(6, 8, 10, channels, generator=g) * 0.3
+    # a walk through face-adjacent cells with jumps, some cells at the far faces
+    cell = (torch.rand(n, 3, generator=g) * dims).long()
+    for i in range(1, n):
+        if torch.rand((), generator=g) < 0.7:
+            step = torch.zeros(3, dtype=torch.long)
+            step[int(torch.randint(0, 3, (1,), generator=g))] = 1 if torch.rand((), generator=g) < 0.5 else -1
+            cell[i] = torch.minimum((cell[i - 1] + step).clamp_min(0), dims - 1)
+    p = cell[:, None, :] + 0.01 + 0.98 * torch.rand(n, 2, 3, generator=g)
+    ray = torch.cumsum((torch.rand(n, generator=g) < 0.1).long(), 0)
+    ray = (ray - ray[0]).int()
+    dirs = torch.randn(int(ray[-1]) + 1, 3, generator=g)
+    dirs = dirs / dirs.norm(dim=-1, keepdim=True)
+    return vox, p.reshape(n, 6).float(), ray, dirs, random_decoder(kind, channels, seed), torch.randn(n, 4, generator=g)
+
+
+@pytest.mark.parametrize("kind,channels", [("diver32", 32), ("diver64", 32), ("diver64", 64)])
+@pytest.mark.parametrize("n", SIZES)
+def test_plain_decoder_tile_edges(kind, channels, n):
+    from diver_gb300 import _native as N
+    from diver_gb300.decoder import pack_plain, unpack_plain_grad
+
+    vox, seg, ray, dirs, dec, d4 = case(n, channels, kind, 7 * n + channels)
+    k, B, W = int(kind[5:]), dirs.shape[0], dec.width
+    dv, ds, dr, dd, dp, dg = (x.cuda().contiguous() for x in (vox, seg, ray, dirs, pack_plain(dec), d4))
+    st = N.stream(dv.device)
+    pe_feat, pe_out, out4 = (torch.empty(*s, device="cuda") for s in ((B, 28), (B, W), (n, 4)))
+    gv, gp = torch.zeros_like(dv), torch.zeros_like(dp)
+    grid = (N.ptr(dv), 10, 8, 6, N.ptr(ds), N.ptr(dr), n, None)
+    N.call("dv_ray_pe", k, channels, N.ptr(dp), B, N.ptr(dd), N.ptr(pe_feat), N.ptr(pe_out), st)
+    N.call("dv_decode_fwd", k, channels, N.ptr(dp), *grid, N.ptr(pe_out), N.ptr(out4), st)
+    N.call("dv_decode_bwd", k, channels, N.ptr(dp), *grid, N.ptr(pe_feat), N.ptr(pe_out), N.ptr(dg), N.ptr(gv),
+           N.ptr(gp), st)
+
+    v64 = vox.double().requires_grad_(True)
+    layers = [(w.double().requires_grad_(True), b.double().requires_grad_(True)) for w, b in dec.layers]
+    feat = torch_ref.integrate(v64, seg[:, :3].double(), seg[:, 3:].double(), per_axis=True)
+    sigma, rgb = torch_ref.decode(layers, dec.n_mlp1, feat, dirs.double()[ray.long()])
+    ref = torch.cat([sigma[:, None], rgb], 1)
+    (ref * d4.double()).sum().backward()
+    assert (out4.cpu().double() - ref.detach()).abs().max() < 1e-5
+    assert (gv.cpu().double() - v64.grad).norm() <= 1e-4 * v64.grad.norm()
+    for (gw, gb), (w, b) in zip(unpack_plain_grad(kind, channels, gp.cpu().double()), layers):
+        assert (gw - w.grad).norm() <= 1e-4 * w.grad.norm()
+        assert (gb - b.grad).norm() <= 1e-4 * b.grad.norm()
