@@ -147,295 +147,378 @@ __global__ void __launch_bounds__(256) dense_walk_kernel(const WalkArgs a) {
   if (MODE != WALK_SEGMENTS) warp_max_atomic(a.max_count, count, live);
 }
 
-// Segment record writer for the compacted (CSR) output.  A segment at an even
-// global index is held back in registers; its successor then goes out with it
-// as one 48-byte pair (three aligned 16-byte stores of the six coordinates,
-// 8-byte stores of the two t and ray values).  A segment that has no
-// successor slot, or that sits at an odd index with nothing held, is written
-// alone (8-byte stores).  Needs seg 16-byte and seg_t / seg_ray 8-byte aligned
-// buffers, which the entry points check.
-struct SegWriter {
-  float h[7];  // held segment: entry xyz, exit xyz, t
-  int64_t hi;  // its global index, -1 when nothing is held
-  __device__ __forceinline__ SegWriter() : hi(-1) {}
-
-  __device__ __forceinline__ void single(const WalkArgs& a, int b, int64_t g, const float* v, float t) {
-    float2* sg = reinterpret_cast<float2*>(a.seg + g * 6);
-    sg[0] = make_float2(v[0], v[1]);
-    sg[1] = make_float2(v[2], v[3]);
-    sg[2] = make_float2(v[4], v[5]);
-    if (a.seg_t) a.seg_t[g] = t;
-    if (a.seg_ray) a.seg_ray[g] = b;
-  }
-
-  __device__ __forceinline__ void put(const WalkArgs& a, int b, int64_t g, bool has_next, const float3 p,
-                                      const float3 q, float t) {
-    if (hi >= 0) {  // g == hi + 1, hi even
-      float4* s4 = reinterpret_cast<float4*>(a.seg + hi * 6);
-      s4[0] = make_float4(h[0], h[1], h[2], h[3]);
-      s4[1] = make_float4(h[4], h[5], p.x, p.y);
-      s4[2] = make_float4(p.z, q.x, q.y, q.z);
-      if (a.seg_t) *reinterpret_cast<float2*>(a.seg_t + hi) = make_float2(h[6], t);
-      if (a.seg_ray) *reinterpret_cast<int2*>(a.seg_ray + hi) = make_int2(b, b);
-      hi = -1;
-    } else if (((g & 1) == 0) && has_next) {
-      h[0] = p.x;
-      h[1] = p.y;
-      h[2] = p.z;
-      h[3] = q.x;
-      h[4] = q.y;
-      h[5] = q.z;
-      h[6] = t;
-      hi = g;
-    } else {
-      const float v[6] = {p.x, p.y, p.z, q.x, q.y, q.z};
-      single(a, b, g, v, t);
-    }
-  }
-
-  __device__ __forceinline__ void flush(const WalkArgs& a, int b) {
-    if (hi >= 0) single(a, b, hi, h, h[6]);
-    hi = -1;
-  }
-};
-
 // Masked walk: (entry, exit) of every voxel whose occupancy byte is set.
 // Reference ray_voxel_intersect.cu:203-318.
 //
-// The crossing points form a dependent chain, but the occupancy byte of a
-// voxel only decides whether its segment is recorded.  The walk therefore
-// runs LOOKAHEAD steps ahead: it computes up to LOOKAHEAD crossings and issues
-// their occupancy loads back to back, then records the occupied ones in
-// order, so a ray waits for one load latency per LOOKAHEAD voxels instead of
-// one per voxel (which bounds small batches, where few warps are resident).
-template <int MODE, bool FAST, int LOOKAHEAD>
-__device__ __forceinline__ int masked_walk(const WalkArgs& a, int b, float3 p, const float3 d, float t) {
-  const float3 s = signs(d);
-  const float3 r = FAST ? recip3(d) : d;
-  float* row = nullptr;
-  float* trow = nullptr;
-  int64_t base = 0, cap = 0;
-  if (MODE == WALK_PADDED) {
-    row = a.inter + (long long)b * a.max_n * 6;
-    trow = a.tns + (long long)b * a.max_n;
-  }
-  if (MODE == WALK_SEGMENTS) {
-    base = a.offsets[b];
-    cap = a.offsets[b + 1] - base;
-  }
-  if (MODE == WALK_SLOTS) {
-    base = (int64_t)b * a.slot;
-    cap = a.slot;
-  }
-  SegWriter w;
-  int count = 0;
-  bool done = false;
-  // steps taken so far, the step of the last occupied voxel (counting), and
-  // where the walk may stop (emitting: nothing occupied lies beyond it)
-  int steps = 0, last = 0;
-  const int step_cap = walk_cap(a.n3.x, a.n3.y, a.n3.z);
-  const int limit = min((MODE == WALK_SEGMENTS && a.stop_step) ? a.stop_step[b] : 0x7fffffff, step_cap);
-  bool left = false;  // the walk left the grid
-  while (!done) {
-    float3 P[LOOKAHEAD + 1];
-    float T[LOOKAHEAD];
-    uint8_t occ[LOOKAHEAD];
-    unsigned inb = 0;  // bit k: step k stayed in the box and its cell is inside the mask
-    const int first = steps;
-    P[0] = p;
-#pragma unroll
-    for (int k = 0; k < LOOKAHEAD; ++k) {
-      if (!done && steps >= limit) done = true;
-      if (!done) {
-        ++steps;
-        float3 q;
-        float dt;
-        grid_step<FAST>(P[k], d, r, s, q, dt);
-        t = __fadd_rn(t, dt);
-        if (outside_closed3(q, a.n3)) {
-          done = true;
-          left = true;
-        } else {
-          P[k + 1] = q;
-          T[k] = t;
-          const long long idx = cell_index3(P[k], q, a.mask_scale, a.mx, a.my);
-          const bool in_mask = idx >= 0 && idx < a.cells;
-          // the address is clamped rather than the loaded value selected, so
-          // nothing reads the byte before all LOOKAHEAD loads are in flight
-          occ[k] = __ldg(a.mask + (in_mask ? idx : 0));
-          inb |= (in_mask ? 1u : 0u) << k;
-        }
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < LOOKAHEAD; ++k) {
-      if (((inb >> k) & 1u) && occ[k] != 0) {
-        last = first + k + 1;
-        if (MODE == WALK_PADDED && count < a.max_n) {
-          float* rr = row + 6 * count;
-          rr[0] = P[k].x;
-          rr[1] = P[k].y;
-          rr[2] = P[k].z;
-          rr[3] = P[k + 1].x;
-          rr[4] = P[k + 1].y;
-          rr[5] = P[k + 1].z;
-          trow[count] = __fmul_rn(T[k], a.voxel_size);
-        }
-        if ((MODE == WALK_SEGMENTS || MODE == WALK_SLOTS) && count < cap)
-          w.put(a, b, base + count, count + 1 < cap, P[k], P[k + 1], __fmul_rn(T[k], a.voxel_size));
-        ++count;
-      }
-    }
-    p = P[LOOKAHEAD];  // only read again when all LOOKAHEAD steps stayed inside
-  }
-  if (!left && steps >= step_cap) note_cap_hit();
-  if (MODE == WALK_SEGMENTS || MODE == WALK_SLOTS) w.flush(a, b);
-  if (MODE == WALK_COUNT && a.last_step) a.last_step[b] = last;
-  return count;
+// A ray's crossing points are a dependent chain of some hundred steps; what
+// each point means (its voxel, the occupancy byte, the output record) is not.
+// So the two are different warps' work.  Warp 0 walks 32 rays, a lane each,
+// and does nothing else: it writes chunks of 32 points per ray into a
+// double-buffered ring in shared memory.  The other warps take the rays one
+// by one, a lane per step of the chunk: the 32 occupancy bytes of a ray's
+// chunk are one load per lane, a ballot gives the count and every segment's
+// place, and a ray's run goes out as contiguous stores.
+//
+// What bounds it: a small batch, the walker's step (68 clocks of dependent
+// chain measured alone, against 93 with the planes recomputed each step); a
+// large one, the hand-over's latency and instruction issue.
+template <int NC>
+struct WalkRing {
+  static constexpr int STEPS = 32, ROW = STEPS + 1;  // points per ray and chunk: the chunk's start and its steps' ends
+  float4 pt[2][32 * ROW];                            // (x, y, z, t); rows of 33 keep both access patterns conflict-free
+  int steps[2][32];                                  // steps of the chunk that count, if they stay inside the box
+  int more[2];                                       // another chunk follows
+  float2 out[NC][STEPS * 3];                         // a ray's segments of one chunk on their way out
+};
+
+// Ring barriers of slot 0 / 1: FULL (the walker arrives, the consumers wait) and
+// EMPTY (the consumers arrive, the walker waits), n threads in all.
+template <int ID>
+__device__ __forceinline__ void ring_sync(int slot, int n) {
+  if (slot)
+    asm volatile("bar.sync %0, %1;" ::"n"(ID + 1), "r"(n) : "memory");
+  else
+    asm volatile("bar.sync %0, %1;" ::"n"(ID), "r"(n) : "memory");
+}
+template <int ID>
+__device__ __forceinline__ void ring_arrive(int slot, int n) {
+  if (slot)
+    asm volatile("bar.arrive %0, %1;" ::"n"(ID + 1), "r"(n) : "memory");
+  else
+    asm volatile("bar.arrive %0, %1;" ::"n"(ID), "r"(n) : "memory");
 }
 
-// K steps of lookahead: 16 for small batches (one warp per SM: registers are
-// plentiful and the occupancy-load latency is what is left), 8 otherwise
-// (the walk is issue-bound once several warps share a scheduler).
-template <int MODE, int K = 8>
-__global__ void __launch_bounds__(256) masked_walk_kernel(const WalkArgs a) {
+// A ray's walk state: the point, the next plane of each axis, the distance.
+struct Walk {
+  float3 a, B;
+  float t;
+};
+
+__device__ __forceinline__ float3 next_planes(const float3 a, const float3 s) {
+  return make_float3(floorf(__fmaf_rn(a.x, s.x, 1.f)), floorf(__fmaf_rn(a.y, s.y, 1.f)),
+                     floorf(__fmaf_rn(a.z, s.z, 1.f)));
+}
+
+// grid_step<true>, bit for bit, without recomputing the next plane of an
+// axis, floor(a s + 1) s, from the point each time (FRND runs at a quarter of
+// the rate and sits on the step's dependent chain).  B = floor(a s + 1) is
+// kept instead: an axis that was hit sits on its plane, so its B grows by
+// exactly 1; on another axis the coordinate moved towards its plane and B
+// stands, unless rounding took a s + 1 up to B + 1, which needs a point within
+// a few ulp of the plane.  `gap` takes the smallest distance to a next plane
+// met so far: when it ends up below near_plane() the caller redoes its steps
+// with EXACT, which recomputes the planes every time.
+template <bool EXACT>
+__device__ __forceinline__ void walk_step(Walk& w, const float3 d, const float3 r, const float3 s, float& gap) {
+  if (EXACT) w.B = next_planes(w.a, s);
+  const float gx = __fmaf_rn(w.B.x, s.x, -w.a.x), gy = __fmaf_rn(w.B.y, s.y, -w.a.y), gz = __fmaf_rn(w.B.z, s.z, -w.a.z);
+  if (!EXACT) gap = fminf(gap, fminf(fminf(fabsf(gx), fabsf(gy)), fabsf(gz)));
+  const float tx = div_by_recip(gx, d.x, r.x), ty = div_by_recip(gy, d.y, r.y), tz = div_by_recip(gz, d.z, r.z);
+  const float dt = fminf(tx, fminf(ty, tz));
+  const bool hx = dt == tx, hy = !hx && dt == ty, hz = !hx && !hy;
+  w.a = make_float3(hx ? __fmul_rn(w.B.x, s.x) : __fmaf_rn(d.x, dt, w.a.x),
+                    hy ? __fmul_rn(w.B.y, s.y) : __fmaf_rn(d.y, dt, w.a.y),
+                    hz ? __fmul_rn(w.B.z, s.z) : __fmaf_rn(d.z, dt, w.a.z));
+  w.B.x = __fadd_rn(w.B.x, hx ? 1.f : 0.f);
+  w.B.y = __fadd_rn(w.B.y, hy ? 1.f : 0.f);
+  w.B.z = __fadd_rn(w.B.z, hz ? 1.f : 0.f);
+  w.t = __fadd_rn(w.t, dt);
+}
+
+// 2^-22 of the extent, 2 ulp of any coordinate or more: a point that rounding
+// carried to or past its plane is nearer (within half an ulp before it, or past
+// it by the rounding of dt and of the point, at most one ulp).
+__device__ __forceinline__ float near_plane(const float3 n) {
+  return (fmaxf(n.x, fmaxf(n.y, n.z)) + 2.f) * 2.38418579e-7f;
+}
+
+// 32 steps of a lane's ray, written to row[1..32] (row[0]: where they start).
+// The coordinates only move outwards, so a ray that left the box is outside
+// at the chunk's end too: the walker looks there, the consumers find the step.
+// Every lane of the warp takes part (planes are checked once per 8 steps and
+// warp).
+__device__ __forceinline__ void walk_chunk_fast(Walk& w, const float3 d, const float3 r, const float3 s, float near,
+                                                float4* row) {
+  row[0] = make_float4(w.a.x, w.a.y, w.a.z, w.t);
+#pragma unroll 1
+  for (int k0 = 1; k0 <= 32; k0 += 8) {
+    const Walk w0 = w;
+    float gap = near;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      walk_step<false>(w, d, r, s, gap);
+      row[k0 + k] = make_float4(w.a.x, w.a.y, w.a.z, w.t);
+    }
+    if (__any_sync(0xffffffffu, gap < near)) {
+      w = w0;
+#pragma unroll 1
+      for (int k = 0; k < 8; ++k) {
+        walk_step<true>(w, d, r, s, gap);
+        row[k0 + k] = make_float4(w.a.x, w.a.y, w.a.z, w.t);
+      }
+    }
+  }
+}
+
+// The same for warps with a ray whose direction has a zero or extreme
+// component (recip_ok): the plain step, until the first point outside.  The
+// rest of the row repeats that point.
+__device__ __forceinline__ void walk_chunk_any(Walk& w, const float3 d, const float3 r, const float3 s, bool fast,
+                                               const float3 n, bool alive, float4* row) {
+  row[0] = make_float4(w.a.x, w.a.y, w.a.z, w.t);
+#pragma unroll 1
+  for (int k = 1; k <= 32; ++k) {
+    if (alive) {
+      float3 q;
+      float dt;
+      if (fast)
+        grid_step<true>(w.a, d, r, s, q, dt);
+      else
+        grid_step<false>(w.a, d, r, s, q, dt);
+      w.t = __fadd_rn(w.t, dt);
+      alive = !outside_closed3(q, n);
+      w.a = q;
+    }
+    row[k] = make_float4(w.a.x, w.a.y, w.a.z, w.t);
+  }
+}
+
+// Threads of a block: the walker, an idle warp 4 (warps 0, 4, 8, ... share a
+// scheduler, and the walker's should be the least loaded) and NC consumers.
+__host__ __device__ constexpr int walk_threads(int nc) { return 32 * (2 + nc); }
+
+// MODE: WALK_COUNT counts (num, max_count, last_step); WALK_PADDED fills rows
+// of max_n; WALK_SEGMENTS fills CSR ranges up to stop_step; WALK_SLOTS counts
+// and fills fixed ranges.  NC consumer warps, each owning 32 / NC of the rays.
+template <int MODE, int NC>
+__global__ void __launch_bounds__(walk_threads(NC)) masked_walk_kernel(const WalkArgs a) {
+  using R = WalkRing<NC>;
+  constexpr int FULL = 1, EMPTY = 3, ALL = 32 * (1 + NC), OWN = 32 / NC;
+  extern __shared__ __align__(16) uint8_t walk_smem[];
+  R& ring = *reinterpret_cast<R*>(walk_smem);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int b = blockIdx.x * 32 + lane;
+  if (warp == 0) {
+    bool alive = false, fast = true;
+    // a lane without a ray walks a harmless one
+    float3 d = make_float3(1.f, 1.f, 1.f), p = make_float3(0.5f, 0.25f, 0.125f);
+    float t = 0.f;
+    if (b < a.batch) {
+      const float3 v = load3(a.v, b);
+      float3 o = ray_origin_voxel3(a.o, b, a.o3, a.voxel_size);
+      float te;
+      if (dir_ok(v) && box_entry3(o, v, a.n3, te)) {
+        alive = true;
+        fast = a.fast && recip_ok(v);
+        d = v;
+        p = o;
+        t = te;
+      }
+    }
+    const float3 s = signs(d);
+    const float3 r = fast ? recip3(d) : d;
+    Walk w{p, next_planes(p, s), t};
+    const float near = near_plane(a.n3);
+    const int step_cap = walk_cap(a.n3.x, a.n3.y, a.n3.z);
+    const int limit =
+        alive && MODE == WALK_SEGMENTS && a.stop_step ? min(a.stop_step[b], step_cap) : step_cap;
+    alive = alive && limit > 0;
+    const bool all_fast = __all_sync(0xffffffffu, fast);
+    int steps = 0, c = 0;
+    for (;; ++c) {
+      const int slot = c & 1;
+      if (c >= 2) ring_sync<EMPTY>(slot, ALL);
+      float4* row = ring.pt[slot] + lane * R::ROW;
+      const int allowed = alive ? min(32, limit - steps) : 0;  // steps that the consumers may look at
+      if (all_fast)
+        walk_chunk_fast(w, d, r, s, near, row);
+      else
+        walk_chunk_any(w, d, r, s, fast, a.n3, alive, row);
+      steps += 32;
+      alive = alive && !outside_closed3(w.a, a.n3);
+      if (alive && steps >= limit) {
+        if (limit == step_cap) note_cap_hit();
+        alive = false;
+      }
+      ring.steps[slot][lane] = allowed;
+      const bool more = __any_sync(0xffffffffu, alive);
+      if (lane == 0) ring.more[slot] = more;
+      __threadfence_block();
+      ring_arrive<FULL>(slot, ALL);
+      if (!more) break;
+    }
+    // the consumers' last releases
+    if (c >= 1) ring_sync<EMPTY>((c - 1) & 1, ALL);
+    ring_sync<EMPTY>(c & 1, ALL);
+    return;
+  }
+  if (warp == 4) return;
+  const int consumer = warp > 4 ? warp - 2 : warp - 1;
+  const int first = consumer * OWN;  // this warp's rays: first .. first + OWN - 1, state in the lane of that number
+  const bool own = lane >= first && lane < first + OWN && b < a.batch;
+  int count = 0, last = 0;
+  long long base = 0, cap = 0x7fffffff;
+  if (own) {
+    if (MODE == WALK_SEGMENTS) {
+      base = a.offsets[b];
+      cap = a.offsets[b + 1] - base;
+    } else if (MODE == WALK_SLOTS) {
+      base = (long long)b * a.slot;
+      cap = a.slot;
+    } else if (MODE == WALK_PADDED) {
+      base = (long long)b * a.max_n;
+      cap = a.max_n;
+    }
+  }
+  const int room = (int)(cap < 0x7fffffff ? cap : 0x7fffffff);
+  float2* out = ring.out[consumer];
+  float* seg = MODE == WALK_PADDED ? a.inter : a.seg;
+  float* seg_t = MODE == WALK_PADDED ? a.tns : a.seg_t;
+  int* seg_ray = MODE == WALK_SEGMENTS ? a.seg_ray : nullptr;
+  for (int c = 0;; ++c) {
+    const int slot = c & 1;
+    ring_sync<FULL>(slot, ALL);
+    const int steps = ring.steps[slot][lane];
+    const bool more = ring.more[slot] != 0;
+    constexpr int U = OWN < 8 ? OWN : 8;  // rays whose occupancy loads are in flight together
+#pragma unroll 1
+    for (int i = first; i < first + OWN; i += U) {
+      uint8_t occ[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int n = __shfl_sync(0xffffffffu, steps, i + u);
+        occ[u] = 0;
+        if (n == 0) continue;
+        const float4* row = ring.pt[slot] + (i + u) * R::ROW + lane;
+        const float4 p = row[0], q = row[1];
+        const unsigned out = __ballot_sync(0xffffffffu, outside_closed3(make_float3(q.x, q.y, q.z), a.n3));
+        if (lane < n && (out & (0xffffffffu >> (31 - lane))) == 0u) {  // no step up to this one left the box
+          const long long idx =
+              cell_index3(make_float3(p.x, p.y, p.z), make_float3(q.x, q.y, q.z), a.mask_scale, a.mx, a.my);
+          if (idx >= 0 && idx < a.cells) occ[u] = __ldg(a.mask + idx);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const unsigned m = __ballot_sync(0xffffffffu, occ[u] != 0);
+        if (m == 0u) continue;
+        const int got = __popc(m);
+        if (MODE != WALK_COUNT) {
+          const int have = __shfl_sync(0xffffffffu, count, i + u);
+          const long long g = __shfl_sync(0xffffffffu, base, i + u) + have;
+          const int n = min(got, __shfl_sync(0xffffffffu, room, i + u) - have);  // segments that fit
+          const int rank = __popc(m & ((1u << lane) - 1u));
+          __syncwarp();  // the previous ray's run has left `out`
+          if (occ[u] != 0 && rank < n) {
+            const float4* row = ring.pt[slot] + (i + u) * R::ROW + lane;
+            const float4 p = row[0], q = row[1];
+            out[3 * rank] = make_float2(p.x, p.y);
+            out[3 * rank + 1] = make_float2(p.z, q.x);
+            out[3 * rank + 2] = make_float2(q.y, q.z);
+            if (seg_t) seg_t[g + rank] = __fmul_rn(q.w, a.voxel_size);
+            if (seg_ray) seg_ray[g + rank] = blockIdx.x * 32 + i + u;
+          }
+          __syncwarp();
+          if (MODE == WALK_PADDED) {
+            for (int w = lane; w < 6 * n; w += 32) seg[6 * g + w] = reinterpret_cast<const float*>(out)[w];
+          } else {
+            for (int w = lane; w < 3 * n; w += 32) reinterpret_cast<float2*>(seg)[3 * g + w] = out[w];
+          }
+        }
+        if (lane == i + u) {
+          count += got;
+          last = 32 * c + 32 - __clz(m);
+        }
+      }
+    }
+    __threadfence_block();
+    ring_arrive<EMPTY>(slot, ALL);
+    if (!more) break;
+  }
+  if (MODE != WALK_SEGMENTS) {
+    if (own) a.num[b] = count;
+    if (MODE == WALK_COUNT && own && a.last_step) a.last_step[b] = last;
+    const int mx = __reduce_max_sync(0xffffffffu, own ? count : 0);
+    if (a.max_count && lane == 0) atomicMax(a.max_count, mx);
+  }
+}
+
+// Counts for large batches: a thread per ray, 8 steps at a time, their 8
+// occupancy loads issued back to back.  With enough rays to fill the
+// schedulers, total instructions set the time and the ring's hand-over only
+// adds to them.
+__global__ void __launch_bounds__(256) masked_count_kernel(const WalkArgs a) {
+  constexpr int K = 8;
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool live = b < a.batch;
-  int count = 0;
-  if (live) {
+  int count = 0, last = 0;
+  if (b < a.batch) {
     const float3 d = load3(a.v, b);
     float3 p = ray_origin_voxel3(a.o, b, a.o3, a.voxel_size);
     float t;
-    if (dir_ok(d) && box_entry3(p, d, a.n3, t))
-      count = (a.fast && recip_ok(d)) ? masked_walk<MODE, true, K>(a, b, p, d, t)
-                                      : masked_walk<MODE, false, K>(a, b, p, d, t);
-    else if (MODE == WALK_COUNT && a.last_step)
-      a.last_step[b] = 0;
-    if (MODE != WALK_SEGMENTS) a.num[b] = count;
-  }
-  if (MODE != WALK_SEGMENTS) warp_max_atomic(a.max_count, count, live);
-}
-
-// Masked-walk emission for large batches, warp-staged.  The 32 rays of a
-// warp own separate CSR ranges, so each lane writing its own segments
-// scatters 32 stores per instruction across the output.  Here every lane
-// stages its segments in shared memory (16 slots: at least two lookahead
-// batches between flushes), and when any lane could overflow in the next
-// batch, or the warp finishes, the warp writes each lane's run with
-// consecutive stores (the run of lane l is contiguous: seg[g_l .. g_l + n_l)).
-// Same values, same places as the per-lane writer; the walk arithmetic is the
-// same masked walk.  Blocks of one warp: the slots cost 512 B per lane, and
-// smaller blocks measured faster (800x800 frame: 2.1 ms, against 2.4 ms with
-// two warps per block, 3.3 ms with 8 slots and 4 warps, 3.5 ms per-lane).
-constexpr int STAGE_THREADS = 32;
-constexpr int STAGE_SLOTS = 16;
-
-__device__ __forceinline__ void grid_step_sel(const float3 a, const float3 d, const float3 r, const float3 s, bool fast,
-                                              float3& b, float& dt) {
-  if (fast)
-    grid_step<true>(a, d, r, s, b, dt);
-  else
-    grid_step<false>(a, d, r, s, b, dt);
-}
-
-__global__ void __launch_bounds__(STAGE_THREADS) masked_emit_staged_kernel(const WalkArgs a) {
-  constexpr int K = 8;  // lookahead steps per batch
-  __shared__ __align__(16) float stage[STAGE_THREADS * STAGE_SLOTS * 8];  // (6 coords, t, pad) per slot
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  const int lane = threadIdx.x & 31;
-  const int warp0 = threadIdx.x - lane;  // first thread of this warp in the block
-  float* mine = stage + threadIdx.x * STAGE_SLOTS * 8;
-  bool done = true, fast = false;
-  float3 p = make_float3(0.f, 0.f, 0.f), d = p, r = p, sg = p;
-  float t = 0.f;
-  int64_t base = 0, cap = 0;
-  int count = 0;
-  if (b < a.batch) {
-    d = load3(a.v, b);
-    p = ray_origin_voxel3(a.o, b, a.o3, a.voxel_size);
     if (dir_ok(d) && box_entry3(p, d, a.n3, t)) {
-      done = false;
-      fast = a.fast && recip_ok(d);
-      r = fast ? recip3(d) : d;
-      sg = signs(d);
-      base = a.offsets[b];
-      cap = a.offsets[b + 1] - base;
-    }
-  }
-  int nb = 0;         // staged segments of this lane
-  int64_t g = base;   // global index of the first staged one
-  int steps = 0;      // walk steps taken; nothing occupied lies beyond `limit`
-  const int step_cap = walk_cap(a.n3.x, a.n3.y, a.n3.z);
-  const int limit = min((!done && a.stop_step) ? a.stop_step[b] : 0x7fffffff, step_cap);
-  bool left = false;  // the walk left the grid
-  while (__any_sync(0xffffffffu, !done) || __any_sync(0xffffffffu, nb > 0)) {
-    if (!done) {
-      float3 P[K + 1];
-      float T[K];
-      uint8_t occ[K];
-      unsigned inb = 0;
-      P[0] = p;
+      const bool fast = a.fast && recip_ok(d);
+      const float3 s = signs(d), r = fast ? recip3(d) : d;
+      const float near = near_plane(a.n3);
+      const int step_cap = walk_cap(a.n3.x, a.n3.y, a.n3.z);
+      Walk w{p, next_planes(p, s), t};
+      for (int steps = 0;; steps += K) {
+        float3 P[K + 1];
+        unsigned out = 0;
+        P[0] = w.a;
+        const Walk w0 = w;
+        float gap = near;
+        if (fast) {
 #pragma unroll
-      for (int k = 0; k < K; ++k) {
-        if (!done && steps >= limit) done = true;
-        if (!done) {
-          ++steps;
-          float3 q;
-          float dt;
-          grid_step_sel(P[k], d, r, sg, fast, q, dt);
-          t = __fadd_rn(t, dt);
-          if (outside_closed3(q, a.n3)) {
-            done = true;
-            left = true;
-          } else {
-            P[k + 1] = q;
-            T[k] = t;
-            const long long idx = cell_index3(P[k], q, a.mask_scale, a.mx, a.my);
-            const bool in_mask = idx >= 0 && idx < a.cells;
-            occ[k] = __ldg(a.mask + (in_mask ? idx : 0));
-            inb |= (in_mask ? 1u : 0u) << k;
+          for (int k = 0; k < K; ++k) {
+            walk_step<false>(w, d, r, s, gap);
+            P[k + 1] = w.a;
+            out |= outside_closed3(w.a, a.n3) ? 1u << k : 0u;
           }
         }
-      }
+        if (!fast || gap < near) {
+          w = w0;
+          out = 0;
 #pragma unroll
-      for (int k = 0; k < K; ++k) {
-        if (((inb >> k) & 1u) && occ[k] != 0) {
-          if (count < cap) {
-            float4* slot = reinterpret_cast<float4*>(mine + nb * 8);
-            slot[0] = make_float4(P[k].x, P[k].y, P[k].z, P[k + 1].x);
-            slot[1] = make_float4(P[k + 1].y, P[k + 1].z, __fmul_rn(T[k], a.voxel_size), 0.f);
-            ++nb;
+          for (int k = 0; k < K; ++k) {
+            if (out != 0) continue;
+            float3 q;
+            float dt;
+            if (fast)
+              grid_step<true>(w.a, d, r, s, q, dt);
+            else
+              grid_step<false>(w.a, d, r, s, q, dt);
+            w.a = P[k + 1] = q;
+            out |= outside_closed3(q, a.n3) ? 1u << k : 0u;
           }
-          ++count;
+          w.B = next_planes(w.a, s);
+        }
+        const int inside = min(out ? __ffs(out) - 1 : K, step_cap - steps);
+        uint8_t occ[K];
+        unsigned in_mask = 0;
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          const long long idx = cell_index3(P[k], P[k + 1], a.mask_scale, a.mx, a.my);
+          const bool ok = k < inside && idx >= 0 && idx < a.cells;
+          occ[k] = __ldg(a.mask + (ok ? idx : 0));
+          in_mask |= ok ? 1u << k : 0u;
+        }
+        unsigned m = 0;
+#pragma unroll
+        for (int k = 0; k < K; ++k) m |= occ[k] != 0 ? 1u << k : 0u;
+        m &= in_mask;
+        count += __popc(m);
+        if (m) last = steps + 32 - __clz(m);
+        if (out) break;
+        if (steps + K >= step_cap) {
+          note_cap_hit();
+          break;
         }
       }
-      p = P[K];
     }
-    // flush when a lane could overflow in the next batch, or when the warp is finishing
-    if (!(__any_sync(0xffffffffu, nb > STAGE_SLOTS - K) || !__any_sync(0xffffffffu, !done))) continue;
-    __syncwarp();
-    unsigned pending = __ballot_sync(0xffffffffu, nb > 0);
-    while (pending) {
-      const int l = __ffs(pending) - 1;
-      pending &= pending - 1;
-      const int n = __shfl_sync(0xffffffffu, nb, l);
-      const long long gl = (long long)(((unsigned long long)(unsigned)__shfl_sync(0xffffffffu, (int)(g >> 32), l) << 32) |
-                                       (unsigned)__shfl_sync(0xffffffffu, (int)(g & 0xffffffffu), l));
-      const float* src = stage + (warp0 + l) * STAGE_SLOTS * 8;
-      for (int w = lane; w < n * 6; w += 32) {
-        const int k = w / 6;
-        a.seg[gl * 6 + w] = src[k * 8 + (w - k * 6)];
-      }
-      if (lane < n) {
-        if (a.seg_t) a.seg_t[gl + lane] = src[lane * 8 + 6];
-        if (a.seg_ray) a.seg_ray[gl + lane] = blockIdx.x * blockDim.x + warp0 + l;
-      }
-    }
-    g += nb;
-    nb = 0;
-    __syncwarp();
+    a.num[b] = count;
+    if (a.last_step) a.last_step[b] = last;
   }
-  if (b < a.batch && steps > 0 && !left && steps >= step_cap) note_cap_hit();
+  warp_max_atomic(a.max_count, count, b < a.batch);
 }
 
 // Slots -> CSR: row k of ray b moves from b * slot + k to offsets[b] + k.
@@ -711,11 +794,7 @@ static int cells_per_side(float n, float scale) {
   return (int)prod;
 }
 
-// Threads per block of a walk launch.  One thread walks one ray and the walk
-// is a long dependent chain, so a small batch runs faster spread thinly: with
-// fewer rays than 8 warps per SM, blocks of one warp put each warp on its own
-// SM instead of several warps sharing a scheduler.
-static int walk_block(int batch) {
+static int sm_count() {
   static int sms = 0;
   if (sms == 0) {
     int dev = 0;
@@ -723,17 +802,37 @@ static int walk_block(int batch) {
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (sms <= 0) sms = 1;
   }
-  return batch < sms * 256 ? 32 : 256;
+  return sms;
 }
 
-#define DV_COUNT_LAUNCH(batch, stream, args)                                                      \
-  do {                                                                                              \
-    const int bs__ = walk_block(batch);                                                             \
-    if (bs__ == 32)                                                                                 \
-      masked_walk_kernel<WALK_COUNT, 16><<<ceil_div((batch), bs__), bs__, 0, (cudaStream_t)(stream)>>>(args); \
-    else                                                                                            \
-      masked_walk_kernel<WALK_COUNT, 8><<<ceil_div((batch), bs__), bs__, 0, (cudaStream_t)(stream)>>>(args);  \
-  } while (0)
+// Launches a masked walk.  Up to two blocks per SM, 16 consumer warps (2 rays
+// each): the hand-over is latency, and only the walker should set the time;
+// beyond that 8, as blocks share the SM.  Measured, 16 / 8 consumers: a
+// 4096-ray batch into slots 54 / 85 us (4 consumers 165, a thread per ray
+// 251), 65,792 rays' segments 78 / 75 us (4: 99, 2: 150), 640,000 rays'
+// 1442 / 1224 us (a thread per ray with staged stores 2075).  A count has
+// less to hand over: from 768 rays per SM on, a thread per ray is faster
+// (65,792 rays: 91 us here, 105 there; 640,000 rays: 997 and 697 us).
+template <int MODE>
+static int masked_walk_launch(const WalkArgs& a, void* stream) {
+  const long long blocks = ceil_div(a.batch, 32);
+  const cudaStream_t st = (cudaStream_t)stream;
+  const int sms = sm_count();
+  if (MODE == WALK_COUNT && a.batch >= 768LL * sms)
+    masked_count_kernel<<<ceil_div(a.batch, 256), 256, 0, st>>>(a);
+  else if (blocks <= 2LL * sms)
+    masked_walk_kernel<MODE, 16><<<(unsigned)blocks, walk_threads(16), sizeof(WalkRing<16>), st>>>(a);
+  else
+    masked_walk_kernel<MODE, 8><<<(unsigned)blocks, walk_threads(8), sizeof(WalkRing<8>), st>>>(a);
+  DV_TRY_LAUNCH();
+  return DV_OK;
+}
+
+// Threads per block of a dense walk launch.  One thread walks one ray and the
+// walk is a long dependent chain, so a small batch runs faster spread thinly:
+// with fewer rays than 8 warps per SM, blocks of one warp put each warp on its
+// own SM instead of several warps sharing a scheduler.
+static int walk_block(int batch) { return batch < sm_count() * 256 ? 32 : 256; }
 
 #define DV_WALK_LAUNCH(kernel, batch, stream, args)                              \
   do {                                                                             \
@@ -817,9 +916,7 @@ int dv_masked_intersect(int batch_size, int max_n, float xyzmin, float xyzmax, f
   a.num = intersect_num;
   a.tns = tns;
   a.max_count = max_count;
-  DV_WALK_LAUNCH(masked_walk_kernel<WALK_PADDED>, batch_size, stream, a);
-  DV_TRY_LAUNCH();
-  return DV_OK;
+  return masked_walk_launch<WALK_PADDED>(a, stream);
 }
 
 int dv_masked_count(int batch_size, float xyzmin, float voxel_num, float voxel_size,
@@ -832,9 +929,7 @@ int dv_masked_count(int batch_size, float xyzmin, float voxel_num, float voxel_s
   a.num = intersect_num;
   a.max_count = max_count;
   a.last_step = last_step;
-  DV_COUNT_LAUNCH(batch_size, stream, a);
-  DV_TRY_LAUNCH();
-  return DV_OK;
+  return masked_walk_launch<WALK_COUNT>(a, stream);
 }
 
 int dv_masked_segments(int batch_size, float xyzmin, float voxel_num, float voxel_size,
@@ -851,12 +946,7 @@ int dv_masked_segments(int batch_size, float xyzmin, float voxel_num, float voxe
   a.seg_t = seg_t;
   a.seg_ray = seg_ray;
   a.stop_step = stop_step;
-  if (walk_block(batch_size) == 256)
-    masked_emit_staged_kernel<<<ceil_div(batch_size, STAGE_THREADS), STAGE_THREADS, 0, (cudaStream_t)stream>>>(a);
-  else
-    DV_WALK_LAUNCH(masked_walk_kernel<WALK_SEGMENTS>, batch_size, stream, a);
-  DV_TRY_LAUNCH();
-  return DV_OK;
+  return masked_walk_launch<WALK_SEGMENTS>(a, stream);
 }
 
 int dv_masked_segments_slots(int batch_size, float xyzmin, float voxel_num, float voxel_size, float mask_scale,
@@ -873,9 +963,7 @@ int dv_masked_segments_slots(int batch_size, float xyzmin, float voxel_num, floa
   a.seg_t = t_slots;
   a.num = intersect_num;
   a.max_count = max_count;
-  DV_WALK_LAUNCH(masked_walk_kernel<WALK_SLOTS>, batch_size, stream, a);
-  DV_TRY_LAUNCH();
-  return DV_OK;
+  return masked_walk_launch<WALK_SLOTS>(a, stream);
 }
 
 int dv_compact_slots(int batch_size, long long slot, const int64_t* offsets, const float* seg_slots,
@@ -967,9 +1055,7 @@ int dv_masked_count_grid(int batch_size, const float* xyzmin, const int* dims, f
   a.num = intersect_num;
   a.max_count = max_count;
   a.last_step = last_step;
-  DV_COUNT_LAUNCH(batch_size, stream, a);
-  DV_TRY_LAUNCH();
-  return DV_OK;
+  return masked_walk_launch<WALK_COUNT>(a, stream);
 }
 
 int dv_masked_segments_grid(int batch_size, const float* xyzmin, const int* dims, float voxel_size, const float* o,
@@ -985,12 +1071,7 @@ int dv_masked_segments_grid(int batch_size, const float* xyzmin, const int* dims
   a.seg_t = seg_t;
   a.seg_ray = seg_ray;
   a.stop_step = stop_step;
-  if (walk_block(batch_size) == 256)
-    masked_emit_staged_kernel<<<ceil_div(batch_size, STAGE_THREADS), STAGE_THREADS, 0, (cudaStream_t)stream>>>(a);
-  else
-    DV_WALK_LAUNCH(masked_walk_kernel<WALK_SEGMENTS>, batch_size, stream, a);
-  DV_TRY_LAUNCH();
-  return DV_OK;
+  return masked_walk_launch<WALK_SEGMENTS>(a, stream);
 }
 
 long long dv_walk_cap_hits(int reset) {
