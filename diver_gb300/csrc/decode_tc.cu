@@ -10,6 +10,14 @@
 //           mbarrier; thread t then reads its row (TMEM lane t), adds the bias,
 //           applies ReLU and writes the next A tile row
 //   output  sigma (FP32) and sigmoid(rgb) per segment
+// Issue slots and the L1's wavefronts bound it more than the tensor core does
+// (ncu on the form before: 67 % of issue slots, 69 % of LSU wavefronts, 5 %
+// tensor), so a segment's corners are computed once, additions and the
+// integral's FMAs go in packed pairs, biases come in 16-byte loads and ReLU is
+// taken on rounded pairs.  Measured against one thread per 8 channels doing
+// all of it: 800x800 frame of the 256^3 scene, BF16 10.5 -> 8.8 ms; DIVeR64 over
+// 64 channels, 399x401, FP16 5.2 -> 3.8 ms; split, 65,792 rays of the wide grid
+// 647 -> 509 us.
 // The decoder's weights (all layers, B operands in the same K-major layout)
 // and biases stay in shared memory for the CTA's lifetime; the grid is
 // persistent over tiles and sized so TMEM never oversubscribes.
@@ -32,6 +40,7 @@ struct TcLayer {
   int b_off;     // byte offset of the layer's B image in the weight blob
   int K, N;      // padded: K % 16 == 0, N % 16 == 0
   int bias_off;  // float offset of the layer's bias (N entries)
+  int s_bias;    // its offset in shared memory (a multiple of 16)
   int s_off;     // split form: byte offset of the layer's [3 x N][K] image (terms side by side) in shared memory
 };
 
@@ -48,7 +57,7 @@ struct TcArgs {
   const uint8_t* wblob;
   int wbytes;  // bytes of one term's weight images (multiple of 16); TERMS terms follow each other
   const float* bias;
-  int nbias;   // multiple of 4
+  int nbias;   // biases in shared memory
   TcLayer L[TC_MAX_LAYERS];
   int* err;    // set to 1 if an MMA completion wait timed out
   uint8_t* save;       // optional: every layer's input tile, per 128-segment tile (training)
@@ -67,138 +76,191 @@ __device__ __forceinline__ uint8_t* a_term(uint8_t* sA, uint32_t tstride, int r,
   return i < 2 ? sA + tc::kmajor_offset(r, i * K + c, 2 * K) : sA + 2 * tstride + tc::kmajor_offset(r, c, K);
 }
 
-// Gather from the FP32 grid: C/4 threads per segment, each integrating 4
-// channels; the feature row goes to the A tile as TERMS operand terms (a_term).
-template <int C, int BF16, int TERMS>
-__device__ __forceinline__ void gather_tile_lp(const TcArgs& a, long long S, long long s0, uint8_t* sA,
-                                               uint32_t tstride) {
-  constexpr int TPS = C / 4;
-  constexpr int SPP = 128 / TPS;
-  const int t = threadIdx.x;
+// Corner weights and rows of this thread's segment, s0 + threadIdx.x: the
+// weights, the lower corner's row and the row steps to the upper corners
+// (0 where clamped).  Computed once per segment and handed to the C/4 or C/8
+// threads that gather its channels, all in the same warp (computed by each of
+// them, this was a third of the kernel's instructions).  Rows fit 32 bits: 2^32
+// rows of 32 channels are twice the device's memory.
+struct Corners {
+  float w[8];
+  uint32_t row, dx, dy, dz;
+};
+
+__device__ __forceinline__ Corners corners_of(const TcArgs& a, long long S, long long s) {
+  Corners c{};
+  if (s < S) {
+    const float* sg = a.seg + s * 6;
+    const SegCorner sc = segment_corners(__ldg(sg), __ldg(sg + 1), __ldg(sg + 2), __ldg(sg + 3), __ldg(sg + 4),
+                                         __ldg(sg + 5), a.nvx, a.nvy, a.nvz);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) c.w[j] = sc.w[j];
+    c.row = ((uint32_t)sc.z * a.nvy + sc.y) * a.nvx + sc.x;
+    c.dx = sc.x1 - sc.x;
+    c.dy = (uint32_t)(sc.y1 - sc.y) * a.nvx;
+    c.dz = (uint32_t)(sc.z1 - sc.z) * a.nvx * a.nvy;
+  }
+  return c;
+}
+
+// The 8 corner rows (BYTES each) at byte q of a row.
+template <int BYTES>
+__device__ __forceinline__ void load_corners(const uint8_t* grid, uint32_t row, uint32_t dx, uint32_t dy, uint32_t dz,
+                                             uint4* v) {
+  const uint8_t* p = grid + (unsigned long long)row * BYTES;
+  const uint32_t x = dx * BYTES;
+  const uint8_t* py = p + (unsigned long long)dy * BYTES;
+  const uint8_t* pz = p + (unsigned long long)dz * BYTES;
+  const uint8_t* pw = py + (unsigned long long)dz * BYTES;
+  const uint8_t* r[4] = {p, py, pz, pw};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    v[2 * j] = __ldg(reinterpret_cast<const uint4*>(r[j]));
+    v[2 * j + 1] = __ldg(reinterpret_cast<const uint4*>(r[j] + x));
+  }
+}
+
+// Two FP32 values in one 64-bit register pair: the packed FMA and add round
+// each half like fmaf and +, in half the issue slots.
+__device__ __forceinline__ unsigned long long f32x2(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 f32x2_get(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ unsigned long long fma_f32x2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ unsigned long long add_f32x2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+// A 16-bit pair as two FP32 values.
+template <int BF16>
+__device__ __forceinline__ unsigned long long unpack2(uint32_t x) {
+  if (BF16) return f32x2(__uint_as_float(x << 16), __uint_as_float(x & 0xffff0000u));
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&x));
+  return f32x2(f.x, f.y);
+}
+
+constexpr int COEF = 12;  // floats of a segment's Corners in shared memory
+
+__device__ __forceinline__ void put_corners(float* coef, const Corners& c) {
+  float4* d = reinterpret_cast<float4*>(coef + threadIdx.x * COEF);
+  d[0] = make_float4(c.w[0], c.w[1], c.w[2], c.w[3]);
+  d[1] = make_float4(c.w[4], c.w[5], c.w[6], c.w[7]);
+  reinterpret_cast<uint4*>(d)[2] = make_uint4(c.row, c.dx, c.dy, c.dz);
+  __syncwarp();
+}
+
+// Single-term gather: TPS threads per segment, each integrating 16 bytes of
+// every corner row (4 channels of the FP32 grid, or 8 of its 16-bit copy) in
+// FP32, and writing the feature row's 16-bit operand.  U passes' loads are in
+// flight per thread.
+template <int C, int BF16, bool G16, int U>
+__device__ __forceinline__ void gather_tile(const TcArgs& a, long long S, long long s0, uint8_t* sA, float* coef) {
+  constexpr int CH = G16 ? 8 : 4, TPS = C / CH, SPP = 32 / TPS, BYTES = C * (G16 ? 2 : 4);
+  const int lane = threadIdx.x & 31, q = lane % TPS, first = (threadIdx.x & ~31) + lane / TPS;
+  put_corners(coef, corners_of(a, S, s0 + threadIdx.x));
+  const uint8_t* grid = (G16 ? reinterpret_cast<const uint8_t*>(a.grid16) : reinterpret_cast<const uint8_t*>(a.grid)) + 16 * q;
 #pragma unroll 1
-  for (int p = 0; p < TPS; ++p) {
-    const int ls = p * SPP + t / TPS;
-    const int q = t % TPS;
-    const long long s = s0 + ls;
-    float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (s < S) {
-      const float* sg = a.seg + s * 6;
-      const SegCorner sc = segment_corners(__ldg(sg), __ldg(sg + 1), __ldg(sg + 2), __ldg(sg + 3), __ldg(sg + 4),
-                                           __ldg(sg + 5), a.nvx, a.nvy, a.nvz);
-      f = integrate4(a.grid, sc, C, q, a.nvx, a.nvy);
+  for (int p = 0; p < TPS; p += U) {
+    uint4 v[U][8];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint4 m = *reinterpret_cast<const uint4*>(coef + (first + (p + u) * SPP) * COEF + 8);
+      load_corners<BYTES>(grid, m.x, m.y, m.z, m.w, v[u]);  // past the last segment: row 0, weights 0
     }
-    if constexpr (TERMS == 1) {
-      *reinterpret_cast<uint2*>(a_term<1>(sA, tstride, ls, 4 * q, C, 0)) =
-          make_uint2(tc::pack2<BF16>(f.x, f.y), tc::pack2<BF16>(f.z, f.w));
-    } else {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int ls = first + (p + u) * SPP;
+      const float4 wa = *reinterpret_cast<const float4*>(coef + ls * COEF);
+      const float4 wb = *reinterpret_cast<const float4*>(coef + ls * COEF + 4);
+      const float w[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+      unsigned long long f[CH / 2];
+#pragma unroll
+      for (int k = 0; k < CH / 2; ++k) f[k] = 0ull;
+      const bool in = s0 + ls < S;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const unsigned long long ww = f32x2(w[j], w[j]);
+        const uint4 x = v[u][j];
+        if (G16) {
+          f[0] = fma_f32x2(ww, unpack2<BF16>(x.x), f[0]);
+          f[1] = fma_f32x2(ww, unpack2<BF16>(x.y), f[1]);
+          f[CH / 2 - 2] = fma_f32x2(ww, unpack2<BF16>(x.z), f[CH / 2 - 2]);
+          f[CH / 2 - 1] = fma_f32x2(ww, unpack2<BF16>(x.w), f[CH / 2 - 1]);
+        } else {
+          f[0] = fma_f32x2(ww, f32x2(__uint_as_float(x.x), __uint_as_float(x.y)), f[0]);
+          f[1] = fma_f32x2(ww, f32x2(__uint_as_float(x.z), __uint_as_float(x.w)), f[1]);
+        }
+      }
+      uint32_t o[CH / 2];
+#pragma unroll
+      for (int k = 0; k < CH / 2; ++k) {
+        const float2 r = f32x2_get(f[k]);
+        o[k] = in ? tc::pack2<BF16>(r.x, r.y) : 0u;
+      }
+      uint8_t* dst = sA + tc::kmajor_offset(ls, CH * q, C);
+      if (G16)
+        *reinterpret_cast<uint4*>(dst) = make_uint4(o[0], o[1], o[CH / 2 - 2], o[CH / 2 - 1]);
+      else
+        *reinterpret_cast<uint2*>(dst) = make_uint2(o[0], o[1]);
+    }
+  }
+}
+
+// The split form's gather (FP32 grid, three operand terms): two passes at a
+// time, so each thread has 16 corner-row loads in flight.  Its kernel runs 4
+// CTAs per SM (its shared memory), so the registers this takes cost no
+// residency, and the corners go from lane to lane by shuffles, as shared
+// memory is what is short.
+template <int C, int TERMS>
+__device__ __forceinline__ void gather_tile_split(const TcArgs& a, long long S, long long s0, uint8_t* sA,
+                                                  uint32_t tstride) {
+  constexpr int TPS = C / 4, SPP = 32 / TPS;
+  static_assert(TPS % 2 == 0, "passes are taken in pairs");
+  const int lane = threadIdx.x & 31, warp0 = threadIdx.x & ~31, q = lane % TPS;
+  const Corners c = corners_of(a, S, s0 + threadIdx.x);
+  const uint8_t* grid = reinterpret_cast<const uint8_t*>(a.grid) + 16 * q;
+  const uint32_t flags = (c.dx ? 1u : 0u) | (c.dy ? 2u : 0u) | (c.dz ? 4u : 0u);
+#pragma unroll 1
+  for (int p = 0; p < TPS; p += 2) {
+    uint4 v[2][8];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int src = (p + u) * SPP + lane / TPS;
+      const uint32_t row = __shfl_sync(0xffffffffu, c.row, src), m = __shfl_sync(0xffffffffu, flags, src);
+      load_corners<C * 4>(grid, row, m & 1u, (m & 2u) ? a.nvx : 0, (m & 4u) ? (uint32_t)a.nvx * a.nvy : 0, v[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int src = (p + u) * SPP + lane / TPS, ls = warp0 + src;
+      unsigned long long f[2] = {0ull, 0ull};
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float w = __shfl_sync(0xffffffffu, c.w[j], src);
+        const uint4 x = v[u][j];
+        f[0] = fma_f32x2(f32x2(w, w), f32x2(__uint_as_float(x.x), __uint_as_float(x.y)), f[0]);
+        f[1] = fma_f32x2(f32x2(w, w), f32x2(__uint_as_float(x.z), __uint_as_float(x.w)), f[1]);
+      }
+      const bool in = s0 + ls < S;
+      const float2 lo = f32x2_get(f[0]), hi = f32x2_get(f[1]);
       uint32_t x[TERMS], y[TERMS];
-      tc::split_pair<TERMS>(f.x, f.y, x);
-      tc::split_pair<TERMS>(f.z, f.w, y);
+      tc::split_pair<TERMS>(in ? lo.x : 0.f, in ? lo.y : 0.f, x);
+      tc::split_pair<TERMS>(in ? hi.x : 0.f, in ? hi.y : 0.f, y);
 #pragma unroll
       for (int i = 0; i < TERMS; ++i)
         *reinterpret_cast<uint2*>(a_term<TERMS>(sA, tstride, ls, 4 * q, C, i)) = make_uint2(x[i], y[i]);
     }
-  }
-}
-
-// The split form's gather (FP32 grid, three operand terms): the same passes as
-// gather_tile_lp, two at a time, so each thread has 16 corner-row loads in
-// flight.  The split kernel runs 4 CTAs per SM (its shared memory), so the
-// registers this takes cost no residency; the single-term kernels keep the
-// one-pass gather (their residency is register-bound).
-template <int C, int TERMS>
-__device__ __forceinline__ void gather_tile_lp_x2(const TcArgs& a, long long S, long long s0, uint8_t* sA,
-                                                  uint32_t tstride) {
-  constexpr int TPS = C / 4;
-  constexpr int SPP = 128 / TPS;
-  static_assert(TPS % 2 == 0, "passes are taken in pairs");
-  const int t = threadIdx.x;
-  const int q = t % TPS;
-#pragma unroll 1
-  for (int p = 0; p < TPS; p += 2) {
-    SegCorner sc[2];
-    float4 v[2][8];
-    bool in[2];
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const long long s = s0 + (p + u) * SPP + t / TPS;
-      in[u] = s < S;
-      if (in[u]) {
-        const float* sg = a.seg + s * 6;
-        sc[u] = segment_corners(__ldg(sg), __ldg(sg + 1), __ldg(sg + 2), __ldg(sg + 3), __ldg(sg + 4), __ldg(sg + 5),
-                                a.nvx, a.nvy, a.nvz);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[u][j] = ldg4(a.grid + corner_row(sc[u], j, a.nvx, a.nvy) * C + q * 4);
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (in[u]) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) fma4(f, sc[u].w[j], v[u][j]);
-      }
-      uint32_t x[TERMS], y[TERMS];
-      tc::split_pair<TERMS>(f.x, f.y, x);
-      tc::split_pair<TERMS>(f.z, f.w, y);
-#pragma unroll
-      for (int i = 0; i < TERMS; ++i)
-        *reinterpret_cast<uint2*>(a_term<TERMS>(sA, tstride, (p + u) * SPP + t / TPS, 4 * q, C, i)) =
-            make_uint2(x[i], y[i]);
-    }
-  }
-}
-
-template <int BF16>
-__device__ __forceinline__ void unpack8(const uint4 w, float* f) {
-  const uint32_t x[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    if (BF16) {
-      f[2 * j] = __uint_as_float(x[j] << 16);
-      f[2 * j + 1] = __uint_as_float(x[j] & 0xffff0000u);
-    } else {
-      f[2 * j] = __half2float(__ushort_as_half((unsigned short)(x[j] & 0xffffu)));
-      f[2 * j + 1] = __half2float(__ushort_as_half((unsigned short)(x[j] >> 16)));
-    }
-  }
-}
-
-// Gather from the 16-bit copy of the grid: C/8 threads per segment, each
-// reading 16 bytes (8 channels) of every corner row; the integral is FP32.
-template <int C, int BF16>
-__device__ __forceinline__ void gather_tile_16(const TcArgs& a, long long S, long long s0, uint8_t* sA) {
-  constexpr int TPS = C / 8;
-  constexpr int SPP = 128 / TPS;
-  const int t = threadIdx.x;
-#pragma unroll 1
-  for (int p = 0; p < TPS; ++p) {
-    const int ls = p * SPP + t / TPS;
-    const int q = t % TPS;
-    const long long s = s0 + ls;
-    float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    if (s < S) {
-      const float* sg = a.seg + s * 6;
-      const SegCorner sc = segment_corners(__ldg(sg), __ldg(sg + 1), __ldg(sg + 2), __ldg(sg + 3), __ldg(sg + 4),
-                                           __ldg(sg + 5), a.nvx, a.nvy, a.nvz);
-      uint4 w[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-        w[j] = __ldg(reinterpret_cast<const uint4*>(a.grid16 + corner_row(sc, j, a.nvx, a.nvy) * C) + q);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        float g[8];
-        unpack8<BF16>(w[j], g);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) f[k] = fmaf(sc.w[j], g[k], f[k]);
-      }
-    }
-    uint4 o;
-    o.x = tc::pack2<BF16>(f[0], f[1]);
-    o.y = tc::pack2<BF16>(f[2], f[3]);
-    o.z = tc::pack2<BF16>(f[4], f[5]);
-    o.w = tc::pack2<BF16>(f[6], f[7]);
-    *reinterpret_cast<uint4*>(sA + tc::kmajor_offset(ls, 8 * q, C)) = o;
   }
 }
 
@@ -294,21 +356,52 @@ __device__ __forceinline__ void acc_row4(uint32_t taddr, int n, float* v) {
   }
 }
 
+// Adds n (a multiple of 4) values at p (16-byte aligned) to v.
+template <int n>
+__device__ __forceinline__ void add_row(float* v, const float* p) {
+#pragma unroll
+  for (int i = 0; i < n; i += 4) {
+    const float4 b = *reinterpret_cast<const float4*>(p + i);
+    const float2 x = f32x2_get(add_f32x2(f32x2(v[i], v[i + 1]), f32x2(b.x, b.y)));
+    const float2 y = f32x2_get(add_f32x2(f32x2(v[i + 2], v[i + 3]), f32x2(b.z, b.w)));
+    v[i] = x.x;
+    v[i + 1] = x.y;
+    v[i + 2] = y.x;
+    v[i + 3] = y.y;
+  }
+}
+
+// 16-bit pair of max(a, 0), max(b, 0) (NaN gives 0, like fmaxf): rounding is
+// monotone, so the maximum is taken on the rounded pair, one instruction.
+template <int BF16>
+__device__ __forceinline__ uint32_t pack2_relu(float a, float b) {
+  uint32_t r = tc::pack2<BF16>(a, b);
+  if (BF16)
+    asm("max.bf16x2 %0, %0, %1;" : "+r"(r) : "r"(0u));
+  else
+    asm("max.f16x2 %0, %0, %1;" : "+r"(r) : "r"(0u));
+  return r;
+}
+
 // Writes EPI_COLS values (columns c0.. of the next layer's input) of row t,
-// as TERMS operand terms (a_term's layout).
-template <int BF16, int TERMS>
-__device__ __forceinline__ void store_row(uint8_t* sA, uint32_t tstride, int t, int c0, int K, const float* v) {
+// through ReLU if RELU, as TERMS operand terms (a_term's layout).
+template <int BF16, int TERMS, bool RELU>
+__device__ __forceinline__ void store_row(uint8_t* sA, uint32_t tstride, int t, int c0, int K, float* v) {
 #pragma unroll
   for (int j = 0; j < EPI_COLS<TERMS> / 8; ++j) {
     if constexpr (TERMS == 1) {
-      uint4 w;
-      w.x = tc::pack2<BF16>(v[8 * j + 0], v[8 * j + 1]);
-      w.y = tc::pack2<BF16>(v[8 * j + 2], v[8 * j + 3]);
-      w.z = tc::pack2<BF16>(v[8 * j + 4], v[8 * j + 5]);
-      w.w = tc::pack2<BF16>(v[8 * j + 6], v[8 * j + 7]);
-      *reinterpret_cast<uint4*>(a_term<1>(sA, tstride, t, c0 + 8 * j, K, 0)) = w;
+      uint32_t w[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        w[i] = RELU ? pack2_relu<BF16>(v[8 * j + 2 * i], v[8 * j + 2 * i + 1])
+                    : tc::pack2<BF16>(v[8 * j + 2 * i], v[8 * j + 2 * i + 1]);
+      *reinterpret_cast<uint4*>(a_term<1>(sA, tstride, t, c0 + 8 * j, K, 0)) = make_uint4(w[0], w[1], w[2], w[3]);
     } else {
       uint32_t x[TERMS], y[TERMS], z[TERMS], u[TERMS];
+      if (RELU) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[8 * j + i] = fmaxf(v[8 * j + i], 0.f);
+      }
       tc::split_pair<TERMS>(v[8 * j + 0], v[8 * j + 1], x);
       tc::split_pair<TERMS>(v[8 * j + 2], v[8 * j + 3], y);
       tc::split_pair<TERMS>(v[8 * j + 4], v[8 * j + 5], z);
@@ -333,14 +426,15 @@ __device__ __forceinline__ void sync_for_mma() {
 // 8 CTAs per SM for the single-term forms (TMEM), 4 for the DIVeR32 split
 // form (shared memory; its two-pass gather would otherwise take 3).
 template <int C, int W, int D1, int BF16, int NCOLS, int TERMS>
-__global__ void __launch_bounds__(128, TERMS == 1 ? 8 : ((C == 32 && W == 32) ? 4 : 1)) decode_fwd_tc(const TcArgs a) {
+__global__ void __launch_bounds__(128, TERMS == 1 ? (W == 32 ? 8 : 4) : ((C == 32 && W == 32) ? 4 : 1)) decode_fwd_tc(const TcArgs a) {
   constexpr int KMAX = C > W ? C : W;
   constexpr uint32_t TSTRIDE = 128 * KMAX * 2;  // bytes between the A tile's terms
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sB = smem;
   float* sBias = reinterpret_cast<float*>(smem + TERMS * a.wbytes);
   uint8_t* sA = reinterpret_cast<uint8_t*>(sBias + a.nbias);
-  uint64_t* bar = reinterpret_cast<uint64_t*>(sA + TERMS * TSTRIDE);
+  float* coef = reinterpret_cast<float*>(sA + TERMS * TSTRIDE);
+  uint64_t* bar = reinterpret_cast<uint64_t*>(coef + (TERMS == 1 ? 128 * COEF : 0));
   uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 1);
   const int t = threadIdx.x, warp = t >> 5;
   if constexpr (TERMS == 1) {
@@ -359,7 +453,9 @@ __global__ void __launch_bounds__(128, TERMS == 1 ? 8 : ((C == 32 && W == 32) ? 
       }
     }
   }
-  for (int i = t; i < a.nbias; i += 128) sBias[i] = __ldg(a.bias + i);
+#pragma unroll 1
+  for (int l = 0; l < D1 + 3; ++l)
+    for (int i = t; i < a.L[l].N; i += 128) sBias[a.L[l].s_bias + i] = __ldg(a.bias + a.L[l].bias_off + i);
   if (t == 0) {
     tc::mbar_init(bar, 1);
     tc::fence_mbar_init();
@@ -375,97 +471,90 @@ __global__ void __launch_bounds__(128, TERMS == 1 ? 8 : ((C == 32 && W == 32) ? 
   const uint32_t wterm = (uint32_t)a.wbytes;
   uint32_t phase = 0;
   bool ok = true;
+  const bool saving = a.save != nullptr;
   const long long S = segment_total(a.S, a.S_dev);
   const long long tiles = (S + 127) / 128;
   for (long long tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
     const long long s0 = tile * 128;
     const long long s = s0 + t;
     const bool valid = s < S;
-    uint8_t* rec = a.save ? a.save + tile * (long long)a.save_bytes : nullptr;
-#define DV_SAVE(l) (rec ? rec + a.save_off[l] : nullptr)
+    uint8_t* rec = saving ? a.save + tile * (long long)a.save_bytes : nullptr;
+    // A layer's MMAs, then its wait; a wait that gave up is seen by all at the
+    // tile's end.  While the layer's input is being copied out nobody may
+    // overwrite it, which takes a barrier.
+#define DV_LAYER(l)                                                                                              \
+  do {                                                                                                           \
+    ok &= tc_layer<BF16, TERMS>(a.L[l], sB, wterm, sA, TSTRIDE, tmem, bar, phase, rec ? rec + a.save_off[l] : nullptr); \
+    if (saving) __syncthreads();                                                                                 \
+  } while (0)
     if constexpr (TERMS > 1) {
-      gather_tile_lp_x2<C, TERMS>(a, S, s0, sA, TSTRIDE);
+      gather_tile_split<C, TERMS>(a, S, s0, sA, TSTRIDE);
     } else {
+      constexpr int U = W == 32 ? 1 : 2;  // 8 CTAs per SM leave 64 registers a thread, 4 leave 128
       if (a.grid16)
-        gather_tile_16<C, BF16>(a, S, s0, sA);
+        gather_tile<C, BF16, true, U>(a, S, s0, sA, coef);
       else
-        gather_tile_lp<C, BF16, TERMS>(a, S, s0, sA, TSTRIDE);
+        gather_tile<C, BF16, false, U>(a, S, s0, sA, coef);
     }
     sync_for_mma();
-    float v[32];
+    constexpr int EC = EPI_COLS<TERMS>;
+    float v[EC];
     // mlp1 hidden layers: D = relu(A W^T + b)
 #pragma unroll 1
-    for (int l = 0; l < D1 && ok; ++l) {
-      ok = tc_layer<BF16, TERMS>(a.L[l], sB, wterm, sA, TSTRIDE, tmem, bar, phase, DV_SAVE(l));
-      ok = __syncthreads_and(ok);
-      if (!ok) break;
+    for (int l = 0; l < D1; ++l) {
+      DV_LAYER(l);
 #pragma unroll
-      for (int c0 = 0; c0 < W; c0 += EPI_COLS<TERMS>) {
+      for (int c0 = 0; c0 < W; c0 += EC) {
         acc_row<TERMS>(trow + c0, a.L[l].N, v);
-#pragma unroll
-        for (int i = 0; i < EPI_COLS<TERMS>; ++i) v[i] = fmaxf(v[i] + sBias[a.L[l].bias_off + c0 + i], 0.f);
-        store_row<BF16, TERMS>(sA, TSTRIDE, t, c0, W, v);
+        add_row<EC>(v, sBias + a.L[l].s_bias + c0);
+        store_row<BF16, TERMS, true>(sA, TSTRIDE, t, c0, W, v);
       }
       sync_for_mma();
     }
-    if (!ok) break;
     // mlp1 output: columns 0..W-1 hidden (no activation), column W sigma
-    ok = __syncthreads_and(tc_layer<BF16, TERMS>(a.L[D1], sB, wterm, sA, TSTRIDE, tmem, bar, phase, DV_SAVE(D1)));
-    if (!ok) break;
+    DV_LAYER(D1);
     float sigma;
     {
       float sv[4];
       acc_row4<TERMS>(trow + W, a.L[D1].N, sv);
-      sigma = sv[0] + sBias[a.L[D1].bias_off + W];
+      sigma = sv[0] + sBias[a.L[D1].s_bias + W];
     }
 #pragma unroll
-    for (int c0 = 0; c0 < W; c0 += EPI_COLS<TERMS>) {
+    for (int c0 = 0; c0 < W; c0 += EC) {
       acc_row<TERMS>(trow + c0, a.L[D1].N, v);
-#pragma unroll
-      for (int i = 0; i < EPI_COLS<TERMS>; ++i) v[i] += sBias[a.L[D1].bias_off + c0 + i];
-      store_row<BF16, TERMS>(sA, TSTRIDE, t, c0, W, v);
+      add_row<EC>(v, sBias + a.L[D1].s_bias + c0);
+      store_row<BF16, TERMS, false>(sA, TSTRIDE, t, c0, W, v);
     }
     sync_for_mma();
     // mlp2 first layer: relu(hidden W^T + per-ray (bias + PE term))
-    ok = __syncthreads_and(
-        tc_layer<BF16, TERMS>(a.L[D1 + 1], sB, wterm, sA, TSTRIDE, tmem, bar, phase, DV_SAVE(D1 + 1)));
-    if (!ok) break;
+    DV_LAYER(D1 + 1);
     {
       const int ray = valid ? __ldg(a.seg_ray + s) : 0;
-      const float4* po = reinterpret_cast<const float4*>(a.pe_out + (long long)ray * W);
+      const float* po = a.pe_out + (long long)ray * W;
 #pragma unroll
-      for (int c0 = 0; c0 < W; c0 += EPI_COLS<TERMS>) {
+      for (int c0 = 0; c0 < W; c0 += EC) {
         acc_row<TERMS>(trow + c0, a.L[D1 + 1].N, v);
-#pragma unroll
-        for (int i = 0; i < EPI_COLS<TERMS>; i += 4) {
-          const float4 p = __ldg(po + (c0 + i) / 4);
-          v[i] = fmaxf(v[i] + p.x, 0.f);
-          v[i + 1] = fmaxf(v[i + 1] + p.y, 0.f);
-          v[i + 2] = fmaxf(v[i + 2] + p.z, 0.f);
-          v[i + 3] = fmaxf(v[i + 3] + p.w, 0.f);
-        }
-        store_row<BF16, TERMS>(sA, TSTRIDE, t, c0, W, v);
+        add_row<EC>(v, po + c0);
+        store_row<BF16, TERMS, true>(sA, TSTRIDE, t, c0, W, v);
       }
     }
     sync_for_mma();
     // mlp2 output: 3 logits -> sigmoid
-    ok = __syncthreads_and(
-        tc_layer<BF16, TERMS>(a.L[D1 + 2], sB, wterm, sA, TSTRIDE, tmem, bar, phase, DV_SAVE(D1 + 2)));
-#undef DV_SAVE
-    if (!ok) break;
+    DV_LAYER(D1 + 2);
+#undef DV_LAYER
     {
       float o[4];
       acc_row4<TERMS>(trow, a.L[D1 + 2].N, o);
-      const int bo = a.L[D1 + 2].bias_off;
-      if (valid)
-        a.out4[s] = make_float4(sigma, sigmoidf_acc(o[0] + sBias[bo]), sigmoidf_acc(o[1] + sBias[bo + 1]),
-                                sigmoidf_acc(o[2] + sBias[bo + 2]));
+      const float* bo = sBias + a.L[D1 + 2].s_bias;
+      if (valid && ok)
+        a.out4[s] = make_float4(sigma, sigmoidf_acc(o[0] + bo[0]), sigmoidf_acc(o[1] + bo[1]),
+                                sigmoidf_acc(o[2] + bo[2]));
     }
     tc::fence_before_sync();
-    __syncthreads();  // the next gather overwrites A
+    ok = __syncthreads_and(ok);  // the next gather overwrites A
   }
   if (!ok && t == 0 && a.err) atomicExch(a.err, 1);
-  if (a.save != nullptr && t == 0) tc::bulk_wait_all();
+  if (saving && t == 0) tc::bulk_wait_all();
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
@@ -480,7 +569,8 @@ int launch_decode_fwd_tc(const TcArgs& a, cudaStream_t st) {
   // split form: two column blocks of the widest N
   constexpr int NCOLS = TERMS > 1 ? (W == 32 ? 128 : 256) : (W == 32 ? 64 : 128);
   constexpr int KMAX = C > W ? C : W;
-  const size_t smem = (size_t)TERMS * a.wbytes + (size_t)a.nbias * 4 + (size_t)TERMS * 128 * KMAX * 2 + 16;
+  const size_t smem = (size_t)TERMS * a.wbytes + (size_t)a.nbias * 4 + (size_t)TERMS * 128 * KMAX * 2 +
+                      (TERMS == 1 ? 128 * COEF * 4 : 0) + 16;
   auto k = decode_fwd_tc<C, W, D1, BF16, NCOLS, TERMS>;
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return DV_ERR_CUDA;
   int dev = 0, sms = 0;
@@ -589,6 +679,12 @@ static int decode_fwd_tc_args(TcArgs& a, int kind, int channels, int terms, cons
     DV_CHECK(L.K % 16 == 0 && L.N % 16 == 0 && L.N >= 16 && L.N <= 256 && L.b_off % 16 == 0, DV_ERR_ARG);
     DV_CHECK((long long)L.b_off + (long long)L.N * L.K * 2 <= wbytes && L.bias_off + L.N <= nbias, DV_ERR_ARG);
     DV_CHECK(L.N <= (W == 32 ? 64 : 128), DV_ERR_ARG);
+  }
+  // biases layer by layer in shared memory (N is a multiple of 16, so every layer's are 16-byte aligned)
+  a.nbias = 0;
+  for (int l = 0; l < n_layers; ++l) {
+    a.L[l].s_bias = a.nbias;
+    a.nbias += a.L[l].N;
   }
   // the split form's images regrouped in shared memory, layer by layer
   {
