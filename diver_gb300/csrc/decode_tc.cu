@@ -165,7 +165,7 @@ __device__ __forceinline__ void put_corners(float* coef, const Corners& c) {
 // every corner row (4 channels of the FP32 grid, or 8 of its 16-bit copy) in
 // FP32, and writing the feature row's 16-bit operand.  U passes' loads are in
 // flight per thread.
-template <int C, int BF16, bool G16, int U>
+template <int C, int BF16, bool G16, bool SWZ, int U>
 __device__ __forceinline__ void gather_tile(const TcArgs& a, long long S, long long s0, uint8_t* sA, float* coef) {
   constexpr int CH = G16 ? 8 : 4, TPS = C / CH, SPP = 32 / TPS, BYTES = C * (G16 ? 2 : 4);
   const int lane = threadIdx.x & 31, q = lane % TPS, first = (threadIdx.x & ~31) + lane / TPS;
@@ -209,7 +209,7 @@ __device__ __forceinline__ void gather_tile(const TcArgs& a, long long S, long l
         const float2 r = f32x2_get(f[k]);
         o[k] = in ? tc::pack2<BF16>(r.x, r.y) : 0u;
       }
-      uint8_t* dst = sA + tc::kmajor_offset(ls, CH * q, C);
+      uint8_t* dst = sA + (SWZ ? tc::swizzled_offset<C>(ls, CH * q) : tc::kmajor_offset(ls, CH * q, C));
       if (G16)
         *reinterpret_cast<uint4*>(dst) = make_uint4(o[0], o[1], o[CH / 2 - 2], o[CH / 2 - 1]);
       else
@@ -319,6 +319,32 @@ __device__ __forceinline__ bool tc_layer(const TcLayer& L, const uint8_t* sB, ui
   return done;
 }
 
+// A layer of the single-term form without a save record: A is the swizzled
+// feature tile in shared memory (FIRST) or the activations in TMEM columns
+// from `acol`, B as above.
+template <int K, bool FIRST>
+__device__ __forceinline__ bool tc_layer_ts(const TcLayer& L, const uint8_t* sB, const uint8_t* sA, uint32_t tmem,
+                                            uint32_t acol, int bf16, uint64_t* bar, uint32_t& phase) {
+  if (threadIdx.x == 0) {
+    tc::fence_after_sync();
+    const uint32_t idesc = tc::idesc_f16(128, L.N, bf16);
+    const uint64_t b0 = tc::smem_desc(tc::smem_u32(sB + L.b_off), 128, (K / 8) * 128);
+    const uint64_t a0 = tc::swizzled_desc<K>(tc::smem_u32(sA));
+#pragma unroll
+    for (int k = 0; k < K / 16; ++k) {
+      if (FIRST)
+        tc::mma_f16(tmem, tc::desc_plus(a0, k * 32), tc::desc_plus(b0, k * 256), idesc, k > 0 ? 1u : 0u);
+      else
+        tc::mma_f16_ts(tmem, tmem + acol + 8 * k, tc::desc_plus(b0, k * 256), idesc, k > 0 ? 1u : 0u);
+    }
+    tc::mma_commit(bar);
+  }
+  const bool done = tc::mbar_wait_bounded(bar, phase);
+  phase ^= 1u;
+  tc::fence_after_sync();
+  return done;
+}
+
 // Epilogue columns per pass: 32, or 16 for the split form, whose rows are the
 // sum of two TMEM column blocks (registers: its kernel runs 4 CTAs per SM).
 template <int TERMS>
@@ -413,6 +439,22 @@ __device__ __forceinline__ void store_row(uint8_t* sA, uint32_t tstride, int t, 
   }
 }
 
+// The same 32 values of row t into TMEM columns (two per column).
+template <int BF16, bool RELU>
+__device__ __forceinline__ void put_row_ts(uint32_t taddr, const float* v) {
+  uint32_t w[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i)
+    w[i] = RELU ? pack2_relu<BF16>(v[2 * i], v[2 * i + 1]) : tc::pack2<BF16>(v[2 * i], v[2 * i + 1]);
+  tc::st_32x32b_x16(taddr, w);
+}
+
+__device__ __forceinline__ void sync_for_mma_ts() {
+  tc::st_wait();
+  tc::fence_before_sync();
+  __syncthreads();
+}
+
 __device__ __forceinline__ void sync_for_mma() {
   tc::fence_before_sync();
   tc::fence_async_smem();
@@ -425,15 +467,15 @@ __device__ __forceinline__ void sync_for_mma() {
 // Registers per thread are capped to the residency the other resources allow:
 // 8 CTAs per SM for the single-term forms (TMEM), 4 for the DIVeR32 split
 // form (shared memory; its two-pass gather would otherwise take 3).
-template <int C, int W, int D1, int BF16, int NCOLS, int TERMS>
+template <int C, int W, int D1, int BF16, int NCOLS, int TERMS, bool TS>
 __global__ void __launch_bounds__(128, TERMS == 1 ? (W == 32 ? 8 : 4) : ((C == 32 && W == 32) ? 4 : 1)) decode_fwd_tc(const TcArgs a) {
   constexpr int KMAX = C > W ? C : W;
   constexpr uint32_t TSTRIDE = 128 * KMAX * 2;  // bytes between the A tile's terms
   extern __shared__ __align__(1024) uint8_t smem[];
-  uint8_t* sB = smem;
-  float* sBias = reinterpret_cast<float*>(smem + TERMS * a.wbytes);
-  uint8_t* sA = reinterpret_cast<uint8_t*>(sBias + a.nbias);
-  float* coef = reinterpret_cast<float*>(sA + TERMS * TSTRIDE);
+  uint8_t* sA = smem;  // on a 1024-byte boundary (its swizzle)
+  uint8_t* sB = smem + TERMS * TSTRIDE;
+  float* sBias = reinterpret_cast<float*>(sB + TERMS * a.wbytes);
+  float* coef = sBias + a.nbias;
   uint64_t* bar = reinterpret_cast<uint64_t*>(coef + (TERMS == 1 ? 128 * COEF : 0));
   uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 1);
   const int t = threadIdx.x, warp = t >> 5;
@@ -479,69 +521,74 @@ __global__ void __launch_bounds__(128, TERMS == 1 ? (W == 32 ? 8 : 4) : ((C == 3
     const long long s = s0 + t;
     const bool valid = s < S;
     uint8_t* rec = saving ? a.save + tile * (long long)a.save_bytes : nullptr;
+    constexpr int EC = EPI_COLS<TERMS>;
+    constexpr uint32_t ACOL = NCOLS - W / 2;  // TS: the activations' columns, behind the widest layer's output
+    float v[EC];
     // A layer's MMAs, then its wait; a wait that gave up is seen by all at the
     // tile's end.  While the layer's input is being copied out nobody may
     // overwrite it, which takes a barrier.
-#define DV_LAYER(l)                                                                                              \
+#define DV_LAYER(l, first)                                                                                       \
   do {                                                                                                           \
-    ok &= tc_layer<BF16, TERMS>(a.L[l], sB, wterm, sA, TSTRIDE, tmem, bar, phase, rec ? rec + a.save_off[l] : nullptr); \
-    if (saving) __syncthreads();                                                                                 \
+    if constexpr (TS) {                                                                                          \
+      ok &= tc_layer_ts<first ? C : W, first>(a.L[l], sB, sA, tmem, ACOL, BF16, bar, phase);                     \
+    } else {                                                                                                     \
+      ok &= tc_layer<BF16, TERMS>(a.L[l], sB, wterm, sA, TSTRIDE, tmem, bar, phase,                              \
+                                  rec ? rec + a.save_off[l] : nullptr);                                          \
+      if (saving) __syncthreads();                                                                               \
+    }                                                                                                            \
+  } while (0)
+    // Its output plus `bias`, through ReLU if asked, as the next layer's input.
+#define DV_EPILOGUE(l, bias, relu)                                     \
+  do {                                                                 \
+    _Pragma("unroll") for (int c0 = 0; c0 < W; c0 += EC) {             \
+      acc_row<TERMS>(trow + c0, a.L[l].N, v);                          \
+      add_row<EC>(v, (bias) + c0);                                     \
+      if constexpr (TS)                                                \
+        put_row_ts<BF16, relu>(trow + ACOL + c0 / 2, v);               \
+      else                                                             \
+        store_row<BF16, TERMS, relu>(sA, TSTRIDE, t, c0, W, v);        \
+    }                                                                  \
+    if constexpr (TS)                                                  \
+      sync_for_mma_ts();                                               \
+    else                                                               \
+      sync_for_mma();                                                  \
   } while (0)
     if constexpr (TERMS > 1) {
       gather_tile_split<C, TERMS>(a, S, s0, sA, TSTRIDE);
     } else {
       constexpr int U = W == 32 ? 1 : 2;  // 8 CTAs per SM leave 64 registers a thread, 4 leave 128
       if (a.grid16)
-        gather_tile<C, BF16, true, U>(a, S, s0, sA, coef);
+        gather_tile<C, BF16, true, TS, U>(a, S, s0, sA, coef);
       else
-        gather_tile<C, BF16, false, U>(a, S, s0, sA, coef);
+        gather_tile<C, BF16, false, TS, U>(a, S, s0, sA, coef);
     }
     sync_for_mma();
-    constexpr int EC = EPI_COLS<TERMS>;
-    float v[EC];
     // mlp1 hidden layers: D = relu(A W^T + b)
-#pragma unroll 1
-    for (int l = 0; l < D1; ++l) {
-      DV_LAYER(l);
-#pragma unroll
-      for (int c0 = 0; c0 < W; c0 += EC) {
-        acc_row<TERMS>(trow + c0, a.L[l].N, v);
-        add_row<EC>(v, sBias + a.L[l].s_bias + c0);
-        store_row<BF16, TERMS, true>(sA, TSTRIDE, t, c0, W, v);
-      }
-      sync_for_mma();
+    DV_LAYER(0, true);
+    DV_EPILOGUE(0, sBias + a.L[0].s_bias, true);
+    if constexpr (D1 == 2) {
+      DV_LAYER(1, false);
+      DV_EPILOGUE(1, sBias + a.L[1].s_bias, true);
     }
     // mlp1 output: columns 0..W-1 hidden (no activation), column W sigma
-    DV_LAYER(D1);
+    DV_LAYER(D1, false);
     float sigma;
     {
       float sv[4];
       acc_row4<TERMS>(trow + W, a.L[D1].N, sv);
       sigma = sv[0] + sBias[a.L[D1].s_bias + W];
     }
-#pragma unroll
-    for (int c0 = 0; c0 < W; c0 += EC) {
-      acc_row<TERMS>(trow + c0, a.L[D1].N, v);
-      add_row<EC>(v, sBias + a.L[D1].s_bias + c0);
-      store_row<BF16, TERMS, false>(sA, TSTRIDE, t, c0, W, v);
-    }
-    sync_for_mma();
+    DV_EPILOGUE(D1, sBias + a.L[D1].s_bias, false);
     // mlp2 first layer: relu(hidden W^T + per-ray (bias + PE term))
-    DV_LAYER(D1 + 1);
+    DV_LAYER(D1 + 1, false);
     {
-      const int ray = valid ? __ldg(a.seg_ray + s) : 0;
-      const float* po = a.pe_out + (long long)ray * W;
-#pragma unroll
-      for (int c0 = 0; c0 < W; c0 += EC) {
-        acc_row<TERMS>(trow + c0, a.L[D1 + 1].N, v);
-        add_row<EC>(v, po + c0);
-        store_row<BF16, TERMS, true>(sA, TSTRIDE, t, c0, W, v);
-      }
+      const float* po = a.pe_out + (long long)(valid ? __ldg(a.seg_ray + s) : 0) * W;
+      DV_EPILOGUE(D1 + 1, po, true);
     }
-    sync_for_mma();
     // mlp2 output: 3 logits -> sigmoid
-    DV_LAYER(D1 + 2);
+    DV_LAYER(D1 + 2, false);
 #undef DV_LAYER
+#undef DV_EPILOGUE
     {
       float o[4];
       acc_row4<TERMS>(trow, a.L[D1 + 2].N, o);
@@ -564,14 +611,14 @@ __global__ void __launch_bounds__(128, TERMS == 1 ? (W == 32 ? 8 : 4) : ((C == 3
 // The persistent grid holds as many CTAs per SM as registers, shared memory
 // and TMEM (512 columns) allow together (the occupancy API under-reports
 // kernels that allocate TMEM).
-template <int C, int W, int D1, int BF16, int TERMS = 1>
-int launch_decode_fwd_tc(const TcArgs& a, cudaStream_t st) {
+template <int C, int W, int D1, int BF16, int TERMS, bool TS>
+int launch_decode_fwd_tc_as(const TcArgs& a, cudaStream_t st) {
   // split form: two column blocks of the widest N
   constexpr int NCOLS = TERMS > 1 ? (W == 32 ? 128 : 256) : (W == 32 ? 64 : 128);
   constexpr int KMAX = C > W ? C : W;
   const size_t smem = (size_t)TERMS * a.wbytes + (size_t)a.nbias * 4 + (size_t)TERMS * 128 * KMAX * 2 +
                       (TERMS == 1 ? 128 * COEF * 4 : 0) + 16;
-  auto k = decode_fwd_tc<C, W, D1, BF16, NCOLS, TERMS>;
+  auto k = decode_fwd_tc<C, W, D1, BF16, NCOLS, TERMS, TS>;
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return DV_ERR_CUDA;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
@@ -589,6 +636,19 @@ int launch_decode_fwd_tc(const TcArgs& a, cudaStream_t st) {
   k<<<(unsigned)grid, 128, res.dyn_smem, st>>>(a);
   DV_TRY_LAUNCH();
   return DV_OK;
+}
+
+// Single-term forms without a save record keep the activations in TMEM; with
+// one, every layer's input has to be in shared memory for its bulk copy, and
+// the split form's three terms do not fit beside its two column blocks.
+template <int C, int W, int D1, int BF16, int TERMS = 1>
+int launch_decode_fwd_tc(const TcArgs& a, cudaStream_t st) {
+  if constexpr (TERMS == 1) {
+    bool fits = a.save == nullptr;
+    for (int l = 0; l < D1 + 3; ++l) fits = fits && a.L[l].N <= W + 16;  // outputs in front of the activations' columns
+    if (fits) return launch_decode_fwd_tc_as<C, W, D1, BF16, 1, true>(a, st);
+  }
+  return launch_decode_fwd_tc_as<C, W, D1, BF16, TERMS, false>(a, st);
 }
 
 // Exercises the bounded completion wait that every tensor-core kernel uses

@@ -34,6 +34,23 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
   return d;  // base offset 0, LBO mode 0, no swizzle
 }
 
+// Byte offset of element (r, k) in a K-major tile with one swizzle atom of K
+// columns per row (K = 32: 64-byte swizzle, K = 64: 128-byte swizzle): rows are
+// contiguous, and the 16-byte chunks of a row are permuted by the row so that
+// chunk c of 8 rows, and the chunks of one row, fall into different banks.
+template <int K>
+__host__ __device__ __forceinline__ uint32_t swizzled_offset(int r, int k) {
+  static_assert(K == 32 || K == 64, "a row is one swizzle atom");
+  const int x = K == 64 ? (r & 7) : ((r >> 1) & 3);
+  return (uint32_t)(r * (2 * K) + (((k >> 3) ^ x) << 4) + (k & 7) * 2);
+}
+
+// Its descriptor (the tile on a 1024-byte boundary): 8-row groups 16 K bytes apart.
+template <int K>
+__device__ __forceinline__ uint64_t swizzled_desc(uint32_t addr) {
+  return smem_desc(addr, 16, 16 * K) | ((uint64_t)(K == 64 ? 2 : 4) << 61);
+}
+
 // The descriptor of an operand `bytes` further on (a multiple of 16): the
 // start address is the low field (address / 16, 14 bits), and shared-memory
 // addresses stay below 256 KiB, so the add never carries out of it.
@@ -127,11 +144,32 @@ __device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64
       : "memory");
 }
 
+// The same with A in TMEM: rows in lanes, two consecutive 16-bit K elements per
+// 32-bit column (8 columns per instruction).
+__device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
+                                           uint32_t accumulate) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
 // Arrives on the mbarrier once all previously issued MMAs of this thread complete.
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                : "memory");
 }
+
+// 32 lanes x 16 columns: this thread's row (lane base + laneid) gets 16 words.
+__device__ __forceinline__ void st_32x32b_x16(uint32_t taddr, const uint32_t* r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+__device__ __forceinline__ void st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 __device__ __forceinline__ void ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
