@@ -17,7 +17,11 @@
 // taken on rounded pairs.  Measured against one thread per 8 channels doing
 // all of it: 800x800 frame of the 256^3 scene, BF16 10.5 -> 8.8 ms; DIVeR64 over
 // 64 channels, 399x401, FP16 5.2 -> 3.8 ms; split, 65,792 rays of the wide grid
-// 647 -> 509 us.
+// 647 -> 509 us.  Then, single-term forms without a save record: activations
+// in TMEM and a swizzled feature tile (LSU wavefronts 2244 -> 1670 per tile) and
+// tiles taken dynamically: frame 8.8 -> 6.2 ms, DIVeR64 view 3.8 -> 3.1 ms.
+// What is left of a frame's tile (8 CTAs per SM): half of its time gathers at
+// four fifths of the LSU pipe, a fifth waits for the five MMA chains.
 // The decoder's weights (all layers, B operands in the same K-major layout)
 // and biases stay in shared memory for the CTA's lifetime; the grid is
 // persistent over tiles and sized so TMEM never oversubscribes.
@@ -60,6 +64,7 @@ struct TcArgs {
   int nbias;   // biases in shared memory
   TcLayer L[TC_MAX_LAYERS];
   int* err;    // set to 1 if an MMA completion wait timed out
+  int steal;   // one CTA was launched per tile, and running ones take over those not yet started
   uint8_t* save;       // optional: every layer's input tile, per 128-segment tile (training)
   int save_off[TC_MAX_LAYERS];  // byte offset of layer l's input tile inside a tile's record
   int save_bytes;      // bytes per tile record (sum of 256 * K over the layers)
@@ -87,12 +92,24 @@ struct Corners {
   uint32_t row, dx, dy, dz;
 };
 
-__device__ __forceinline__ Corners corners_of(const TcArgs& a, long long S, long long s) {
-  Corners c{};
+// This thread's segment record.
+struct Seg6 {
+  float p[6];
+};
+
+__device__ __forceinline__ Seg6 load_seg(const TcArgs& a, long long S, long long s) {
+  Seg6 r{};
   if (s < S) {
-    const float* sg = a.seg + s * 6;
-    const SegCorner sc = segment_corners(__ldg(sg), __ldg(sg + 1), __ldg(sg + 2), __ldg(sg + 3), __ldg(sg + 4),
-                                         __ldg(sg + 5), a.nvx, a.nvy, a.nvz);
+#pragma unroll
+    for (int i = 0; i < 6; ++i) r.p[i] = __ldg(a.seg + s * 6 + i);
+  }
+  return r;
+}
+
+__device__ __forceinline__ Corners corners_of(const TcArgs& a, bool valid, const Seg6& g) {
+  Corners c{};
+  if (valid) {
+    const SegCorner sc = segment_corners(g.p[0], g.p[1], g.p[2], g.p[3], g.p[4], g.p[5], a.nvx, a.nvy, a.nvz);
 #pragma unroll
     for (int j = 0; j < 8; ++j) c.w[j] = sc.w[j];
     c.row = ((uint32_t)sc.z * a.nvy + sc.y) * a.nvx + sc.x;
@@ -166,10 +183,10 @@ __device__ __forceinline__ void put_corners(float* coef, const Corners& c) {
 // FP32, and writing the feature row's 16-bit operand.  U passes' loads are in
 // flight per thread.
 template <int C, int BF16, bool G16, bool SWZ, int U>
-__device__ __forceinline__ void gather_tile(const TcArgs& a, long long S, long long s0, uint8_t* sA, float* coef) {
+__device__ __forceinline__ void gather_tile(const TcArgs& a, long long S, long long s0, const Seg6& g, uint8_t* sA, float* coef) {
   constexpr int CH = G16 ? 8 : 4, TPS = C / CH, SPP = 32 / TPS, BYTES = C * (G16 ? 2 : 4);
   const int lane = threadIdx.x & 31, q = lane % TPS, first = (threadIdx.x & ~31) + lane / TPS;
-  put_corners(coef, corners_of(a, S, s0 + threadIdx.x));
+  put_corners(coef, corners_of(a, s0 + threadIdx.x < S, g));
   const uint8_t* grid = (G16 ? reinterpret_cast<const uint8_t*>(a.grid16) : reinterpret_cast<const uint8_t*>(a.grid)) + 16 * q;
 #pragma unroll 1
   for (int p = 0; p < TPS; p += U) {
@@ -224,12 +241,12 @@ __device__ __forceinline__ void gather_tile(const TcArgs& a, long long S, long l
 // residency, and the corners go from lane to lane by shuffles, as shared
 // memory is what is short.
 template <int C, int TERMS>
-__device__ __forceinline__ void gather_tile_split(const TcArgs& a, long long S, long long s0, uint8_t* sA,
-                                                  uint32_t tstride) {
+__device__ __forceinline__ void gather_tile_split(const TcArgs& a, long long S, long long s0, const Seg6& g,
+                                                  uint8_t* sA, uint32_t tstride) {
   constexpr int TPS = C / 4, SPP = 32 / TPS;
   static_assert(TPS % 2 == 0, "passes are taken in pairs");
   const int lane = threadIdx.x & 31, warp0 = threadIdx.x & ~31, q = lane % TPS;
-  const Corners c = corners_of(a, S, s0 + threadIdx.x);
+  const Corners c = corners_of(a, s0 + threadIdx.x < S, g);
   const uint8_t* grid = reinterpret_cast<const uint8_t*>(a.grid) + 16 * q;
   const uint32_t flags = (c.dx ? 1u : 0u) | (c.dy ? 2u : 0u) | (c.dz ? 4u : 0u);
 #pragma unroll 1
@@ -476,8 +493,10 @@ __global__ void __launch_bounds__(128, TERMS == 1 ? (W == 32 ? 8 : 4) : ((C == 3
   uint8_t* sB = smem + TERMS * TSTRIDE;
   float* sBias = reinterpret_cast<float*>(sB + TERMS * a.wbytes);
   float* coef = sBias + a.nbias;
-  uint64_t* bar = reinterpret_cast<uint64_t*>(coef + (TERMS == 1 ? 128 * COEF : 0));
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 1);
+  uint8_t* answer = reinterpret_cast<uint8_t*>(coef + (TERMS == 1 ? 128 * COEF : 0));  // 16 bytes
+  uint64_t* bar = reinterpret_cast<uint64_t*>(answer + 16);
+  uint64_t* bar_next = bar + 1;
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 2);
   const int t = threadIdx.x, warp = t >> 5;
   if constexpr (TERMS == 1) {
     for (int i = t; i < a.wbytes / 16; i += 128)
@@ -500,6 +519,7 @@ __global__ void __launch_bounds__(128, TERMS == 1 ? (W == 32 ? 8 : 4) : ((C == 3
     for (int i = t; i < a.L[l].N; i += 128) sBias[a.L[l].s_bias + i] = __ldg(a.bias + a.L[l].bias_off + i);
   if (t == 0) {
     tc::mbar_init(bar, 1);
+    tc::mbar_init(bar_next, 1);
     tc::fence_mbar_init();
   }
   if (warp == 0) {
@@ -516,9 +536,21 @@ __global__ void __launch_bounds__(128, TERMS == 1 ? (W == 32 ? 8 : 4) : ((C == 3
   const bool saving = a.save != nullptr;
   const long long S = segment_total(a.S, a.S_dev);
   const long long tiles = (S + 127) / 128;
-  for (long long tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+  // the next tile's segment is loaded while this one's last layer runs, where
+  // registers allow it (the single-term DIVeR32 forms have none to spare)
+  constexpr bool AHEAD = TERMS > 1 || W > 32;
+  Seg6 seg{};
+  if (AHEAD) seg = load_seg(a, S, (long long)blockIdx.x * 128 + t);
+  uint32_t phase_next = 0;
+  long long next = 0;
+  for (long long tile = blockIdx.x; tile < tiles && ok; tile = next) {
     const long long s0 = tile * 128;
     const long long s = s0 + t;
+    next = tile + gridDim.x;
+    if (a.steal && t == 0) {
+      tc::fence_async_smem();  // the last answer was read (the tile's end barrier) before this one is written
+      tc::clc_request(answer, bar_next);
+    }
     const bool valid = s < S;
     uint8_t* rec = saving ? a.save + tile * (long long)a.save_bytes : nullptr;
     constexpr int EC = EPI_COLS<TERMS>;
@@ -553,14 +585,15 @@ __global__ void __launch_bounds__(128, TERMS == 1 ? (W == 32 ? 8 : 4) : ((C == 3
     else                                                               \
       sync_for_mma();                                                  \
   } while (0)
+    if (!AHEAD) seg = load_seg(a, S, s);
     if constexpr (TERMS > 1) {
-      gather_tile_split<C, TERMS>(a, S, s0, sA, TSTRIDE);
+      gather_tile_split<C, TERMS>(a, S, s0, seg, sA, TSTRIDE);
     } else {
       constexpr int U = W == 32 ? 1 : 2;  // 8 CTAs per SM leave 64 registers a thread, 4 leave 128
       if (a.grid16)
-        gather_tile<C, BF16, true, TS, U>(a, S, s0, sA, coef);
+        gather_tile<C, BF16, true, TS, U>(a, S, s0, seg, sA, coef);
       else
-        gather_tile<C, BF16, false, TS, U>(a, S, s0, sA, coef);
+        gather_tile<C, BF16, false, TS, U>(a, S, s0, seg, sA, coef);
     }
     sync_for_mma();
     // mlp1 hidden layers: D = relu(A W^T + b)
@@ -571,6 +604,7 @@ __global__ void __launch_bounds__(128, TERMS == 1 ? (W == 32 ? 8 : 4) : ((C == 3
       DV_EPILOGUE(1, sBias + a.L[1].s_bias, true);
     }
     // mlp1 output: columns 0..W-1 hidden (no activation), column W sigma
+    const float* po = a.pe_out + (long long)(valid ? __ldg(a.seg_ray + s) : 0) * W;
     DV_LAYER(D1, false);
     float sigma;
     {
@@ -580,12 +614,17 @@ __global__ void __launch_bounds__(128, TERMS == 1 ? (W == 32 ? 8 : 4) : ((C == 3
     }
     DV_EPILOGUE(D1, sBias + a.L[D1].s_bias, false);
     // mlp2 first layer: relu(hidden W^T + per-ray (bias + PE term))
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(po));  // on its way while the layer runs
     DV_LAYER(D1 + 1, false);
-    {
-      const float* po = a.pe_out + (long long)(valid ? __ldg(a.seg_ray + s) : 0) * W;
-      DV_EPILOGUE(D1 + 1, po, true);
-    }
+    DV_EPILOGUE(D1 + 1, po, true);
     // mlp2 output: 3 logits -> sigmoid
+    if (a.steal) {
+      ok &= tc::mbar_wait_bounded(bar_next, phase_next);
+      phase_next ^= 1u;
+      const int got = ok ? tc::clc_answer(answer) : -1;
+      next = got < 0 ? tiles : got;
+    }
+    if (AHEAD) seg = load_seg(a, S, next * 128 + t);
     DV_LAYER(D1 + 2, false);
 #undef DV_LAYER
 #undef DV_EPILOGUE
@@ -612,12 +651,12 @@ __global__ void __launch_bounds__(128, TERMS == 1 ? (W == 32 ? 8 : 4) : ((C == 3
 // and TMEM (512 columns) allow together (the occupancy API under-reports
 // kernels that allocate TMEM).
 template <int C, int W, int D1, int BF16, int TERMS, bool TS>
-int launch_decode_fwd_tc_as(const TcArgs& a, cudaStream_t st) {
+int launch_decode_fwd_tc_as(TcArgs a, cudaStream_t st) {
   // split form: two column blocks of the widest N
   constexpr int NCOLS = TERMS > 1 ? (W == 32 ? 128 : 256) : (W == 32 ? 64 : 128);
   constexpr int KMAX = C > W ? C : W;
   const size_t smem = (size_t)TERMS * a.wbytes + (size_t)a.nbias * 4 + (size_t)TERMS * 128 * KMAX * 2 +
-                      (TERMS == 1 ? 128 * COEF * 4 : 0) + 16;
+                      (TERMS == 1 ? 128 * COEF * 4 : 0) + 48;
   auto k = decode_fwd_tc<C, W, D1, BF16, NCOLS, TERMS, TS>;
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return DV_ERR_CUDA;
   int dev = 0, sms = 0;
@@ -632,8 +671,14 @@ int launch_decode_fwd_tc_as(const TcArgs& a, cudaStream_t st) {
       return DV_ERR_CUDA;
   }
   const long long tiles = (a.S + 127) / 128;
-  const long long grid = std::min<long long>(tiles, (long long)sms * res.per_sm);
-  k<<<(unsigned)grid, 128, res.dyn_smem, st>>>(a);
+  const long long wave = (long long)sms * res.per_sm;
+  // With the count on the host, one CTA per tile, of which the first wave takes
+  // over the others' tiles as it goes: with a fixed share each, the slowest CTA
+  // of an 800x800 frame ended 25 % after the mean.  With the count on the
+  // device most of the capacity's tiles do not exist, and fixed shares of
+  // those that do are what one wave can take.
+  a.steal = a.S_dev == nullptr && tiles > wave && tiles < (1LL << 31);
+  k<<<(unsigned)(a.steal ? tiles : std::min(tiles, wave)), 128, res.dyn_smem, st>>>(a);
   DV_TRY_LAUNCH();
   return DV_OK;
 }

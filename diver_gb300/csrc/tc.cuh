@@ -116,6 +116,35 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
 
+// ---- dynamic tiles: cluster launch control ----
+// A kernel launched with one CTA per tile, of which only the first wave
+// starts: each running CTA asks for the next CTA not yet started, cancels its
+// launch and does its work itself.  Tiles so go to whichever CTA is free, with
+// no counter in memory to set up, share or reset.  The request is answered by
+// a 16-byte write to shared memory that completes on an mbarrier; once one has
+// failed no other may be made.
+__device__ __forceinline__ void clc_request(void* response, uint64_t* bar) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], 16;" ::"r"(smem_u32(bar)) : "memory");
+  asm volatile(
+      "clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
+          smem_u32(response)),
+      "r"(smem_u32(bar))
+      : "memory");
+}
+
+// The cancelled CTA's blockIdx.x, or -1 when none was left.
+__device__ __forceinline__ int clc_answer(const void* response) {
+  uint32_t ok, x;
+  asm volatile(
+      "{\n .reg .pred p;\n .reg .b128 r;\n ld.shared.b128 r, [%2];\n"
+      " clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n selp.u32 %0, 1, 0, p;\n mov.b32 %1, 0;\n"
+      " @p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, r;\n}\n"
+      : "=r"(ok), "=r"(x)
+      : "r"(smem_u32(response))
+      : "memory");
+  return ok ? (int)x : -1;
+}
+
 // Makes generic-proxy shared-memory writes visible to the tensor core.
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 

@@ -125,13 +125,15 @@ class Segments:
     Built with a fixed `capacity`, the buffers hold that many rows and only the
     first offsets[B] are segments; the count (offsets[B]) and max_dev (max
     segments per ray, int32 [1]) then stay on the device and max_count is None.
+    exact: the buffers hold the segments and nothing else, as a host read of
+    the total sized them.
     """
 
-    __slots__ = ("offsets", "seg", "t", "ray", "counts", "max_count", "max_dev")
+    __slots__ = ("offsets", "seg", "t", "ray", "counts", "max_count", "max_dev", "exact")
 
-    def __init__(self, offsets, seg, t, ray, counts, max_count=None, max_dev=None):
+    def __init__(self, offsets, seg, t, ray, counts, max_count=None, max_dev=None, exact=False):
         self.offsets, self.seg, self.t, self.ray, self.counts = offsets, seg, t, ray, counts
-        self.max_dev = max_dev
+        self.max_dev, self.exact = max_dev, exact
         if max_dev is not None:
             self.max_count = max_count
         else:
@@ -152,8 +154,10 @@ class Segments:
 
     @property
     def count_ptr(self) -> int | None:
-        """Device address of the segment count (offsets[B]) for the decode entry points."""
-        if self.offsets.numel() == 0:
+        """Device address of the segment count (offsets[B]) for the decode entry
+        points; None where the buffers' size is the count (the launches then
+        know it, and can spread the work over it)."""
+        if self.exact or self.offsets.numel() == 0:
             return None
         return self.offsets.data_ptr() + (self.offsets.numel() - 1) * self.offsets.element_size()
 
@@ -239,7 +243,7 @@ class PendingSegments:
             N.call("dv_masked_segments", self.num.numel(), float(xyzmin), float(voxel_num), float(voxel_size),
                    float(mask_scale), N.ptr(o), N.ptr(v), N.ptr(m8), N.ptr(self.offsets), N.ptr(seg), N.ptr(t),
                    N.ptr(ray), N.ptr(self.last), N.stream(dev))
-        return Segments(self.offsets, seg, t, ray, self.num, M, None)
+        return Segments(self.offsets, seg, t, ray, self.num, M, None, exact=True)
 
 
 def masked_segments_begin(o, v, xyzmin, voxel_num, voxel_size, mask, mask_scale) -> PendingSegments:
@@ -297,7 +301,7 @@ def dense_segments(o, v, xyzmin, voxel_num, voxel_size, capacity: int | None = N
     if S > 0 and B > 0:
         N.call("dv_dense_segments", B, float(xyzmin), float(voxel_num), float(voxel_size),
                N.ptr(o), N.ptr(v), N.ptr(offsets), N.ptr(seg), N.ptr(t), N.ptr(ray), st)
-    return Segments(offsets, seg, t, ray, pairs, M, mx)
+    return Segments(offsets, seg, t, ray, pairs, M, mx, exact=capacity is None)
 
 
 def masked_segments_grid(o, v, xyzmin, dims, voxel_size, mask, capacity: int | None = None) -> Segments:
@@ -331,4 +335,4 @@ def masked_segments_grid(o, v, xyzmin, dims, voxel_size, mask, capacity: int | N
     if S > 0 and B > 0:
         N.call("dv_masked_segments_grid", B, ctypes.addressof(x0), ctypes.addressof(dd), float(voxel_size), N.ptr(o),
                N.ptr(v), N.ptr(m8), N.ptr(offsets), N.ptr(seg), N.ptr(t), N.ptr(ray), N.ptr(last), st)
-    return Segments(offsets, seg, t, ray, num, M, mx)
+    return Segments(offsets, seg, t, ray, num, M, mx, exact=capacity is None)
