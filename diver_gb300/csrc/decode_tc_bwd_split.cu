@@ -37,15 +37,25 @@
 // sigmoid.  The record is read into shared memory by bulk async copies, one
 // per layer slot.
 //
-// One CTA per SM, 288 threads: chain thread t < 256 owns segment row
-// r = t % 128 (TMEM lane r; warps w and w + 4 share a lane quadrant) and half
-// h = t / 128 of each row's columns in the epilogues; lane 0 of warp 8 issues
-// the MMAs and the record loads.  The scatter of a tile's feature gradient
-// into the grid runs on the chain threads while the next tile's MMAs run.
-// Shared memory (about 184 KiB): the propagation images, the saved record in
-// five per-layer slots, the PE tile, the delta tile, a tile of ones and the
-// FP32 staging rows of the feature gradient.  TMEM: all 512 columns (64
-// working, 384 weight-gradient and 64 bias-gradient columns).
+// One CTA per SM, 544 threads in three roles:
+//   issuer   (warp 0) issues the MMAs and the record loads
+//   chain    (256, warps 1-8) a thread owns one segment row r (TMEM lane r;
+//            warps w and w + 4 share a lane quadrant) and half h of its
+//            columns: it turns a layer's propagated delta into the next one's
+//   scatter  (256) adds the finished tile's feature gradient to the grid
+// A layer's propagation is issued and committed first; its gradient MMAs
+// follow in the same queue and run while the chain forms the next delta, in
+// the other of two delta tiles.  A propagation's commit also covers the
+// gradient MMAs queued before it, which is what frees the delta tile and the
+// record slot of the layer before.
+// Shared memory (226 KiB): the propagation images, the saved record in five
+// per-layer slots, the PE tile, two delta tiles, a tile of ones, the FP32
+// staging rows of the feature gradient and the scatter's corners.  TMEM: all 512
+// columns (64 working, 384 weight-gradient and 64 bias-gradient columns).
+// Measured, captured 4096-ray step of the 256^3 scene (1.26 M segments): 733 us
+// with the chain doing the scatter in its waits and every MMA of a layer ahead
+// of its epilogue, 625 us in this form with one thread issuing and stepping
+// with the chain, 522 us with the issuer's warp running free of it.
 // Reference semantics: the autograd backward of model/diver.py:159-180.
 #include "common.cuh"
 #include "integrate.cuh"
@@ -59,9 +69,10 @@ namespace bws {
 
 constexpr int C = 32, W = 32;
 constexpr int NL = 5;
-constexpr int CHAIN = 256;             // the layer chain's threads: two per segment row (warps 0-7)
-constexpr int ISSUER = CHAIN;          // lane 0 of warp 8: issues the MMAs and the record loads
-constexpr int THREADS = CHAIN + 32;
+constexpr int CHAIN = 256;             // the layer chain's threads: two per segment row (warps 1-8)
+constexpr int CHAIN_ALL = CHAIN + 32;  // chain and issuer warp
+constexpr int SCATTER = 256;           // warps 9-16
+constexpr int THREADS = CHAIN_ALL + SCATTER;
 constexpr int FD = 48;              // delta columns per term (K of the widest propagation MMA)
 constexpr int DW = 3 * FD;          // delta tile columns: the three terms side by side
 constexpr int TILE = 128 * 32 * 2;  // one term of a [128][32] BF16 tile
@@ -84,6 +95,7 @@ __host__ __device__ constexpr int PIMG(int l) { return 32 * KPROP(l) * 2; }  // 
 __host__ __device__ constexpr int POFF(int l) { return l == 0 ? 0 : POFF(l - 1) + 3 * PIMG(l - 1); }
 constexpr uint32_t RECORD = 5 * 2 * TILE;  // saved record of one tile: 5 layer inputs, [128][2 x 32] each
 constexpr uint32_t ONES_BYTES = 128 * 16 * 2;  // a [128][16] BF16 tile of ones
+constexpr int COEF = 12;                       // floats per segment: 8 corner weights, lower corner's row, row steps
 
 struct Args {
   int nvx, nvy, nvz;
@@ -107,20 +119,21 @@ struct Args {
 
 // Shared-memory layout (byte offsets; the propagation images take 3 x 10240 bytes).
 struct Layout {
-  uint32_t bb, rec, pe, d, ones, stage, bar;
+  uint32_t bb, rec, pe, d, ones, stage, coef, bar;
   __host__ __device__ static Layout make() {
     Layout L;
     L.bb = 0;
     L.rec = (uint32_t)(POFF(NL) + 1023) / 1024 * 1024;
     L.pe = L.rec + RECORD;
     L.d = L.pe + 2 * TILE;
-    L.ones = L.d + 3 * DTILE;
+    L.ones = L.d + 2 * 3 * DTILE;
     L.stage = L.ones + ONES_BYTES;
-    L.bar = L.stage + 128 * (C + 4) * 4;
+    L.coef = L.stage + 128 * (C + 4) * 4;
+    L.bar = L.coef + 128 * COEF * 4;
     return L;
   }
-  // barriers: MMA completion, NL record slots; then the TMEM address and the abort flag
-  __host__ __device__ uint32_t bytes() const { return bar + 8 * (1 + NL) + 16; }
+  // barriers: propagation, NL record slots, the last MMAs; then the TMEM address and the stop flag
+  __host__ __device__ uint32_t bytes() const { return bar + 8 * (2 + NL) + 16; }
 };
 
 // Writes n values (multiple of 8) of row r, columns c0.., as three BF16 terms
@@ -175,7 +188,7 @@ __device__ __forceinline__ void relu_mask(const uint8_t* tile, int r, int c0, fl
 // the layer's image [3 x 32][K] (weight term j in rows 32j..32j+31): per 16
 // columns of K, delta_0 x [W0|W1] and delta_1 x [W0|W1] into columns 0..63,
 // delta_0 x W2 into 32..63 and delta_2 x W0 into 0..31.
-__device__ __forceinline__ void mma_prop(uint32_t tmem, const uint8_t* D, const uint8_t* img, int K) {
+__device__ __forceinline__ void mma_prop(uint32_t by, uint32_t tmem, const uint8_t* D, const uint8_t* img, int K) {
   constexpr uint32_t sboA = (DW / 8) * 128, term = (FD / 8) * 128;
   const uint64_t a0 = tc::smem_desc(tc::smem_u32(D), 128, sboA);
   const uint64_t b0 = tc::smem_desc(tc::smem_u32(img), 128, (uint32_t)(K / 8) * 128);
@@ -183,10 +196,10 @@ __device__ __forceinline__ void mma_prop(uint32_t tmem, const uint8_t* D, const 
 #pragma unroll
   for (int k = 0; k < K / 16; ++k) {
     const uint64_t ak = tc::desc_plus(a0, k * 256), bk = tc::desc_plus(b0, k * 256);
-    tc::mma_f16(tmem, ak, bk, i64, k > 0 ? 1u : 0u);
-    tc::mma_f16(tmem, tc::desc_plus(ak, term), bk, i64, 1u);
-    tc::mma_f16(tmem + 32, ak, tc::desc_plus(bk, 2 * 32 * K * 2), i32, 1u);
-    tc::mma_f16(tmem, tc::desc_plus(ak, 2 * term), bk, i32, 1u);
+    tc::mma_f16_by(by, tmem, ak, bk, i64, k > 0 ? 1u : 0u);
+    tc::mma_f16_by(by, tmem, tc::desc_plus(ak, term), bk, i64, 1u);
+    tc::mma_f16_by(by, tmem + 32, ak, tc::desc_plus(bk, 2 * 32 * K * 2), i32, 1u);
+    tc::mma_f16_by(by, tmem, tc::desc_plus(ak, 2 * term), bk, i32, 1u);
   }
 }
 
@@ -201,13 +214,13 @@ constexpr uint32_t DELTA_T_K = 2 * (DW / 8) * 128;  // bytes per 16 segments of 
 
 // Weight gradient over the tile's 128 segments: TMEM dW[128][64] +=
 // delta^T x act, act a [128][2 x 32] tile read transposed (N = 64: both terms).
-__device__ __forceinline__ void mma_dw(uint32_t tmem, const uint8_t* D, const uint8_t* act, bool accumulate) {
+__device__ __forceinline__ void mma_dw(uint32_t by, uint32_t tmem, const uint8_t* D, const uint8_t* act, bool accumulate) {
   const uint32_t idesc = tc::idesc_f16(128, 64, 1) | (1u << 15) | (1u << 16);
   constexpr uint32_t lboB = (64 / 8) * 128;
   const uint64_t a0 = delta_t_desc(D), b0 = tc::smem_desc(tc::smem_u32(act), lboB, 128);
 #pragma unroll
   for (int k = 0; k < 8; ++k)
-    tc::mma_f16(tmem, tc::desc_plus(a0, k * DELTA_T_K), tc::desc_plus(b0, k * 2 * lboB), idesc,
+    tc::mma_f16_by(by, tmem, tc::desc_plus(a0, k * DELTA_T_K), tc::desc_plus(b0, k * 2 * lboB), idesc,
                 (accumulate || k > 0) ? 1u : 0u);
 }
 
@@ -215,83 +228,82 @@ __device__ __forceinline__ void mma_dw(uint32_t tmem, const uint8_t* D, const ui
 // ones, every column the column sum of the delta (terms 0 and 1 in rows 0..47
 // and 48..95; the ones are exact in BF16 and any reading of the all-ones tile
 // is the same).
-__device__ __forceinline__ void mma_db(uint32_t tmem, const uint8_t* D, const uint8_t* ones, bool accumulate) {
+__device__ __forceinline__ void mma_db(uint32_t by, uint32_t tmem, const uint8_t* D, const uint8_t* ones, bool accumulate) {
   const uint32_t idesc = tc::idesc_f16(128, 16, 1) | (1u << 15) | (1u << 16);
   constexpr uint32_t lboB = (16 / 8) * 128;
   const uint64_t a0 = delta_t_desc(D), b0 = tc::smem_desc(tc::smem_u32(ones), lboB, 128);
 #pragma unroll
   for (int k = 0; k < 8; ++k)
-    tc::mma_f16(tmem, tc::desc_plus(a0, k * DELTA_T_K), tc::desc_plus(b0, k * 2 * lboB), idesc,
+    tc::mma_f16_by(by, tmem, tc::desc_plus(a0, k * DELTA_T_K), tc::desc_plus(b0, k * 2 * lboB), idesc,
                 (accumulate || k > 0) ? 1u : 0u);
 }
 
-// Scatter of a finished tile's feature gradient (FP32 staging rows) into the
-// corner rows of its segments, spread over the next tile's first HRUN layer
-// steps, where it fills the wait for their MMAs: thread t takes channel quad
-// q = t % 8 of the HRUN consecutive segments HRUN * (t / 8).. (a half-run),
-// one segment per step.  Consecutive segments of a ray usually sit in
+// Scatter of a finished tile's feature gradient into the corner rows of its
+// segments: thread i takes channel quad q = i % 8 of the HRUN consecutive
+// segments HRUN * (i / 8)...  Consecutive segments of a ray usually sit in
 // face-adjacent voxels and share four corner rows: the shared corners'
 // contributions are added in registers and reach memory with one atomic
 // instead of two.  A merge needs both voxels whole (upper corners not
-// clamped) and one unit step along one axis, so the merged rows are the same
-// rows.  Threads q and q + 4 of a half-run load segment q % 4's coordinates;
-// the others take them by shuffles.
+// clamped) and lower corners one row step apart along one axis, so the merged
+// rows are the same rows.
 constexpr int HRUN = 4;
-static_assert((C / 4) * (128 / HRUN) == CHAIN, "one thread per (channel quad, half-run)");
+static_assert((C / 4) * (128 / HRUN) == SCATTER, "one thread per (channel quad, run)");
 
-struct Scatter {
-  long long s0 = -1;  // first segment of this thread's half-run; -1: nothing to scatter
-  int ls0 = 0, q = 0;
-  float crd[6];       // coordinates of segment s0 + q % HRUN
-  float4 pend[8];     // contributions of the previous segment's corners not yet in memory
-  SegCorner prev{};
-  bool have = false, prev_whole = false;
+// Corner weights and rows of segment s (0 steps where the upper corner is
+// clamped; rows fit 32 bits, 2^32 rows are twice the device's memory), and its
+// row mark for the next step's sparse clear (dv_mark_corner_rows' rule).
+__device__ __forceinline__ void put_coefs(const Args& a, float* coef, long long s) {
+  const float* sg = a.seg + s * 6;
+  const SegCorner sc = segment_corners(__ldg(sg), __ldg(sg + 1), __ldg(sg + 2), __ldg(sg + 3), __ldg(sg + 4),
+                                       __ldg(sg + 5), a.nvx, a.nvy, a.nvz);
+  const uint32_t row = ((uint32_t)sc.z * a.nvy + sc.y) * a.nvx + sc.x;
+  float4* c = reinterpret_cast<float4*>(coef);
+  c[0] = make_float4(sc.w[0], sc.w[1], sc.w[2], sc.w[3]);
+  c[1] = make_float4(sc.w[4], sc.w[5], sc.w[6], sc.w[7]);
+  reinterpret_cast<uint4*>(c)[2] = make_uint4(row, sc.x1 - sc.x, (uint32_t)(sc.y1 - sc.y) * a.nvx,
+                                              (uint32_t)(sc.z1 - sc.z) * a.nvx * a.nvy);
+  if (a.touched) a.touched[row] = 1;
+}
 
-  __device__ __forceinline__ void start(const Args& a, long long tile, int t, long long S) {
-    q = t % (C / 4);
-    ls0 = (t / (C / 4)) * HRUN;
-    s0 = tile * 128 + ls0;
-    const long long s = s0 + q % HRUN;
+__device__ __forceinline__ uint32_t coef_row(const uint4 m, int j) {
+  return m.x + ((j & 1) ? m.y : 0u) + ((j & 2) ? m.z : 0u) + ((j & 4) ? m.w : 0u);
+}
+
+// n: segments of this thread's run (0..HRUN); g: its quad of their gradients.
+__device__ __forceinline__ void scatter_run(const Args& a, const float* coef, int n, const float4* g, int q) {
+  float4 pend[8];  // contributions of the previous segment's corners not yet in memory
+  uint4 pm = make_uint4(0u, 0u, 0u, 0u);
+  bool pwhole = false;
+  float* grid = a.grad_grid + 4 * q;
 #pragma unroll
-    for (int i = 0; i < 6; ++i) crd[i] = s < S ? __ldg(a.seg + s * 6 + i) : 0.f;
-    have = false;
-  }
-
-  // Segment k of the half-run (every lane takes every shuffle); k = HRUN - 1
-  // also writes what is still pending and ends the scatter.
-  __device__ __forceinline__ void step(const Args& a, const float* stage, int k, long long S) {
-    float p[6];
-#pragma unroll
-    for (int i = 0; i < 6; ++i) p[i] = __shfl_sync(0xffffffffu, crd[i], k, C / 4);
-    if (s0 + k < S) {
-      const SegCorner sc = segment_corners(p[0], p[1], p[2], p[3], p[4], p[5], a.nvx, a.nvy, a.nvz);
-      // the row marks for the next step's sparse clear (dv_mark_corner_rows' rule)
-      if (a.touched && q == 0) a.touched[((long long)sc.z * a.nvy + sc.y) * a.nvx + sc.x] = 1;
-      const float4 g = *reinterpret_cast<const float4*>(stage + (ls0 + k) * (C + 4) + 4 * q);
-      const bool whole = sc.x1 == sc.x + 1 && sc.y1 == sc.y + 1 && sc.z1 == sc.z + 1;
+  for (int k = 0; k < HRUN; ++k) {
+    if (k < n) {
+      const float4 wa = *reinterpret_cast<const float4*>(coef + k * COEF);
+      const float4 wb = *reinterpret_cast<const float4*>(coef + k * COEF + 4);
+      const uint4 m = *reinterpret_cast<const uint4*>(coef + k * COEF + 8);
+      const float w[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+      const bool whole = m.y != 0u && m.z != 0u && m.w != 0u;
       int axis = -1;
       bool up = false;
-      if (have && whole && prev_whole) {
-        const int dx = sc.x - prev.x, dy = sc.y - prev.y, dz = sc.z - prev.z;
-        if (abs(dx) + abs(dy) + abs(dz) == 1) {
-          axis = dx != 0 ? 0 : (dy != 0 ? 1 : 2);
-          up = dx + dy + dz > 0;
-        }
+      if (k > 0 && whole && pwhole) {
+        const uint32_t d = m.x - pm.x, e = pm.x - m.x;
+        if (d == m.y || e == m.y) axis = 0;
+        if (d == m.z || e == m.z) axis = 1;
+        if (d == m.w || e == m.w) axis = 2;
+        up = d < e;
       }
-      // the previous segment's corners off the shared face go to memory
-      if (have) {
+      if (k > 0) {  // the previous segment's corners off the shared face go to memory
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const bool shared = axis >= 0 && ((j >> axis) & 1) == (up ? 1 : 0);
-          if (!shared) red_add4(a.grad_grid + corner_row(prev, j, a.nvx, a.nvy) * C + 4 * q, pend[j]);
+          if (!shared) red_add4(grid + (long long)coef_row(pm, j) * C, pend[j]);
         }
       }
       float4 nx[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const float w = sc.w[j];
-        float4 c = make_float4(w * g.x, w * g.y, w * g.z, w * g.w);
-        if (axis >= 0 && ((j >> axis) & 1) == (up ? 0 : 1)) {
+        float4 c = make_float4(w[j] * g[k].x, w[j] * g[k].y, w[j] * g[k].z, w[j] * g[k].w);
+        if (k > 0 && axis >= 0 && ((j >> axis) & 1) == (up ? 0 : 1)) {
           const float4 o = axis == 0 ? pend[j ^ 1] : (axis == 1 ? pend[j ^ 2] : pend[j ^ 4]);
           c.x += o.x;
           c.y += o.y;
@@ -302,25 +314,27 @@ struct Scatter {
       }
 #pragma unroll
       for (int j = 0; j < 8; ++j) pend[j] = nx[j];
-      prev = sc;
-      prev_whole = whole;
-      have = true;
-    }
-    if (k == HRUN - 1) {
-      if (have) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) red_add4(a.grad_grid + corner_row(prev, j, a.nvx, a.nvy) * C + 4 * q, pend[j]);
-      }
-      have = false;
-      s0 = -1;
+      pm = m;
+      pwhole = whole;
     }
   }
-};
+  if (n > 0) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) red_add4(grid + (long long)coef_row(pm, j) * C, pend[j]);
+  }
+}
 
-// Named barrier of the chain (barrier 0 is __syncthreads).
-constexpr int BAR_CHAIN = 1;
+// Named barriers (0 is __syncthreads): a delta in place (the chain arrives, the
+// issuer waits); the whole chain with the issuer; the scatter group; the
+// staging rows handed to it (the chain arrives, it waits) and taken by it (the
+// other way round).
+constexpr int BAR_DELTA = 1, BAR_CHAIN = 2, BAR_SCATTER = 3, BAR_STAGED = 4, BAR_TAKEN = 5;
 
 __device__ __forceinline__ void named_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+__device__ __forceinline__ void named_arrive(int id, int n) {
+  __threadfence_block();
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory");
+}
 // AND of `v` over the n threads of named barrier `id` (all of them wait).
 __device__ __forceinline__ bool named_and(int id, int n, bool v) {
   uint32_t r;
@@ -332,22 +346,21 @@ __device__ __forceinline__ bool named_and(int id, int n, bool v) {
   return r != 0;
 }
 
-// Chain-group barrier that also orders generic-proxy shared-memory writes
-// before the tensor core's reads (and tcgen05 work across the barrier).
-__device__ __forceinline__ void chain_sync() {
+// The chain's side of a delta hand-over: its generic-proxy shared-memory
+// writes before the tensor core's reads, its TMEM reads before the next MMAs'
+// writes.
+__device__ __forceinline__ void delta_ready() {
   tc::fence_before_sync();
   tc::fence_async_smem();
-  named_sync(BAR_CHAIN, THREADS);
+  named_arrive(BAR_DELTA, CHAIN_ALL);
 }
 
 // PE tile row r, columns 16h..16h+15 (PE_DIM = 27 values, then a one in
 // column PE_ONES for layer 3's bias gradient, zeros after), two terms.
-__device__ __forceinline__ void write_pe(const Args& a, uint8_t* PE, int ray, int r, int h) {
-  float v[16];
+__device__ __forceinline__ void load_pe(const Args& a, int ray, int h, float* v) {
   const float* pf = a.pe_feat + (long long)ray * PE_PAD + 16 * h;
 #pragma unroll
   for (int i = 0; i < 16; ++i) v[i] = (16 * h + i < PE_DIM) ? __ldg(pf + i) : (16 * h + i == PE_ONES ? 1.f : 0.f);
-  put2(PE, r, 16 * h, v, 16);
 }
 
 // Delta of the colour logits (dL/drgb * sigmoid') into columns 0..15 of row r.
@@ -379,30 +392,30 @@ __device__ __forceinline__ void prop_row32(uint32_t taddr, float* v) {
 }
 
 // One tile per step of the persistent loop: the five layer steps, each the
-// propagation and gradient MMAs and the epilogue that forms the next delta;
-// the last stages the tile's feature gradient (FP32), which the next tile's
-// first four steps scatter into the grid (Scatter) while their MMAs run.
-// The saved record sits in five per-layer slots, each with its own mbarrier:
-// when a layer step of tile i is done with its slot, that slot is refilled
-// with tile i + gridDim.x's layer input, so the next tile's loads run behind
-// the rest of this tile.  The PE tile and the first delta of the next tile are
-// also written as soon as this tile is done with them.
+// propagation, its gradient MMAs and the epilogue that forms the next delta;
+// the last stages the tile's feature gradient (FP32) for the scatter group.
+// The saved record sits in five per-layer slots, each with its own mbarrier: a
+// slot is refilled with the next input of that layer once the MMAs that read
+// it are done, so the loads run behind the steps in between.  What the chain
+// reads from global memory for the next tile (ray, PE row, the first delta's
+// inputs) is loaded before a wait and used after it.  Waits are bounded: a
+// thread whose wait gave up goes on through the tile, and all stop at its end.
 __global__ void __launch_bounds__(THREADS, 1) decode_bwd_tc_split_kernel(const Args a) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const Layout lay = Layout::make();
   uint8_t* Bb = smem + lay.bb;
   uint8_t* REC = smem + lay.rec;
   uint8_t* PE = smem + lay.pe;
-  uint8_t* D = smem + lay.d;
   uint8_t* ONES = smem + lay.ones;
   float* stage = reinterpret_cast<float*>(smem + lay.stage);  // [128][C + 4] FP32
+  float* coefs = reinterpret_cast<float*>(smem + lay.coef);   // [128][COEF]
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem + lay.bar);
   uint64_t* bar_rec = bar + 1;  // [NL]: completion of slot l's record load
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 1 + NL);
+  uint64_t* bar_end = bar + 1 + NL;
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 2 + NL);
+  volatile uint32_t* stop = tslot + 1;  // the chain gave up: nothing was staged
 
-  const int t = threadIdx.x, warp = t >> 5;
-  const bool chain = t < CHAIN, issuer = t == ISSUER;
-  const int r = t & 127, h = (t >> 7) & 1;
+  const int t = threadIdx.x, warp = __shfl_sync(0xffffffffu, t >> 5, 0);
   const long long S = segment_total(a.S, a.S_dev);
   const long long tiles = (S + 127) / 128;
 
@@ -414,13 +427,15 @@ __global__ void __launch_bounds__(THREADS, 1) decode_bwd_tc_split_kernel(const A
       reinterpret_cast<uint4*>(Bb + POFF(l))[i] =
           __ldg(reinterpret_cast<const uint4*>(a.wb + j * a.wterm + a.b_img[l]) + o);
     }
-  for (int i = t; i < 3 * DTILE / 16; i += THREADS) reinterpret_cast<uint4*>(D)[i] = make_uint4(0, 0, 0, 0);
+  for (int i = t; i < 2 * 3 * DTILE / 16; i += THREADS) reinterpret_cast<uint4*>(smem + lay.d)[i] = make_uint4(0, 0, 0, 0);
   for (int i = t; i < (int)ONES_BYTES / 16; i += THREADS)
     reinterpret_cast<uint4*>(ONES)[i] = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);  // bf16 1.0
   if (t == 0) {
     tc::mbar_init(bar, 1);
+    tc::mbar_init(bar_end, 1);
     for (int l = 0; l < NL; ++l) tc::mbar_init(bar_rec + l, 1);
     tc::fence_mbar_init();
+    *stop = 0;
   }
   if (warp == 0) {
     tc::tmem_alloc(tslot, TMEM_COLS);
@@ -432,34 +447,97 @@ __global__ void __launch_bounds__(THREADS, 1) decode_bwd_tc_split_kernel(const A
   tc::fence_after_sync();
   const uint32_t tmem = *tslot;
 
-  {
+  bool ok = true, first = true;  // first: no tile done yet
+  if (warp == 0) {
+    // ---- issuer
+    const uint32_t by = tc::elect_one();
+    uint32_t phase_rec = 0;  // bit l = parity of slot l's next completion
+    uint32_t pending = 0;    // slots with a load in flight
+    uint32_t db = 0;         // the delta tile of the next step
+    auto load_slot = [&](int l, long long tile) {
+      if (by) {
+        tc::mbar_arrive_expect_tx(bar_rec + l, 2 * TILE);
+        tc::bulk_load(REC + l * 2 * TILE, a.saved + tile * (long long)RECORD + l * 2 * TILE, 2 * TILE, bar_rec + l);
+      }
+      pending |= 1u << l;
+    };
+    if (blockIdx.x < tiles)
+      for (int l = 0; l < NL; ++l) load_slot(l, blockIdx.x);
+    for (long long tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+      const long long next = tile + gridDim.x;
+#pragma unroll
+      for (int l = NL - 1; l >= 0; --l) {
+        const uint8_t* D = smem + lay.d + db * (3 * DTILE);
+        named_sync(BAR_DELTA, CHAIN_ALL);  // this delta is in place; the previous propagation was waited for
+        tc::fence_after_sync();
+        mma_prop(by, tmem, D, Bb + POFF(l), KPROP(l));
+        tc::mma_commit_by(by, bar);
+        // that propagation's commit covered the gradient MMAs of two steps ago: their slot takes
+        // its next input (layers 0 and 1: this tile's)
+        const int f = (l + 2) % NL;
+        if (f >= 2 ? next < tiles : !first) load_slot(f, f >= 2 ? next : tile);
+        const bool arrived = tc::mbar_wait_bounded(bar_rec + l, (phase_rec >> l) & 1u);
+        if (arrived) {
+          phase_rec ^= 1u << l;
+          pending &= ~(1u << l);
+          const uint8_t* act = REC + l * 2 * TILE;  // this layer's input, two terms TILE apart
+          mma_dw(by, tmem + DWCOL(l), D, act, !first);
+          if (l == 3)
+            mma_dw(by, tmem + DWCOL(3) + 64, D, PE, !first);  // with layer 3's bias gradient (the ones column)
+          else
+            mma_db(by, tmem + DBCOL(l), D, ONES, !first);
+        }
+        ok &= arrived;
+        db ^= 1u;
+      }
+      first = false;
+      ok = named_and(BAR_CHAIN, CHAIN_ALL, ok);
+    }
+    // what is still in flight ends before the CTA frees its shared memory and
+    // TMEM: the last MMAs, and after a failure record loads (bounded waits)
+    if (!first) {
+      tc::mma_commit_by(by, bar_end);
+      for (int l = 0; l < NL; ++l)
+        if ((pending >> l) & 1u) tc::mbar_wait_bounded(bar_rec + l, (phase_rec >> l) & 1u);
+      ok &= tc::mbar_wait_bounded(bar_end, 0);
+      ok = named_and(BAR_CHAIN, CHAIN_ALL, ok);
+      if (!ok && by && a.err) atomicExch(a.err, 1);
+    }
+  } else if (warp > CHAIN / 32) {
+    // ---- scatter group
+    const int i = t - CHAIN_ALL, q = i % (C / 4), ls = (i / (C / 4)) * HRUN;
+    for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+      const long long s0 = tile * 128;
+      if (i < 128 && s0 + i < S) put_coefs(a, coefs + i * COEF, s0 + i);
+      named_sync(BAR_SCATTER, SCATTER);
+      named_sync(BAR_STAGED, CHAIN + SCATTER);
+      if (*stop) break;
+      float4 g[HRUN];
+#pragma unroll
+      for (int k = 0; k < HRUN; ++k) g[k] = *reinterpret_cast<const float4*>(stage + (ls + k) * (C + 4) + 4 * q);
+      named_arrive(BAR_TAKEN, CHAIN + SCATTER);
+      const long long left = S - (s0 + ls);
+      scatter_run(a, coefs + ls * COEF, left >= HRUN ? HRUN : (left > 0 ? (int)left : 0), g, q);
+      named_sync(BAR_SCATTER, SCATTER);  // the next tile's corners overwrite these
+    }
+  } else {
+    // ---- chain
     const uint32_t lane = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t trow = tmem + lane;
-    uint32_t phase = 0, phase_rec = 0;  // phase_rec: bit l = parity of slot l's next completion
-    uint32_t pending = 0;               // issuer: slots with a load in flight
-    bool mma_inflight = false;          // issuer: an MMA batch committed and not yet waited for
-    bool ok = true, first = true;
+    const int r = 32 * (warp & 3) + (t & 31), h = warp > 4 ? 1 : 0;
+    uint32_t phase = 0, phase_rec = 0, db = 0;
     float v[32];
-    Scatter sc;  // the previous tile's feature-gradient scatter
-    // the CTA's first tile: record loads, PE tile, first delta
+    // the CTA's first tile: PE tile, first delta
     long long tile = blockIdx.x;
     if (tile < tiles) {
-      if (issuer) {
-        const uint8_t* rec = a.saved + tile * (long long)RECORD;
-        for (int l = 0; l < NL; ++l) {
-          tc::mbar_arrive_expect_tx(bar_rec + l, 2 * TILE);
-          tc::bulk_load(REC + l * 2 * TILE, rec + l * 2 * TILE, 2 * TILE, bar_rec + l);
-        }
-        pending = (1u << NL) - 1;
-      }
       const long long s = tile * 128 + r;
       const bool valid = s < S;
-      if (chain) {
-        write_pe(a, PE, valid ? __ldg(a.seg_ray + s) : 0, r, h);
-        if (h == 0)
-          write_delta4(D, r, valid ? a.d4[s] : make_float4(0.f, 0.f, 0.f, 0.f),
-                       valid ? a.out4[s] : make_float4(0.f, 0.f, 0.f, 0.f));
-      }
+      load_pe(a, valid ? __ldg(a.seg_ray + s) : 0, h, v);
+      put2(PE, r, 16 * h, v, 16);
+      if (h == 0)
+        write_delta4(smem + lay.d, r, valid ? a.d4[s] : make_float4(0.f, 0.f, 0.f, 0.f),
+                     valid ? a.out4[s] : make_float4(0.f, 0.f, 0.f, 0.f));
+      delta_ready();
     }
     for (; tile < tiles && ok; tile += gridDim.x) {
       const long long s = tile * 128 + r;
@@ -467,46 +545,27 @@ __global__ void __launch_bounds__(THREADS, 1) decode_bwd_tc_split_kernel(const A
       const long long next = tile + gridDim.x;
       const long long sn = next * 128 + r;
       const bool valid_next = next < tiles && sn < S;
-      const float gx = chain && valid ? a.d4[s].x : 0.f;  // dL/dsigma of this row (layer 2's delta)
-      chain_sync();  // the PE tile and the first delta are in place
+      const float gx = valid ? a.d4[s].x : 0.f;  // dL/dsigma of this row (layer 2's delta)
+      const int ray_next = valid_next ? __ldg(a.seg_ray + sn) : 0;
+      float4 gn = make_float4(0.f, 0.f, 0.f, 0.f), on = gn;  // the next tile's first delta
+      float pe[16];                                          // the next tile's PE row
       // layers last to first (unrolled: every layer constant is a compile-time value)
 #pragma unroll
       for (int l = NL - 1; l >= 0; --l) {
         const uint8_t* act = REC + l * 2 * TILE;  // this layer's input, two terms TILE apart
-        // this layer's record slot has arrived (bounded wait; the parities
-        // advance only on success: after a timeout the abort path waits with them)
-        const bool arrived = tc::mbar_wait_bounded(bar_rec + l, (phase_rec >> l) & 1u);
-        if (arrived) phase_rec ^= 1u << l;
-        if (issuer && arrived) {
-          pending &= ~(1u << l);
-          tc::fence_after_sync();
-          mma_prop(tmem, D, Bb + POFF(l), KPROP(l));
-          mma_dw(tmem + DWCOL(l), D, act, !first);
-          if (l == 3)
-            mma_dw(tmem + DWCOL(3) + 64, D, PE, !first);  // with layer 3's bias gradient (the ones column)
-          else
-            mma_db(tmem + DBCOL(l), D, ONES, !first);
-          tc::mma_commit(bar);
-          mma_inflight = true;
+        uint8_t* Dn = smem + lay.d + (db ^ 1u) * (3 * DTILE);
+        if (l == 2 && next < tiles) load_pe(a, ray_next, h, pe);
+        if (l == 1 && valid_next && h == 0) {
+          gn = a.d4[sn];
+          on = a.out4[sn];
         }
-        // while the MMAs run: one segment of the previous tile's scatter (steps 4..1)
-        if (chain && l >= NL - HRUN && !first) sc.step(a, stage, NL - 1 - l, S);
-        // if the issuer's slot wait gave up it issued nothing: every thread's MMA wait then
-        // runs out too, and the AND below stops them all
-        bool done = false;
-        if (arrived) {
-          done = tc::mbar_wait_bounded(bar, phase);
-          if (done) {
-            phase ^= 1u;
-            if (issuer) mma_inflight = false;
-          }
-        }
+        // this layer's input for the ReLU masks, and its propagation
+        ok &= tc::mbar_wait_bounded(bar_rec + l, (phase_rec >> l) & 1u);
+        phase_rec ^= 1u << l;
+        ok &= tc::mbar_wait_bounded(bar, phase);
+        phase ^= 1u;
         tc::fence_after_sync();
-        ok = named_and(BAR_CHAIN, THREADS, arrived && done);
-        if (!ok) break;
-        if (!chain) {
-          // the issuer warp has no rows
-        } else if (l == 3) {
+        if (l == 3) {
           // delta of layer 2: (dL/dsigma, d hidden[0..31]) in columns 0..32, zeros to 47;
           // half 0 writes columns 0..23, half 1 columns 24..47
           prop_row32(trow, v);
@@ -519,64 +578,47 @@ __global__ void __launch_bounds__(THREADS, 1) decode_bwd_tc_split_kernel(const A
 #pragma unroll
             for (int i = 0; i < 24; ++i) w[i] = (i + 23 < W) ? v[i + 23] : 0.f;
           }
-          put3(D, r, 24 * h, w, 24);
-          // this tile's PE is consumed: the next tile's goes in now
-          if (next < tiles) write_pe(a, PE, valid_next ? __ldg(a.seg_ray + sn) : 0, r, h);
+          put3(Dn, r, 24 * h, w, 24);
         } else if (l > 0) {
           prop_row16(trow + 16 * h, v);
           relu_mask(act, r, 16 * h, v, 16);  // this layer's input is relu of the previous layer's output
-          put3(D, r, 16 * h, v, 16);
+          put3(Dn, r, 16 * h, v, 16);
+          // layer 3's gradient MMAs are done with this tile's PE: the next tile's goes in
+          if (l == 2 && next < tiles) put2(PE, r, 16 * h, pe, 16);
         } else {
-          // dL/dfeature (FP32) to the staging rows (the previous tile's scatter
-          // finished in step 1), scattered during the next tile's steps
-          float4 gn = make_float4(0.f, 0.f, 0.f, 0.f), on = gn;
-          if (valid_next && h == 0) {
-            gn = a.d4[sn];
-            on = a.out4[sn];
-          }
+          // the next tile's first delta; then dL/dfeature (FP32) to the staging rows, once the
+          // scatter group has taken the last tile's
           prop_row16(trow + 16 * h, v);
+          if (next < tiles) {
+            if (h == 0) write_delta4(Dn, r, gn, on);
+            delta_ready();
+          }
+          if (!first) named_sync(BAR_TAKEN, CHAIN + SCATTER);
           float* st = stage + r * (C + 4) + 16 * h;
 #pragma unroll
           for (int i = 0; i < 16; i += 4)
             *reinterpret_cast<float4*>(st + i) =
                 valid ? make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]) : make_float4(0.f, 0.f, 0.f, 0.f);
-          sc.start(a, tile, t, S);
-          // this tile's deltas are consumed: the next tile's first delta goes in now
-          if (next < tiles && h == 0) write_delta4(D, r, gn, on);
         }
-        chain_sync();  // D is complete for the next layer; every read of this layer's slot is done
-        if (issuer && next < tiles) {
-          // refill this layer's slot with the next tile's input
-          tc::mbar_arrive_expect_tx(bar_rec + l, 2 * TILE);
-          tc::bulk_load(REC + l * 2 * TILE, a.saved + next * (long long)RECORD + l * 2 * TILE, 2 * TILE,
-                        bar_rec + l);
-          pending |= 1u << l;
-        }
+        if (l > 0) delta_ready();
+        db ^= 1u;
       }
-      if (!ok) break;
       first = false;
+      ok = named_and(BAR_CHAIN, CHAIN_ALL, ok);
+      if (!ok && t == 32) *stop = 1;
+      if (!ok) named_sync(BAR_CHAIN + 4, CHAIN);
+      named_arrive(BAR_STAGED, CHAIN + SCATTER);
     }
-    // the last tile's scatter (its staging rows are complete: every step ends with chain_sync)
-    if (chain && ok && !first) {
-#pragma unroll 1
-      for (int k = 0; k < HRUN; ++k) sc.step(a, stage, k, S);
-    }
-    if (!ok) {
-      if (issuer) {
-        if (a.err) atomicExch(a.err, 1);
-        // record loads and MMAs still in flight complete before the CTA frees
-        // its shared memory and TMEM (bounded waits)
-        for (int l = 0; l < NL; ++l)
-          if ((pending >> l) & 1u) tc::mbar_wait_bounded(bar_rec + l, (phase_rec >> l) & 1u);
-        if (mma_inflight) tc::mbar_wait_bounded(bar, phase);
-      }
-      __threadfence_block();
-      named_sync(BAR_CHAIN, THREADS);
+    if (!first && ok) named_sync(BAR_TAKEN, CHAIN + SCATTER);  // the last tile's
+    if (!first) {
+      tc::fence_before_sync();
+      ok = named_and(BAR_CHAIN, CHAIN_ALL, ok);  // the issuer has seen the last MMAs end
+      tc::fence_after_sync();
     }
     // ---- flush: accumulator row m holds delta term 0 (m < 48) or 1 (48 <= m < 96) of
     // output o = m % 48; per input block, columns c and 32 + c hold activation terms 0
     // and 1 of input c.  Rows of both delta terms add into the same gradient entries.
-    if (chain && ok && !first) {
+    if (ok && !first) {
       const int o = r < FD ? r : r - FD;
       const bool row = r < 2 * FD;
 #pragma unroll

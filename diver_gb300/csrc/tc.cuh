@@ -173,6 +173,34 @@ __device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64
       : "memory");
 }
 
+// One lane of a converged warp (the same one every time).
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+  return p;
+}
+
+// mma_f16 and mma_commit for code that a whole warp runs: only the lane with
+// `lane` set issues.  Operands then stay warp-uniform, and an instruction takes
+// a few uniform additions instead of moves of every operand out of a thread's
+// registers (a warp with one thread inside a branch issued one MMA in about 130
+// clocks beside four busy warps).
+__device__ __forceinline__ void mma_f16_by(uint32_t lane, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
+                                           uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n .reg .pred p, q;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %5, 0;\n"
+      " @q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(lane)
+      : "memory");
+}
+__device__ __forceinline__ void mma_commit_by(uint32_t lane, uint64_t* bar) {
+  asm volatile(
+      "{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n"
+      " @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(smem_u32(bar)),
+      "r"(lane)
+      : "memory");
+}
+
 // The same with A in TMEM: rows in lanes, two consecutive 16-bit K elements per
 // 32-bit column (8 columns per instruction).
 __device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
