@@ -55,7 +55,8 @@
 // Measured, captured 4096-ray step of the 256^3 scene (1.26 M segments): 733 us
 // with the chain doing the scatter in its waits and every MMA of a layer ahead
 // of its epilogue, 625 us in this form with one thread issuing and stepping
-// with the chain, 522 us with the issuer's warp running free of it.
+// with the chain, 522 us with the issuer's warp running free of it, 513 us with
+// the layer loops rolled (instruction cache).
 // Reference semantics: the autograd backward of model/diver.py:159-180.
 #include "common.cuh"
 #include "integrate.cuh"
@@ -84,7 +85,7 @@ __host__ __device__ constexpr int OUT(int l) { return l == 2 ? W + 1 : (l == 4 ?
 __host__ __device__ constexpr int OUT4(int l) { return pad4(OUT(l)); }
 __host__ __device__ constexpr int NBLK(int l) { return l == 3 ? 2 : 1; }  // 32-column input blocks (layer 3: + PE)
 // weight gradient of layer l: per input block, 64 columns (activation terms 0 and 1)
-__host__ __device__ constexpr int DWCOL(int l) { return l == 0 ? 64 : DWCOL(l - 1) + 64 * NBLK(l - 1); }
+__host__ __device__ constexpr int DWCOL(int l) { return 64 + 64 * l + (l > 3 ? 64 : 0); }
 // bias gradient of layer l != 3 (column 0 of 16); layer 3's is column 27 of its PE block
 __host__ __device__ constexpr int DBCOL(int l) { return 448 + 16 * (l < 3 ? l : l - 1); }
 constexpr int PE_ONES = 27;  // the PE tile's column of ones (PE_DIM = 27 values before it)
@@ -92,7 +93,9 @@ __host__ __device__ constexpr int KPROP(int l) { return l == 4 ? 16 : (l == 2 ? 
 // propagation image of layer l in shared memory: [3 terms x 32 rows][KPROP(l)],
 // the three terms side by side along N, layers one after the other
 __host__ __device__ constexpr int PIMG(int l) { return 32 * KPROP(l) * 2; }  // one term's bytes
-__host__ __device__ constexpr int POFF(int l) { return l == 0 ? 0 : POFF(l - 1) + 3 * PIMG(l - 1); }
+__host__ __device__ constexpr int POFF(int l) { return 3 * 64 * (32 * l + (l > 2 ? 16 : 0) - (l > 4 ? 16 : 0)); }
+static_assert(POFF(3) == POFF(2) + 3 * PIMG(2) && POFF(5) == POFF(4) + 3 * PIMG(4), "images one after the other");
+static_assert(DWCOL(4) == DWCOL(3) + 64 * NBLK(3), "gradient blocks one after the other");
 constexpr uint32_t RECORD = 5 * 2 * TILE;  // saved record of one tile: 5 layer inputs, [128][2 x 32] each
 constexpr uint32_t ONES_BYTES = 128 * 16 * 2;  // a [128][16] BF16 tile of ones
 constexpr int COEF = 12;                       // floats per segment: 8 corner weights, lower corner's row, row steps
@@ -193,7 +196,7 @@ __device__ __forceinline__ void mma_prop(uint32_t by, uint32_t tmem, const uint8
   const uint64_t a0 = tc::smem_desc(tc::smem_u32(D), 128, sboA);
   const uint64_t b0 = tc::smem_desc(tc::smem_u32(img), 128, (uint32_t)(K / 8) * 128);
   const uint32_t i64 = tc::idesc_f16(128, 64, 1), i32 = tc::idesc_f16(128, 32, 1);
-#pragma unroll
+#pragma unroll 1
   for (int k = 0; k < K / 16; ++k) {
     const uint64_t ak = tc::desc_plus(a0, k * 256), bk = tc::desc_plus(b0, k * 256);
     tc::mma_f16_by(by, tmem, ak, bk, i64, k > 0 ? 1u : 0u);
@@ -218,7 +221,7 @@ __device__ __forceinline__ void mma_dw(uint32_t by, uint32_t tmem, const uint8_t
   const uint32_t idesc = tc::idesc_f16(128, 64, 1) | (1u << 15) | (1u << 16);
   constexpr uint32_t lboB = (64 / 8) * 128;
   const uint64_t a0 = delta_t_desc(D), b0 = tc::smem_desc(tc::smem_u32(act), lboB, 128);
-#pragma unroll
+#pragma unroll 1
   for (int k = 0; k < 8; ++k)
     tc::mma_f16_by(by, tmem, tc::desc_plus(a0, k * DELTA_T_K), tc::desc_plus(b0, k * 2 * lboB), idesc,
                 (accumulate || k > 0) ? 1u : 0u);
@@ -232,10 +235,32 @@ __device__ __forceinline__ void mma_db(uint32_t by, uint32_t tmem, const uint8_t
   const uint32_t idesc = tc::idesc_f16(128, 16, 1) | (1u << 15) | (1u << 16);
   constexpr uint32_t lboB = (16 / 8) * 128;
   const uint64_t a0 = delta_t_desc(D), b0 = tc::smem_desc(tc::smem_u32(ones), lboB, 128);
-#pragma unroll
+#pragma unroll 1
   for (int k = 0; k < 8; ++k)
     tc::mma_f16_by(by, tmem, tc::desc_plus(a0, k * DELTA_T_K), tc::desc_plus(b0, k * 2 * lboB), idesc,
                 (accumulate || k > 0) ? 1u : 0u);
+}
+
+// Named barriers (0 is __syncthreads): a delta in place (the chain arrives, the
+// issuer waits); the whole chain with the issuer; the scatter group; the
+// staging rows handed to it (the chain arrives, it waits) and taken by it (the
+// other way round).
+constexpr int BAR_DELTA = 1, BAR_CHAIN = 2, BAR_SCATTER = 3, BAR_STAGED = 4, BAR_TAKEN = 5;
+
+__device__ __forceinline__ void named_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+__device__ __forceinline__ void named_arrive(int id, int n) {
+  __threadfence_block();
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory");
+}
+// AND of `v` over the n threads of named barrier `id` (all of them wait).
+__device__ __forceinline__ bool named_and(int id, int n, bool v) {
+  uint32_t r;
+  asm volatile(
+      "{\n .reg .pred p, q;\n setp.ne.u32 q, %1, 0;\n bar.red.and.pred p, %2, %3, q;\n selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(r)
+      : "r"((uint32_t)v), "r"(id), "r"(n)
+      : "memory");
+  return r != 0;
 }
 
 // Scatter of a finished tile's feature gradient into the corner rows of its
@@ -269,81 +294,60 @@ __device__ __forceinline__ uint32_t coef_row(const uint4 m, int j) {
   return m.x + ((j & 1) ? m.y : 0u) + ((j & 2) ? m.z : 0u) + ((j & 4) ? m.w : 0u);
 }
 
-// n: segments of this thread's run (0..HRUN); g: its quad of their gradients.
-__device__ __forceinline__ void scatter_run(const Args& a, const float* coef, int n, const float4* g, int q) {
+// n: segments of this thread's run (0..HRUN); st: its quad in the run's first
+// staging row.
+__device__ __forceinline__ void scatter_run(const Args& a, const float* coef, int n, const float* st, int q) {
   float4 pend[8];  // contributions of the previous segment's corners not yet in memory
   uint4 pm = make_uint4(0u, 0u, 0u, 0u);
   bool pwhole = false;
   float* grid = a.grad_grid + 4 * q;
-#pragma unroll
-  for (int k = 0; k < HRUN; ++k) {
-    if (k < n) {
-      const float4 wa = *reinterpret_cast<const float4*>(coef + k * COEF);
-      const float4 wb = *reinterpret_cast<const float4*>(coef + k * COEF + 4);
-      const uint4 m = *reinterpret_cast<const uint4*>(coef + k * COEF + 8);
-      const float w[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
-      const bool whole = m.y != 0u && m.z != 0u && m.w != 0u;
-      int axis = -1;
-      bool up = false;
-      if (k > 0 && whole && pwhole) {
-        const uint32_t d = m.x - pm.x, e = pm.x - m.x;
-        if (d == m.y || e == m.y) axis = 0;
-        if (d == m.z || e == m.z) axis = 1;
-        if (d == m.w || e == m.w) axis = 2;
-        up = d < e;
-      }
-      if (k > 0) {  // the previous segment's corners off the shared face go to memory
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const bool shared = axis >= 0 && ((j >> axis) & 1) == (up ? 1 : 0);
-          if (!shared) red_add4(grid + (long long)coef_row(pm, j) * C, pend[j]);
-        }
-      }
-      float4 nx[8];
+#pragma unroll 1
+  for (int k = 0; k < n; ++k) {
+    const float4 g = *reinterpret_cast<const float4*>(st + k * (C + 4));
+    const float4 wa = *reinterpret_cast<const float4*>(coef + k * COEF);
+    const float4 wb = *reinterpret_cast<const float4*>(coef + k * COEF + 4);
+    const uint4 m = *reinterpret_cast<const uint4*>(coef + k * COEF + 8);
+    const float w[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+    const bool whole = m.y != 0u && m.z != 0u && m.w != 0u;
+    int axis = -1;
+    bool up = false;
+    if (k > 0 && whole && pwhole) {
+      const uint32_t d = m.x - pm.x, e = pm.x - m.x;
+      if (d == m.y || e == m.y) axis = 0;
+      if (d == m.z || e == m.z) axis = 1;
+      if (d == m.w || e == m.w) axis = 2;
+      up = d < e;
+    }
+    if (k > 0) {  // the previous segment's corners off the shared face go to memory
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        float4 c = make_float4(w[j] * g[k].x, w[j] * g[k].y, w[j] * g[k].z, w[j] * g[k].w);
-        if (k > 0 && axis >= 0 && ((j >> axis) & 1) == (up ? 0 : 1)) {
-          const float4 o = axis == 0 ? pend[j ^ 1] : (axis == 1 ? pend[j ^ 2] : pend[j ^ 4]);
-          c.x += o.x;
-          c.y += o.y;
-          c.z += o.z;
-          c.w += o.w;
-        }
-        nx[j] = c;
+        const bool shared = axis >= 0 && ((j >> axis) & 1) == (up ? 1 : 0);
+        if (!shared) red_add4(grid + (long long)coef_row(pm, j) * C, pend[j]);
       }
-#pragma unroll
-      for (int j = 0; j < 8; ++j) pend[j] = nx[j];
-      pm = m;
-      pwhole = whole;
     }
+    float4 nx[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      float4 c = make_float4(w[j] * g.x, w[j] * g.y, w[j] * g.z, w[j] * g.w);
+      if (axis >= 0 && ((j >> axis) & 1) == (up ? 0 : 1)) {
+        const float4 o = axis == 0 ? pend[j ^ 1] : (axis == 1 ? pend[j ^ 2] : pend[j ^ 4]);
+        c.x += o.x;
+        c.y += o.y;
+        c.z += o.z;
+        c.w += o.w;
+      }
+      nx[j] = c;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) pend[j] = nx[j];
+    pm = m;
+    pwhole = whole;
   }
+  named_arrive(BAR_TAKEN, CHAIN + SCATTER);
   if (n > 0) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) red_add4(grid + (long long)coef_row(pm, j) * C, pend[j]);
   }
-}
-
-// Named barriers (0 is __syncthreads): a delta in place (the chain arrives, the
-// issuer waits); the whole chain with the issuer; the scatter group; the
-// staging rows handed to it (the chain arrives, it waits) and taken by it (the
-// other way round).
-constexpr int BAR_DELTA = 1, BAR_CHAIN = 2, BAR_SCATTER = 3, BAR_STAGED = 4, BAR_TAKEN = 5;
-
-__device__ __forceinline__ void named_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
-__device__ __forceinline__ void named_arrive(int id, int n) {
-  __threadfence_block();
-  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory");
-}
-// AND of `v` over the n threads of named barrier `id` (all of them wait).
-__device__ __forceinline__ bool named_and(int id, int n, bool v) {
-  uint32_t r;
-  asm volatile(
-      "{\n .reg .pred p, q;\n setp.ne.u32 q, %1, 0;\n bar.red.and.pred p, %2, %3, q;\n selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(r)
-      : "r"((uint32_t)v), "r"(id), "r"(n)
-      : "memory");
-  return r != 0;
 }
 
 // The chain's side of a delta hand-over: its generic-proxy shared-memory
@@ -465,7 +469,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_bwd_tc_split_kernel(const A
       for (int l = 0; l < NL; ++l) load_slot(l, blockIdx.x);
     for (long long tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
       const long long next = tile + gridDim.x;
-#pragma unroll
+#pragma unroll 1
       for (int l = NL - 1; l >= 0; --l) {
         const uint8_t* D = smem + lay.d + db * (3 * DTILE);
         named_sync(BAR_DELTA, CHAIN_ALL);  // this delta is in place; the previous propagation was waited for
@@ -512,12 +516,8 @@ __global__ void __launch_bounds__(THREADS, 1) decode_bwd_tc_split_kernel(const A
       named_sync(BAR_SCATTER, SCATTER);
       named_sync(BAR_STAGED, CHAIN + SCATTER);
       if (*stop) break;
-      float4 g[HRUN];
-#pragma unroll
-      for (int k = 0; k < HRUN; ++k) g[k] = *reinterpret_cast<const float4*>(stage + (ls + k) * (C + 4) + 4 * q);
-      named_arrive(BAR_TAKEN, CHAIN + SCATTER);
       const long long left = S - (s0 + ls);
-      scatter_run(a, coefs + ls * COEF, left >= HRUN ? HRUN : (left > 0 ? (int)left : 0), g, q);
+      scatter_run(a, coefs + ls * COEF, left >= HRUN ? HRUN : (left > 0 ? (int)left : 0), stage + ls * (C + 4) + 4 * q, q);
       named_sync(BAR_SCATTER, SCATTER);  // the next tile's corners overwrite these
     }
   } else {
@@ -549,8 +549,8 @@ __global__ void __launch_bounds__(THREADS, 1) decode_bwd_tc_split_kernel(const A
       const int ray_next = valid_next ? __ldg(a.seg_ray + sn) : 0;
       float4 gn = make_float4(0.f, 0.f, 0.f, 0.f), on = gn;  // the next tile's first delta
       float pe[16];                                          // the next tile's PE row
-      // layers last to first (unrolled: every layer constant is a compile-time value)
-#pragma unroll
+      // layers last to first
+#pragma unroll 1
       for (int l = NL - 1; l >= 0; --l) {
         const uint8_t* act = REC + l * 2 * TILE;  // this layer's input, two terms TILE apart
         uint8_t* Dn = smem + lay.d + (db ^ 1u) * (3 * DTILE);
