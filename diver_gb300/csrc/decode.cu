@@ -10,23 +10,56 @@
 
 namespace dv {
 
+// W / 4 threads per ray, 4 outputs each, their 27 x 4 weights in registers for
+// all the rays that a block takes in turn; a ray is encoded once, into shared
+// memory.  Each output is the chain of FMAs over the encoding from the bias, in
+// order.
 template <int W, int D1>
-__global__ void __launch_bounds__(128) ray_pe_kernel(const DecodeArgs a) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= a.B) return;
-  float pe[PE_PAD];
-  pos_enc(__ldg(a.dirs + 3 * b), __ldg(a.dirs + 3 * b + 1), __ldg(a.dirs + 3 * b + 2), pe);
+__global__ void __launch_bounds__(256) ray_pe_kernel(const DecodeArgs a) {
+  constexpr int TPR = W / 4, RAYS = 256 / TPR;
+  __shared__ __align__(16) float pes[RAYS][PE_PAD];
+  const int t = threadIdx.x, r = t / TPR, j = 4 * (t % TPR);
+  const float* Wt = a.params + a.w_off[D1 + 1] + W * W + j;  // rows W .. W+26 of [W+27][W]
+  const float* bias = a.params + a.b_off[D1 + 1] + j;
+  float w[PE_DIM][4], b4[4];
 #pragma unroll
-  for (int k = 0; k < PE_PAD; k += 4)
-    *reinterpret_cast<float4*>(a.pe_feat + (long long)b * PE_PAD + k) = make_float4(pe[k], pe[k + 1], pe[k + 2], pe[k + 3]);
-  const float* Wt = a.params + a.w_off[D1 + 1] + W * W;  // rows W .. W+26 of [W+27][W]
-  const float* bias = a.params + a.b_off[D1 + 1];
-  float* out = a.pe_out + (long long)b * W;
-#pragma unroll 4
-  for (int j = 0; j < W; ++j) {
-    float acc = __ldg(bias + j);
-    for (int k = 0; k < PE_DIM; ++k) acc = fmaf(pe[k], __ldg(Wt + k * W + j), acc);
-    out[j] = acc;
+  for (int i = 0; i < 4; ++i) b4[i] = __ldg(bias + i);
+#pragma unroll
+  for (int k = 0; k < PE_DIM; ++k)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[k][i] = __ldg(Wt + k * W + i);
+  for (long long b0 = (long long)blockIdx.x * RAYS; b0 < a.B; b0 += (long long)gridDim.x * RAYS) {
+    if (t < 3 * RAYS) {  // one component of one ray's direction: its entry, 4 sines, 4 cosines (pos_enc)
+      const int e = t / 3, c = t - 3 * e;
+      const float x = b0 + e < a.B ? __ldg(a.dirs + 3 * b0 + t) : 0.f;
+      pes[e][c] = x;
+      float f = 3.14159265358979323846f;
+#pragma unroll
+      for (int l = 0; l < 4; ++l) {
+        float sn, cs;
+        sincosf(f * x, &sn, &cs);
+        pes[e][3 + 6 * l + c] = sn;
+        pes[e][6 + 6 * l + c] = cs;
+        f *= 2.f;
+      }
+      if (c == 0) pes[e][PE_DIM] = 0.f;
+    }
+    __syncthreads();
+    for (int i = t; i < RAYS * PE_PAD && i < (a.B - b0) * PE_PAD; i += 256)
+      a.pe_feat[b0 * PE_PAD + i] = (&pes[0][0])[i];
+    if (b0 + r < a.B) {
+      float o[4] = {b4[0], b4[1], b4[2], b4[3]};
+#pragma unroll
+      for (int k = 0; k < PE_DIM; ++k) {
+        const float p = pes[r][k];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) o[i] = fmaf(p, w[k][i], o[i]);
+      }
+      float* out = a.pe_out + (b0 + r) * W + j;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) out[i] = o[i];
+    }
+    __syncthreads();
   }
 }
 
@@ -280,8 +313,10 @@ int dv_ray_pe(int kind, int channels, const float* params, int batch, const floa
   a.pe_feat = pe_feat;
   a.pe_out = pe_out;
   cudaStream_t st = (cudaStream_t)stream;
-  if (kind == 32) ray_pe_kernel<32, 2><<<ceil_div(batch, 128), 128, 0, st>>>(a);
-  else ray_pe_kernel<64, 1><<<ceil_div(batch, 128), 128, 0, st>>>(a);
+  // 256 / (W / 4) rays per block and turn, two blocks per SM (registers)
+  const unsigned blocks = std::min<unsigned>(ceil_div(batch, kind == 32 ? 32 : 16), 2u * sm_count());
+  if (kind == 32) ray_pe_kernel<32, 2><<<blocks, 256, 0, st>>>(a);
+  else ray_pe_kernel<64, 1><<<blocks, 256, 0, st>>>(a);
   DV_TRY_LAUNCH();
   return DV_OK;
 }
