@@ -39,6 +39,8 @@ SIGNATURES = {
     "dv_scan_scratch_bytes": (I64, [I64]),
     "dv_walk_cap_hits": (I64, [I32]),
     "dv_exclusive_scan": (I32, [P, I64, P, P, P]),
+    "dv_segment_offsets_scratch_bytes": (I64, [I64]),
+    "dv_segment_offsets": (I32, [P, I64, P, P, P, P]),
     "dv_exclusive_scan_static_max": (I64, []),
     "dv_exclusive_scan_static": (I32, [P, I64, P, P]),
     "dv_integrate_fwd": (I32, [P, I32, I32, I32, I32, P, P, I64, I64, P, P]),
@@ -113,8 +115,13 @@ def ptr(t: torch.Tensor | None) -> int | None:
     return None if t is None else t.data_ptr()
 
 
-def stream(device: torch.device | None = None) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+def stream(device: torch.device | str | int | None = None) -> int:
+    """The current stream's handle (a stream object per launch costs more than
+    the launch)."""
+    index = device
+    if index is not None and not isinstance(index, int):  # a torch.device, or its name
+        index = (index if isinstance(index, torch.device) else torch.device(index)).index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
 def need_cuda(name: str, t: torch.Tensor, dtype: torch.dtype | None = None) -> None:

@@ -781,6 +781,105 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_tiles(const int* __restrict
   if (base < n && base + SCAN_ITEMS >= n) out[n] = run;  // thread owning the last element
 }
 
+// ---- offsets, total and largest count in one go -----------------------------
+
+__device__ __forceinline__ long long warp_max64(long long v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+
+// Up to SMALL_SCAN counts in one block: SMALL_SCAN / 1024 consecutive ones per
+// thread.  totals = (sum, largest count).
+constexpr int SMALL_SCAN = 16384;
+
+__global__ void __launch_bounds__(1024) small_offsets_kernel(const int* __restrict__ in, int n, int64_t* __restrict__ out,
+                                                             long long* __restrict__ totals) {
+  __shared__ long long sums[32], maxs[32];
+  constexpr int PER = SMALL_SCAN / 1024;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int per = (n + 1023) / 1024;  // <= PER, spread over all threads
+  int v[PER];
+  long long s = 0, m = 0;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    v[i] = i < per && t * per + i < n ? in[t * per + i] : 0;
+    s += v[i];
+    m = max(m, (long long)v[i]);
+  }
+  long long incl = s;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const long long y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  m = warp_max64(m);
+  if (lane == 31) {
+    sums[warp] = incl;
+    maxs[warp] = m;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    long long w = sums[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long y = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += y;
+    }
+    sums[lane] = w;
+    const long long mm = warp_max64(maxs[lane]);
+    if (lane == 31) {
+      totals[0] = w;
+      totals[1] = mm;
+      out[n] = w;
+    }
+  }
+  __syncthreads();
+  long long run = (warp ? sums[warp - 1] : 0) + incl - s;
+#pragma unroll
+  for (int i = 0; i < PER; ++i)
+    if (i < per && t * per + i < n) {
+      out[t * per + i] = run;
+      run += v[i];
+    }
+}
+
+// Larger n: the tiles' sums as in scan_tile_sums, and their largest counts.
+__global__ void __launch_bounds__(SCAN_THREADS) tile_max_kernel(const int* __restrict__ in, long long n,
+                                                                long long* __restrict__ tile_max) {
+  __shared__ long long maxs[SCAN_THREADS / 32];
+  const long long base = (long long)blockIdx.x * SCAN_TILE + threadIdx.x;
+  long long m = 0;
+#pragma unroll
+  for (int i = 0; i < SCAN_ITEMS; ++i)
+    if (base + i * SCAN_THREADS < n) m = max(m, (long long)in[base + i * SCAN_THREADS]);
+  m = warp_max64(m);
+  if ((threadIdx.x & 31) == 0) maxs[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int w = 1; w < SCAN_THREADS / 32; ++w) m = max(m, maxs[w]);
+    tile_max[blockIdx.x] = m;
+  }
+}
+
+__global__ void __launch_bounds__(1024) totals_kernel(const long long* __restrict__ tile_max, long long tiles,
+                                                      const int64_t* __restrict__ end, long long* __restrict__ totals) {
+  __shared__ long long maxs[32];
+  long long m = 0;
+  for (long long i = threadIdx.x; i < tiles; i += 1024) m = max(m, tile_max[i]);
+  m = warp_max64(m);
+  if ((threadIdx.x & 31) == 0) maxs[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    m = warp_max64(maxs[threadIdx.x]);
+    if (threadIdx.x == 0) {
+      totals[0] = *end;
+      totals[1] = m;
+    }
+  }
+}
+
 }  // namespace dv
 
 using namespace dv;
@@ -1102,6 +1201,35 @@ int dv_exclusive_scan(const int* counts, long long n, int64_t* offsets, void* sc
   scan_tile_sums<<<(unsigned)tiles, SCAN_THREADS, 0, st>>>(counts, n, tile_sum);
   scan_tile_prefix<<<1, SCAN_THREADS, 0, st>>>(tile_sum, tiles);
   scan_tiles<<<(unsigned)tiles, SCAN_THREADS, 0, st>>>(counts, n, tile_sum, offsets);
+  DV_TRY_LAUNCH();
+  return DV_OK;
+}
+
+long long dv_segment_offsets_scratch_bytes(long long n) {
+  return n <= SMALL_SCAN ? 0 : 2 * dv_scan_scratch_bytes(n);
+}
+
+int dv_segment_offsets(const int* counts, long long n, int64_t* offsets, int64_t* totals, void* scratch, void* stream) {
+  DV_CHECK(n >= 0 && offsets && totals, DV_ERR_ARG);
+  cudaStream_t st = (cudaStream_t)stream;
+  if (n == 0) {
+    if (cudaMemsetAsync(offsets, 0, sizeof(int64_t), st) != cudaSuccess) return DV_ERR_CUDA;
+    if (cudaMemsetAsync(totals, 0, 2 * sizeof(int64_t), st) != cudaSuccess) return DV_ERR_CUDA;
+    return DV_OK;
+  }
+  DV_CHECK(counts && (scratch || n <= SMALL_SCAN), DV_ERR_ARG);
+  long long* tot = reinterpret_cast<long long*>(totals);
+  if (n <= SMALL_SCAN) {
+    small_offsets_kernel<<<1, 1024, 0, st>>>(counts, (int)n, offsets, tot);
+    DV_TRY_LAUNCH();
+    return DV_OK;
+  }
+  const int rc = dv_exclusive_scan(counts, n, offsets, scratch, stream);
+  if (rc != DV_OK) return rc;
+  const long long tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
+  long long* tile_max = (long long*)scratch + tiles;
+  tile_max_kernel<<<(unsigned)tiles, SCAN_THREADS, 0, st>>>(counts, n, tile_max);
+  totals_kernel<<<1, 1024, 0, st>>>(tile_max, tiles, offsets + n, tot);
   DV_TRY_LAUNCH();
   return DV_OK;
 }

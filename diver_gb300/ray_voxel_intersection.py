@@ -15,6 +15,8 @@ DIVeR.extract_features builds from those buffers by boolean indexing
 """
 from __future__ import annotations
 
+import ctypes
+
 import torch
 from torch.autograd import Function
 
@@ -33,7 +35,8 @@ def _check_rays(o: torch.Tensor, v: torch.Tensor) -> int:
 
 def mask_side(voxel_num: float, mask_scale: float) -> int:
     """int(voxel_num * mask_scale) with the product rounded to float32, as the reference computes it."""
-    return int(torch.tensor(float(voxel_num), dtype=torch.float32).mul(float(mask_scale)).item())
+    f32 = ctypes.c_float  # the product of two FP32 values is exact in double, so this rounds once
+    return int(f32(f32(voxel_num).value * f32(mask_scale).value).value)
 
 
 def _check_mask(mask: torch.Tensor, voxel_num: float, mask_scale: float) -> torch.Tensor:
@@ -162,12 +165,21 @@ class Segments:
         return self.offsets.data_ptr() + (self.offsets.numel() - 1) * self.offsets.element_size()
 
 
-def _totals(offsets: torch.Tensor, counts: torch.Tensor) -> tuple[int, int]:
+def _offsets_totals(counts: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
+    """(offsets [n+1], totals [2] = total segments, max per ray), on the device."""
+    n = counts.numel()
+    dev = counts.device
+    out = torch.empty(n + 3, dtype=torch.int64, device=dev)
+    nbytes = int(N.lib().dv_segment_offsets_scratch_bytes(n))
+    scratch = torch.empty(nbytes, dtype=torch.uint8, device=dev) if nbytes else None
+    N.call("dv_segment_offsets", N.ptr(counts), n, N.ptr(out), out.data_ptr() + 8 * (n + 1), N.ptr(scratch), N.stream(dev))
+    return out[:n + 1], out[n + 1:]
+
+
+def _read_totals(totals: torch.Tensor) -> tuple[int, int]:
     """(total segments, max per ray) with a single device-to-host read."""
-    if counts.numel() == 0:
-        return 0, 0
-    S, M = torch.stack([offsets[-1], counts.max().to(torch.int64)]).tolist()
-    return int(S), int(M)
+    S, M = totals.tolist()
+    return S, M
 
 
 def _capacity(capacity: int, B: int, planes: int) -> int:
@@ -229,15 +241,15 @@ class PendingSegments:
     emission walk.  Launching the count walks of several batches (on their
     own streams) before finishing any lets them run together."""
 
-    __slots__ = ("args", "num", "offsets", "last")
+    __slots__ = ("args", "num", "offsets", "totals", "last")
 
-    def __init__(self, args, num, offsets, last):
-        self.args, self.num, self.offsets, self.last = args, num, offsets, last
+    def __init__(self, args, num, offsets, totals, last):
+        self.args, self.num, self.offsets, self.totals, self.last = args, num, offsets, totals, last
 
     def finish(self) -> Segments:
         o, v, xyzmin, voxel_num, voxel_size, m8, mask_scale = self.args
         dev = o.device
-        S, M = _totals(self.offsets, self.num)
+        S, M = _read_totals(self.totals)
         seg, t, ray = _buffers(S, dev)
         if S > 0:
             N.call("dv_masked_segments", self.num.numel(), float(xyzmin), float(voxel_num), float(voxel_size),
@@ -251,12 +263,11 @@ def masked_segments_begin(o, v, xyzmin, voxel_num, voxel_size, mask, mask_scale)
     B = _check_rays(o, v)
     m8 = _check_mask(mask, voxel_num, mask_scale)
     dev = o.device
-    num = torch.empty(B, dtype=torch.int32, device=dev)
-    last = torch.empty(B, dtype=torch.int32, device=dev)  # where each ray's emission walk may stop
+    num, last = torch.empty(2, B, dtype=torch.int32, device=dev)  # last: where each ray's emission walk may stop
     if B > 0:
         N.call("dv_masked_count", B, float(xyzmin), float(voxel_num), float(voxel_size), float(mask_scale),
                N.ptr(o), N.ptr(v), N.ptr(m8), N.ptr(num), None, N.ptr(last), N.stream(dev))
-    return PendingSegments((o, v, xyzmin, voxel_num, voxel_size, m8, mask_scale), num, exclusive_scan(num), last)
+    return PendingSegments((o, v, xyzmin, voxel_num, voxel_size, m8, mask_scale), num, *_offsets_totals(num), last)
 
 
 def masked_segments(o, v, xyzmin, voxel_num, voxel_size, mask, mask_scale, capacity: int | None = None) -> Segments:
@@ -290,11 +301,12 @@ def dense_segments(o, v, xyzmin, voxel_num, voxel_size, capacity: int | None = N
            N.ptr(o), N.ptr(v), N.ptr(num), None, st)
     pairs = torch.empty_like(num)
     N.call("dv_dense_pair_counts", B, N.ptr(num), N.ptr(pairs), st)
-    offsets = exclusive_scan(pairs)
     mx = None
     if capacity is None:
-        S, M = _totals(offsets, pairs)
+        offsets, totals = _offsets_totals(pairs)
+        S, M = _read_totals(totals)
     else:
+        offsets = exclusive_scan(pairs)
         S, M = _capacity(capacity, B, 3 * int(voxel_num)), None
         mx = pairs.max().reshape(1) if B > 0 else torch.zeros(1, dtype=torch.int32, device=dev)
     seg, t, ray = _buffers(S, dev)
@@ -315,8 +327,6 @@ def masked_segments_grid(o, v, xyzmin, dims, voxel_size, mask, capacity: int | N
     if mask.numel() != nx * ny * nz:
         raise ValueError(f"mask must hold {nz}x{ny}x{nx} cells, got {tuple(mask.shape)}")
     m8 = mask.view(torch.uint8) if mask.dtype == torch.bool else mask
-    import ctypes
-
     x0 = (ctypes.c_float * 3)(*[float(x) for x in xyzmin])
     dd = (ctypes.c_int * 3)(nx, ny, nz)
     dev = o.device
@@ -326,10 +336,11 @@ def masked_segments_grid(o, v, xyzmin, dims, voxel_size, mask, capacity: int | N
     mx = torch.zeros(1, dtype=torch.int32, device=dev) if capacity is not None else None
     N.call("dv_masked_count_grid", B, ctypes.addressof(x0), ctypes.addressof(dd), float(voxel_size), N.ptr(o), N.ptr(v),
            N.ptr(m8), N.ptr(num), N.ptr(mx), N.ptr(last), st)
-    offsets = exclusive_scan(num)
     if capacity is None:
-        S, M = _totals(offsets, num)
+        offsets, totals = _offsets_totals(num)
+        S, M = _read_totals(totals)
     else:
+        offsets = exclusive_scan(num)
         S, M = _capacity(capacity, B, nx + ny + nz), None
     seg, t, ray = _buffers(S, dev)
     if S > 0 and B > 0:

@@ -68,6 +68,11 @@ def _check_params(kind: int, channels: int, params: torch.Tensor):
 FORMS = ("fp32", "bf16", "fp16", "bf16s")
 
 
+# Rays up to which their directions' encoding runs on the calling stream (8 us
+# at this many, against about 25 us of host time for a side stream).
+PE_INLINE = 16384
+
+
 class TcWeights:
     """Decoder weights in the tensor-core operand layout on the device.  The
     images are gathered from the packed plain parameters on the device
@@ -351,6 +356,13 @@ class DIVeRField(torch.nn.Module):
             tw.version = self.params._version
         return tw
 
+    def _refreshes(self, form: str) -> bool:
+        """Whether tc_weights(form) would rebuild its images."""
+        if form not in FORMS or form == "fp32":
+            return False
+        tw = self._tc.get(form)
+        return tw is None or self.refresh_always or tw.version != self.params._version
+
     @staticmethod
     def from_scene(scene, device="cuda") -> "DIVeRField":
         return DIVeRField(scene.features.to(device), scene.decoder, scene.mask.to(device), scene.xyzmin,
@@ -438,22 +450,32 @@ class DIVeRField(torch.nn.Module):
         N.need_cuda("dirs", ds, torch.float32)
         dev = self.voxels.device
         kind = KIND_ID[self.kind]
-        # the tensor-core weight images and the directions' encoding do not
-        # depend on the segments: they run on a side stream beside the
-        # traversal, which occupies one warp per SM (the outputs are
-        # allocated on the calling stream, which waits for the side stream)
-        main = torch.cuda.current_stream(dev)
-        side = self._side_stream(dev)
         pe = (torch.empty(ds.shape[0], 28, device=dev), torch.empty(ds.shape[0], WIDTH[kind], device=dev))
-        side.wait_stream(main)
-        with torch.cuda.stream(side):
+
+        def prepare():
             tc = self.tc_weights(form)
             if ds.shape[0]:
                 _check_params(kind, self.voxels.shape[-1], self.params)
                 _timed("dv_ray_pe", kind, self.voxels.shape[-1], N.ptr(self.params), ds.shape[0], N.ptr(ds),
                        N.ptr(pe[0]), N.ptr(pe[1]), N.stream(dev))
-        seg = segments if segments is not None else self.segments(os, ds, capacity)
-        main.wait_stream(side)
+            return tc
+
+        if ds.shape[0] <= PE_INLINE and not self._refreshes(form):
+            # a few microseconds of encoding: less than going to another stream and back
+            tc = prepare()
+            seg = segments if segments is not None else self.segments(os, ds, capacity)
+        else:
+            # the tensor-core weight images and the directions' encoding do not
+            # depend on the segments: they run on a side stream beside the
+            # traversal (the outputs are allocated on the calling stream, which
+            # waits for the side stream)
+            main = torch.cuda.current_stream(dev)
+            side = self._side_stream(dev)
+            side.wait_stream(main)
+            with torch.cuda.stream(side):
+                tc = prepare()
+            seg = segments if segments is not None else self.segments(os, ds, capacity)
+            main.wait_stream(side)
         g16 = self.grid16(form) if not torch.is_grad_enabled() else None
         return render_segments(self.voxels, self.params, seg, ds, self.kind, self.white_back, tc, g16, grad_voxels,
                                pe)

@@ -171,6 +171,17 @@ DV_API long long dv_scan_scratch_bytes(long long n);
 DV_API int dv_exclusive_scan(const int* counts, long long n, int64_t* offsets, void* scratch,
                       void* stream);
 
+/*
+ * dv_exclusive_scan of n counts that also leaves totals[2] = (their sum, the
+ * largest one) on the device, what a caller reads back to size the segment
+ * buffers.  scratch: dv_segment_offsets_scratch_bytes(n) bytes (none, and one
+ * launch, up to 16,384 counts).
+ */
+DV_API long long dv_segment_offsets_scratch_bytes(long long n);
+DV_API int dv_segment_offsets(const int* counts, long long n, int64_t* offsets, int64_t* totals, void* scratch,
+                              void* stream);
+
+
 /* ------------------------------------------------------------------------
  * Feature integration.
  * ------------------------------------------------------------------------ */
