@@ -78,6 +78,9 @@ SIGNATURES = {
     "dv_realtime_tc_bytes": (I32, [I32]),
     "dv_realtime_tc_pack": (I32, [I32, P, P, P]),
     "dv_mlp_eval_tc": (I32, [I32, I32, P, P, P, I32, P, P, P, P, P, P, P]),
+    "dv_mlp_eval_live": (I32, [I32, I32, P, P, P, P, P, I32, P, P, P, P, P, P, P, P]),
+    "dv_realtime_begin": (I32, [I32, P, P, P, I32, P, P, P, P, P]),
+    "dv_march_live": (I32, [I32, P, P, P, P, P, P, I32, P]),
     "dv_realtime_frame": (I32, [I32, I32, P, P, P, I32, P, P, P, I32, P, P, P]),
     "dv_aabb_intersect": (I32, [I32, P, P, P, P, P, P, I32, P]),
     "dv_ray_march": (I32, [I32, P, P, P, P, I32, P]),

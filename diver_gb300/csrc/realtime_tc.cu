@@ -103,6 +103,13 @@ struct Args {
   uint8_t* finish;       // [B]
   const uint8_t* wblob;  // three terms of the images
   int* err;
+  // a frame's live pixels (null: every pixel that finish leaves): pixel of each
+  // of the first *count list positions, which coords is stored by; those still
+  // alive afterwards are appended to next
+  const int* list;
+  const int* count;
+  int* next;
+  int* next_count;
 };
 
 __device__ __forceinline__ int clampi(int x, int hi) { return x < 0 ? 0 : (x > hi ? hi : x); }
@@ -176,35 +183,56 @@ __device__ __forceinline__ void put_row3(uint8_t* sA, uint32_t tstride, int t, c
   }
 }
 
+// A pixel's hit, prepared once by its own thread for the 8 that integrate it:
+// the 8 corner weights and the table rows of the 8 corners (first one -1
+// without a hit).
+constexpr int HIT = 16;
+
+__device__ __forceinline__ void put_hit(const Args& a, float* h, const float* cp) {
+  const SegCorner sc = segment_corners(__ldg(cp), __ldg(cp + 1), __ldg(cp + 2), __ldg(cp + 3), __ldg(cp + 4),
+                                       __ldg(cp + 5), 1 << 30, 1 << 30, 1 << 30);
+  const int x0 = clampi(sc.x, a.ms - 1), x1 = clampi(sc.x + 1, a.ms - 1);
+  int row[8];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int y = clampi(sc.y + (j & 1), a.ms - 1), z = clampi(sc.z + (j >> 1), a.ms - 1);
+    const int* m = a.vmap + ((long long)z * a.ms + y) * a.ms;
+    row[2 * j] = __ldg(m + x0);
+    row[2 * j + 1] = __ldg(m + x1);
+  }
+  float4* d = reinterpret_cast<float4*>(h);
+  d[0] = make_float4(sc.w[0], sc.w[1], sc.w[2], sc.w[3]);
+  d[1] = make_float4(sc.w[4], sc.w[5], sc.w[6], sc.w[7]);
+  reinterpret_cast<int4*>(d)[2] = make_int4(row[0], row[1], row[2], row[3]);
+  reinterpret_cast<int4*>(d)[3] = make_int4(row[4], row[5], row[6], row[7]);
+}
+
 // The tile's integrals, written as the A operand (three terms, K = 32
-// columns): each pixel's hit k (coords and a flag in sHit, 8 floats per row)
-// is integrated by 8 threads, each reading 16 bytes of every corner row, so a
-// warp's loads cover 4 whole rows (coalesced).  FIRST: the integral starts
-// from the pre-multiplied first layer's bias and goes through relu; rows
-// without a hit are zero.
+// columns): 8 threads per row, each reading 16 bytes of every corner row, so a
+// warp's loads cover 4 whole rows (coalesced), each warp its own 32 pixels.
+// FIRST: the integral starts from the pre-multiplied first layer's bias and
+// goes through relu; rows without a hit are zero.
 template <int FIRST>
 __device__ __forceinline__ void integrate_tile(const Args& a, const float* sHit, const float* b_in, uint8_t* sA,
                                                uint32_t tstride) {
-  const int t = threadIdx.x, q = t & 7;
+  const int t = threadIdx.x, q = t & 7, first = (t & ~31) + ((t & 31) >> 3);
 #pragma unroll 1
   for (int p = 0; p < 8; ++p) {
-    const int row = p * 16 + (t >> 3);
-    const float* h = sHit + row * 8;
+    const int row = first + 4 * p;
+    const float* h = sHit + row * HIT;
     float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (h[6] != 0.f) {
-      const SegCorner sc = segment_corners(h[0], h[1], h[2], h[3], h[4], h[5], 1 << 30, 1 << 30, 1 << 30);
+    const int4 ra = *reinterpret_cast<const int4*>(h + 8);
+    if (ra.x >= 0) {
+      const int4 rb = *reinterpret_cast<const int4*>(h + 12);
+      const int rows[8] = {ra.x, ra.y, ra.z, ra.w, rb.x, rb.y, rb.z, rb.w};
       float4 v[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int x = clampi(sc.x + (j & 1), a.ms - 1);
-        const int yy = clampi(sc.y + ((j >> 1) & 1), a.ms - 1);
-        const int z = clampi(sc.z + (j >> 2), a.ms - 1);
-        const int idx = __ldg(a.vmap + ((long long)z * a.ms + yy) * a.ms + x);
-        v[j] = __ldg(reinterpret_cast<const float4*>(a.feats + (long long)idx * 32) + q);
-      }
+      for (int j = 0; j < 8; ++j) v[j] = __ldg(reinterpret_cast<const float4*>(a.feats + (long long)rows[j] * 32) + q);
+      const float4 wa = *reinterpret_cast<const float4*>(h), wb = *reinterpret_cast<const float4*>(h + 4);
+      const float w[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
       if (FIRST) f = *reinterpret_cast<const float4*>(b_in + 4 * q);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) fma4(f, sc.w[j], v[j]);
+      for (int j = 0; j < 8; ++j) fma4(f, w[j], v[j]);
       if (FIRST) f = make_float4(fmaxf(f.x, 0.f), fmaxf(f.y, 0.f), fmaxf(f.z, 0.f), fmaxf(f.w, 0.f));
     }
     uint32_t x[3], y[3];
@@ -240,10 +268,13 @@ __global__ void __launch_bounds__(128, W == 32 ? 4 : 1) mlp_eval_tc_kernel(const
   uint8_t* sB = smem;
   uint8_t* sA = smem + 3 * I::TERM;
   float* sb = reinterpret_cast<float*>(sA + 3 * TSTRIDE);
-  float* sHit = sb + (Bi::size + 3) / 4 * 4;  // [128][8]: this hit's coords and a hit flag per pixel
-  uint64_t* bar = reinterpret_cast<uint64_t*>(sHit + 128 * 8);
+  float* sHit = sb + (Bi::size + 3) / 4 * 4;  // [128][HIT]
+  uint64_t* bar = reinterpret_cast<uint64_t*>(sHit + 128 * HIT);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 1);
   const int t = threadIdx.x, warp = t >> 5;
+  const int n = a.list ? min(*a.count, a.batch) : a.batch;
+  const long long tiles = (n + 127) / 128;
+  if (blockIdx.x >= tiles) return;  // the last rounds of a frame fill a few blocks
   for (int i = t; i < 3 * I::TERM / 16; i += 128)
     reinterpret_cast<uint4*>(sB)[i] = __ldg(reinterpret_cast<const uint4*>(a.wblob) + i);
   for (int i = t; i < Bi::size; i += 128) {
@@ -269,10 +300,10 @@ __global__ void __launch_bounds__(128, W == 32 ? 4 : 1) mlp_eval_tc_kernel(const
   uint32_t phase = 0;
   bool ok = true;
   const long long stride = (long long)a.batch * 6;
-  const long long tiles = (a.batch + 127) / 128;
   for (long long tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
     const long long b = tile * 128 + t;
-    const bool start = b < a.batch && !a.finish[b];
+    const bool start = b < n && (a.list || !a.finish[b]);
+    const long long px = start && a.list ? a.list[b] : b;
     if (!__syncthreads_or(start)) continue;
     bool alive = start, fin = false;
     float4 acc = make_float4(0.f, 0.f, 0.f, 1.f);
@@ -280,9 +311,9 @@ __global__ void __launch_bounds__(128, W == 32 ? 4 : 1) mlp_eval_tc_kernel(const
 #pragma unroll
     for (int j = 0; j < W; ++j) pe2[j] = 0.f;
     if (start) {
-      acc = reinterpret_cast<const float4*>(a.rgba)[b];
+      acc = reinterpret_cast<const float4*>(a.rgba)[px];
       float pe[PE_PAD];
-      pos_enc(__ldg(a.v + 3 * b), __ldg(a.v + 3 * b + 1), __ldg(a.v + 3 * b + 2), pe);
+      pos_enc(__ldg(a.v + 3 * px), __ldg(a.v + 3 * px + 1), __ldg(a.v + 3 * px + 2), pe);
 #pragma unroll
       for (int j = 0; j < W; ++j) pe2[j] = __ldg(a.params + L::l2_b + j);
 #pragma unroll
@@ -297,6 +328,7 @@ __global__ void __launch_bounds__(128, W == 32 ? 4 : 1) mlp_eval_tc_kernel(const
         }
       }
     }
+    // A wait that gave up is seen by all at the tile's end.
 #pragma unroll 1
     for (int k = 0; k < 8; ++k) {
       bool hit = false;
@@ -307,31 +339,34 @@ __global__ void __launch_bounds__(128, W == 32 ? 4 : 1) mlp_eval_tc_kernel(const
           fin = true;
         } else {
           hit = true;
-#pragma unroll
-          for (int i = 0; i < 6; ++i) sHit[t * 8 + i] = __ldg(cp + i);
+          put_hit(a, sHit + t * HIT, cp);
         }
       }
-      sHit[t * 8 + 6] = hit ? 1.f : 0.f;
+      if (!hit) reinterpret_cast<int*>(sHit)[t * HIT + 8] = -1;
       if (!__syncthreads_or(hit)) break;
       integrate_tile<FIRST>(a, sHit, sb + Bi::b_in, sA, TSTRIDE);
       sync_for_mma();
       // L0: h1 = W0 x + b0, relu
-      ok = __syncthreads_and(tc_layer3<32, W>(sA, TSTRIDE, sB, I::off0, tmem, bar, phase));
-      if (!ok) break;
+      ok &= tc_layer3<32, W>(sA, TSTRIDE, sB, I::off0, tmem, bar, phase);
       {
         float v[16];
 #pragma unroll
         for (int c0 = 0; c0 < W; c0 += 16) {
           row16(trow + c0, I::n0, v);
 #pragma unroll
-          for (int i = 0; i < 16; ++i) v[i] = fmaxf(v[i] + sb[Bi::l0_b + c0 + i], 0.f);
+          for (int i = 0; i < 16; i += 4) {
+            const float4 bv = *reinterpret_cast<const float4*>(sb + Bi::l0_b + c0 + i);
+            v[i] = fmaxf(v[i] + bv.x, 0.f);
+            v[i + 1] = fmaxf(v[i + 1] + bv.y, 0.f);
+            v[i + 2] = fmaxf(v[i + 2] + bv.z, 0.f);
+            v[i + 3] = fmaxf(v[i + 3] + bv.w, 0.f);
+          }
           put_row3<W, 16>(sA + tc::kmajor_offset(0, c0, W), TSTRIDE, t, v);
         }
       }
       sync_for_mma();
       // L1: h2 (+ pixel constant) and sigma
-      ok = __syncthreads_and(tc_layer3<W, W + 16>(sA, TSTRIDE, sB, I::off1, tmem, bar, phase));
-      if (!ok) break;
+      ok &= tc_layer3<W, W + 16>(sA, TSTRIDE, sB, I::off1, tmem, bar, phase);
       float alpha;
       {
         float sv[4];
@@ -348,8 +383,7 @@ __global__ void __launch_bounds__(128, W == 32 ? 4 : 1) mlp_eval_tc_kernel(const
       }
       sync_for_mma();
       // L2: colour logits, sigmoid, compositing (skip alpha < 1e-2, stop at T < 1e-2)
-      ok = __syncthreads_and(tc_layer3<W, 16>(sA, TSTRIDE, sB, I::off2, tmem, bar, phase));
-      if (!ok) break;
+      ok &= tc_layer3<W, 16>(sA, TSTRIDE, sB, I::off2, tmem, bar, phase);
       {
         float o[4];
         row4(trow, I::n2, o);
@@ -366,12 +400,22 @@ __global__ void __launch_bounds__(128, W == 32 ? 4 : 1) mlp_eval_tc_kernel(const
         }
       }
       tc::fence_before_sync();
-      __syncthreads();  // the next hit rewrites A and TMEM
+      // the next hit's barrier lies before anything rewrites A or TMEM
     }
+    ok = __syncthreads_and(ok);
     if (!ok) break;
-    if (start) {
-      reinterpret_cast<float4*>(a.rgba)[b] = acc;
-      if (fin) a.finish[b] = 1;
+    if (start) reinterpret_cast<float4*>(a.rgba)[px] = acc;
+    if (a.list) {
+      const unsigned m = __ballot_sync(0xffffffffu, start && !fin);
+      if (m) {
+        const int lane = t & 31, leader = __ffs(m) - 1;
+        int at = 0;
+        if (lane == leader) at = atomicAdd(a.next_count, __popc(m));
+        at = __shfl_sync(0xffffffffu, at, leader);
+        if (start && !fin) a.next[at + __popc(m & ((1u << lane) - 1u))] = (int)px;
+      }
+    } else if (start && fin) {
+      a.finish[b] = 1;
     }
   }
   if (!ok && t == 0 && a.err) atomicExch(a.err, 1);
@@ -387,7 +431,7 @@ int launch(const Args& a, cudaStream_t st) {
   constexpr int NCOLS = W == 32 ? 128 : 256;  // two column blocks of the widest layer (W + 16)
   constexpr int KMAX = W > 32 ? W : 32;
   const size_t smem = 3 * (size_t)I::TERM + 3 * (size_t)128 * KMAX * 2 + (size_t)(Bias<W>::size + 3) / 4 * 16 +
-                      128 * 8 * 4 + 16;
+                      128 * HIT * 4 + 16;
   auto k = mlp_eval_tc_kernel<W, FIRST, NCOLS>;
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return DV_ERR_CUDA;
@@ -444,7 +488,23 @@ int dv_mlp_eval_tc(int width, int batch_size, const float* coords, const float* 
                ((uintptr_t)tc_blob & 15) == 0,
            DV_ERR_ARG);
   rtc::Args a{batch_size, coords, voxels, voxel_map, map_size, packed_params, v, rgba, finish,
-              reinterpret_cast<const uint8_t*>(tc_blob), err};
+              reinterpret_cast<const uint8_t*>(tc_blob), err, nullptr, nullptr, nullptr, nullptr};
+  cudaStream_t st = (cudaStream_t)stream;
+  return width == 32 ? rtc::launch<32, 1>(a, st) : rtc::launch<64, 0>(a, st);
+}
+
+int dv_mlp_eval_live(int width, int capacity, const int* list, const int* count, const float* hits, const float* voxels,
+                     const int* voxel_map, int map_size, const float* packed_params, const void* tc_blob, const float* v,
+                     float* rgba, int* next, int* next_count, int* err, void* stream) {
+  DV_CHECK((width == 32 || width == 64) && capacity >= 0 && map_size > 0, DV_ERR_ARG);
+  if (capacity == 0) return DV_OK;
+  DV_CHECK(list && count && hits && voxels && voxel_map && packed_params && tc_blob && v && rgba && next && next_count,
+           DV_ERR_ARG);
+  DV_CHECK(((uintptr_t)voxels & 15) == 0 && ((uintptr_t)rgba & 15) == 0 && ((uintptr_t)packed_params & 15) == 0 &&
+               ((uintptr_t)tc_blob & 15) == 0,
+           DV_ERR_ARG);
+  rtc::Args a{capacity, hits, voxels, voxel_map, map_size, packed_params, v, rgba, nullptr,
+              reinterpret_cast<const uint8_t*>(tc_blob), err, list, count, next, next_count};
   cudaStream_t st = (cudaStream_t)stream;
   return width == 32 ? rtc::launch<32, 1>(a, st) : rtc::launch<64, 0>(a, st);
 }

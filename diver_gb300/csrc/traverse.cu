@@ -612,43 +612,84 @@ __global__ void __launch_bounds__(256) aabb_kernel(int batch, float* __restrict_
     octree_descend<false>(slot, finish, b, p, d, oct, N, oct_cells);
 }
 
-// Next 8 occupied voxels.  Reference ray_march.cu:159-229.  The reference
-// leaves its grid-stride loop when an unfinished ray has no resume point
-// (x < 0), a state that aabb_intersect + mlp_eval never produce; here such a
-// ray is skipped on its own so the result does not depend on the launch shape.
-template <bool FAST>
-__device__ __forceinline__ void march8(float* __restrict__ coords, long long stride, int b, float3 last,
-                                       const float3 d, const uint8_t* __restrict__ mask, int N) {
+// Next 8 occupied voxels of a ray, put(k, entry, exit) for each in order and
+// put_end(k) where the ray leaves the grid before its k-th.  Reference
+// ray_march.cu:159-229.  8 steps at a time: their occupancy loads are issued
+// back to back (one at a time the walk waits for every byte), and the planes
+// are kept from step to step (walk_step).
+template <class Put, class End>
+__device__ __forceinline__ void march8(const float3 last, const float3 d, bool fast, const uint8_t* __restrict__ mask,
+                                       int N, Put put, End put_end) {
+  constexpr int K = 8;
   const float3 s = signs(d);
-  const float3 r = FAST ? recip3(d) : d;
+  const float3 r = fast ? recip3(d) : d;
   const float n = (float)N;
   const long long cells = (long long)N * N * N;
   const int cap = walk_cap(n, n, n);
-  int hits = 0, steps = 0;
-  while (hits < 8) {
-    if (steps++ == cap) {
-      note_cap_hit();
-      coords[hits * stride + (long long)b * 6] = -1.f;
-      break;
+  const float near = near_plane(make_float3(n, n, n));
+  int hits = 0;
+  Walk w{last, next_planes(last, s), 0.f};
+  for (int steps = 0;; steps += K) {
+    float3 P[K + 1];
+    unsigned out = 0;
+    P[0] = w.a;
+    const Walk w0 = w;
+    float gap = near;
+    if (fast) {
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        walk_step<false>(w, d, r, s, gap);
+        P[k + 1] = w.a;
+        out |= outside_open(w.a, n) ? 1u << k : 0u;
+      }
     }
-    float3 q;
-    float dt;
-    grid_step<FAST>(last, d, r, s, q, dt);
-    if (outside_open(q, n)) {
-      coords[hits * stride + (long long)b * 6] = -1.f;
-      break;
+    if (!fast || gap < near) {
+      w = w0;
+      out = 0;
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        if (out != 0) continue;
+        float3 q;
+        float dt;
+        if (fast)
+          grid_step<true>(w.a, d, r, s, q, dt);
+        else
+          grid_step<false>(w.a, d, r, s, q, dt);
+        w.a = P[k + 1] = q;
+        out |= outside_open(q, n) ? 1u << k : 0u;
+      }
+      w.B = next_planes(w.a, s);
     }
-    if (occupied(mask, cell_index1(last, q, N), cells)) {
-      float2* rr = reinterpret_cast<float2*>(coords + hits * stride + (long long)b * 6);
-      rr[0] = make_float2(last.x, last.y);
-      rr[1] = make_float2(last.z, q.x);
-      rr[2] = make_float2(q.y, q.z);
-      ++hits;
+    const int inside = min(out ? __ffs(out) - 1 : K, cap - steps);
+    uint8_t occ[K];
+    unsigned in_mask = 0;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const long long idx = cell_index1(P[k], P[k + 1], N);
+      const bool ok = k < inside && idx >= 0 && idx < cells;
+      occ[k] = __ldg(mask + (ok ? idx : 0));
+      in_mask |= ok ? 1u << k : 0u;
     }
-    last = q;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      if (((in_mask >> k) & 1u) && occ[k] != 0 && hits < 8) {
+        put(hits, P[k], P[k + 1]);
+        ++hits;
+      }
+    }
+    if (hits == 8) return;
+    if (out != 0 || steps + K >= cap) {
+      if (out == 0) note_cap_hit();
+      put_end(hits);
+      return;
+    }
   }
 }
 
+// The reference leaves its grid-stride loop when an unfinished ray has no
+// resume point (x < 0), a state that aabb_intersect + mlp_eval never produce;
+// here such a ray is skipped on its own so the result does not depend on the
+// launch shape.
 __global__ void __launch_bounds__(256) march_kernel(int batch, float* __restrict__ coords,
                                                     const float* __restrict__ v,
                                                     const uint8_t* __restrict__ mask,
@@ -657,16 +698,102 @@ __global__ void __launch_bounds__(256) march_kernel(int batch, float* __restrict
   if (b >= batch || finish[b]) return;
   const long long stride = (long long)batch * 6;
   const float* rs = coords + 7 * stride + (long long)b * 6 + 3;
-  float3 last = make_float3(rs[0], rs[1], rs[2]);
+  const float3 last = make_float3(rs[0], rs[1], rs[2]);
   coords[(long long)b * 6] = -1.f;
   if (last.x < 0.f) return;
   const float3 d = load3(v, b);
   if (!dir_ok(d)) return;  // a miss (aabb_intersect finished such a ray already)
   const float lim = (float)N;  // a resume point from outside the grid takes the __fdiv_rn form
-  if (N < (1 << 22) && recip_ok(d) && fabsf(last.x) <= lim && fabsf(last.y) <= lim && fabsf(last.z) <= lim)
-    march8<true>(coords, stride, b, last, d, mask, N);
-  else
-    march8<false>(coords, stride, b, last, d, mask, N);
+  const bool fast = N < (1 << 22) && recip_ok(d) && fabsf(last.x) <= lim && fabsf(last.y) <= lim && fabsf(last.z) <= lim;
+  march8(
+      last, d, fast, mask, N,
+      [&](int k, const float3 p, const float3 q) {
+        float2* rr = reinterpret_cast<float2*>(coords + k * stride + (long long)b * 6);
+        rr[0] = make_float2(p.x, p.y);
+        rr[1] = make_float2(p.z, q.x);
+        rr[2] = make_float2(q.y, q.z);
+      },
+      [&](int k) { coords[k * stride + (long long)b * 6] = -1.f; });
+}
+
+// ---- the same over the live pixels of a frame --------------------------------
+//
+// Most pixels of a frame finish in its first rounds, the last ones after
+// dozens.  Each round works on a list of the pixels still alive, so that its
+// tiles of pixels are full: begin makes the first list, the decoder
+// (mlp_eval_tc_kernel) the next one.  Hits are stored by list position,
+// resume points by pixel; what happens to a pixel does not depend on its
+// position.
+
+// Appends `pixel` of the lanes with `alive` to list (one atomic per warp; every lane takes part).
+__device__ __forceinline__ void append_live(bool alive, int pixel, int* __restrict__ list, int* __restrict__ count) {
+  const unsigned m = __ballot_sync(0xffffffffu, alive);
+  if (m == 0u) return;
+  const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
+  int at = 0;
+  if (lane == leader) at = atomicAdd(count, __popc(m));
+  at = __shfl_sync(0xffffffffu, at, leader);
+  if (alive) list[at + __popc(m & ((1u << lane) - 1u))] = pixel;
+}
+
+__global__ void __launch_bounds__(256) begin_kernel(int batch, const float* __restrict__ v,
+                                                    const float* __restrict__ center, const uint8_t* __restrict__ oct,
+                                                    int N, long long oct_cells, float* __restrict__ resume,
+                                                    float* __restrict__ rgba, int* __restrict__ list,
+                                                    int* __restrict__ count) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  uint8_t done = 1;
+  if (b < batch) {
+    done = 0;
+    reinterpret_cast<float4*>(rgba)[b] = make_float4(0.f, 0.f, 0.f, 1.f);
+    const float3 d = load3(v, b);
+    float3 p = make_float3(__ldg(center + 0), __ldg(center + 1), __ldg(center + 2));
+    float t;
+    if (!dir_ok(d) || !box_entry(p, d, (float)N, t)) {
+      done = 1;
+    } else {
+      p = make_float3(__fmul_rn(p.x, 0.015625f), __fmul_rn(p.y, 0.015625f), __fmul_rn(p.z, 0.015625f));
+      float slot[3];
+      if (N < (1 << 22) && recip_ok(d))
+        octree_descend<true>(slot, &done, 0, p, d, oct, N, oct_cells);
+      else
+        octree_descend<false>(slot, &done, 0, p, d, oct, N, oct_cells);
+      if (!done) {
+        resume[3LL * b] = slot[0];
+        resume[3LL * b + 1] = slot[1];
+        resume[3LL * b + 2] = slot[2];
+      }
+    }
+  }
+  append_live(!done, b, list, count);
+}
+
+__global__ void __launch_bounds__(256) march_live_kernel(int capacity, const int* __restrict__ list,
+                                                         const int* __restrict__ count, float* __restrict__ hits,
+                                                         float* __restrict__ resume, const float* __restrict__ v,
+                                                         const uint8_t* __restrict__ mask, int N) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= min(*count, capacity)) return;
+  const int b = list[i];
+  const long long stride = (long long)capacity * 6;
+  const float3 last = make_float3(resume[3LL * b], resume[3LL * b + 1], resume[3LL * b + 2]);
+  const float3 d = load3(v, b);
+  const float lim = (float)N;
+  const bool fast = N < (1 << 22) && recip_ok(d) && fabsf(last.x) <= lim && fabsf(last.y) <= lim && fabsf(last.z) <= lim;
+  march8(
+      last, d, fast, mask, N,
+      [&](int k, const float3 p, const float3 q) {
+        float2* rr = reinterpret_cast<float2*>(hits + k * stride + (long long)i * 6);
+        rr[0] = make_float2(p.x, p.y);
+        rr[1] = make_float2(p.z, q.x);
+        rr[2] = make_float2(q.y, q.z);
+        if (k == 7) {
+          resume[3LL * b] = q.x;
+          resume[3LL * b + 1] = q.y;
+          resume[3LL * b + 2] = q.z;
+        }
+      },
+      [&](int k) { hits[k * stride + (long long)i * 6] = -1.f; });
 }
 
 // Pinhole camera rays (utils/dataset/ray_utils.py:5-55): pixel (i, j) looks
@@ -1245,6 +1372,29 @@ int dv_aabb_intersect(int batch_size, float* coords, const float* v, const float
   const long long cells = a * a * a + b * b * b + c * c * c;
   aabb_kernel<<<ceil_div(batch_size, 256), 256, 0, (cudaStream_t)stream>>>(
       batch_size, coords, v, center, finish, rgba, octrees, voxel_num, cells);
+  DV_TRY_LAUNCH();
+  return DV_OK;
+}
+
+int dv_realtime_begin(int batch_size, const float* v, const float* center, const uint8_t* octrees, int voxel_num,
+                      float* resume, float* rgba, int* list, int* count, void* stream) {
+  DV_CHECK(batch_size >= 0 && voxel_num >= 64 && voxel_num % 64 == 0, DV_ERR_ARG);
+  if (batch_size == 0) return DV_OK;
+  DV_CHECK(v && center && octrees && resume && rgba && list && count && ((uintptr_t)rgba & 15) == 0, DV_ERR_ARG);
+  const long long a = voxel_num / 64, b = voxel_num / 16, c = voxel_num / 4;
+  begin_kernel<<<ceil_div(batch_size, 256), 256, 0, (cudaStream_t)stream>>>(
+      batch_size, v, center, octrees, voxel_num, a * a * a + b * b * b + c * c * c, resume, rgba, list, count);
+  DV_TRY_LAUNCH();
+  return DV_OK;
+}
+
+int dv_march_live(int capacity, const int* list, const int* count, float* hits, float* resume, const float* v,
+                  const uint8_t* mask, int voxel_num, void* stream) {
+  DV_CHECK(capacity >= 0 && voxel_num > 0, DV_ERR_ARG);
+  if (capacity == 0) return DV_OK;
+  DV_CHECK(list && count && hits && resume && v && mask && aligned_to(hits, 8), DV_ERR_ARG);
+  march_live_kernel<<<ceil_div(capacity, 256), 256, 0, (cudaStream_t)stream>>>(capacity, list, count, hits, resume, v,
+                                                                              mask, voxel_num);
   DV_TRY_LAUNCH();
   return DV_OK;
 }

@@ -22,7 +22,7 @@ import torch
 
 from . import _native as N
 from .decoder import Decoder, pack_realtime, premultiply_features
-from .ray_march import aabb_intersect, build_octree_levels, ray_march
+from .ray_march import _u8, aabb_intersect, build_octree_levels, ray_march
 
 
 def convert(state_dict: dict, alpha_map: torch.Tensor, thresh: float = 1e-2) -> dict:
@@ -118,8 +118,9 @@ class RealtimeModel:
         directions `dirs` [B,3] (eval_rt.py:106-122); also returns the number of
         host rounds.  mode:
           "tc"     (default) the reference's loop of aabb_intersect, then rounds
-                   of ray_march + the tensor-core decoder (dv_mlp_eval_tc,
-                   FP32-grade) until every pixel is finished
+                   of ray_march + the tensor-core decoder (FP32-grade) until every
+                   pixel is finished, each over the pixels still alive
+                   (dv_realtime_begin, dv_march_live, dv_mlp_eval_live)
           "fused"  the whole frame in one launch with the FP32 decoder
                    (dv_realtime_frame)
           "loop"   the reference's loop with the FP32 decoder (dv_mlp_eval);
@@ -142,35 +143,59 @@ class RealtimeModel:
                    N.ptr(self.features), N.ptr(self.voxel_map), self.voxel_map.shape[0], N.ptr(self.packed),
                    N.ptr(rgba), N.stream(dev))
             return rgba[:, :3] + rgba[:, 3:], 1
-        coords = torch.zeros(8, B, 6, device=dev)
-        rgba = torch.zeros(B, 4, device=dev)
-        finish = torch.zeros(B, dtype=torch.bool, device=dev)
-        aabb_intersect(coords, v, center, finish, rgba, self.octrees, self.voxel_num)
         rounds = 0
         limit = max_rounds if max_rounds is not None else 3 * self.voxel_num
         if mode == "loop":
+            coords = torch.zeros(8, B, 6, device=dev)
+            rgba = torch.zeros(B, 4, device=dev)
+            finish = torch.zeros(B, dtype=torch.bool, device=dev)
+            aabb_intersect(coords, v, center, finish, rgba, self.octrees, self.voxel_num)
             while rounds < limit and not bool(finish.all()):
                 ray_march(coords, v, self.voxel_masks, finish, self.voxel_num)
                 self.mlp_eval(rgba, coords, v, finish, False)
                 rounds += 1
             return rgba[:, :3] + rgba[:, 3:], rounds
-        # "tc": the host learns one round late that every pixel has finished, so
-        # round k + 1 is queued while it waits for round k's flag (a round after
-        # the last pixel finished changes nothing; the frame is the same, the
+        # "tc": every round goes over the pixels still alive, a list that the
+        # previous round made on the device.  The host learns one round late that
+        # it is empty, so round k + 1 is queued while it waits for round k's count
+        # (a round over an empty list changes nothing; the frame is the same, the
         # round count at most one higher)
+        n = self.voxel_num
+        N.need_cuda("dirs", v, torch.float32)
+        N.need_cuda("center", center, torch.float32)
+        m8, o8 = _u8("mask", self.voxel_masks), _u8("octrees", self.octrees)
+        if n % 64 != 0 or o8.numel() != (n // 64) ** 3 + (n // 16) ** 3 + (n // 4) ** 3 or m8.numel() != n ** 3:
+            raise ValueError(f"voxel_num {n} must be a multiple of 64, with {n}^3 mask cells and their octree levels")
+        rgba = torch.empty(B, 4, device=dev)
+        if B == 0:
+            return rgba[:, :3] + rgba[:, 3:], 0
+        limit = max(0, min(limit, 3 * n + 4))  # a round takes at least one grid plane per live pixel
+        hits = torch.empty(8, B, 6, device=dev)
+        resume = torch.empty(B, 3, device=dev)
+        lists = torch.empty(2, B, dtype=torch.int32, device=dev)
+        counts = torch.zeros(limit + 1, dtype=torch.int32, device=dev)
+        blob = self.tc_blob()
+        st = N.stream(dev)
+        N.call("dv_realtime_begin", B, N.ptr(v), N.ptr(center), N.ptr(o8), n, N.ptr(resume), N.ptr(rgba),
+               N.ptr(lists[0]), N.ptr(counts), st)
         if getattr(self, "_flags", None) is None:
-            self._flags = (torch.zeros(2, dtype=torch.bool, pin_memory=True), [torch.cuda.Event(), torch.cuda.Event()])
-        flags, events = self._flags
+            self._flags = (torch.zeros(2, dtype=torch.int32, pin_memory=True), [torch.cuda.Event(), torch.cuda.Event()])
+        left, events = self._flags
         while rounds < limit:
-            ray_march(coords, v, self.voxel_masks, finish, self.voxel_num)
-            self.mlp_eval(rgba, coords, v, finish, True)
+            live, after = lists[rounds % 2], lists[1 - rounds % 2]
+            count = counts.data_ptr() + 4 * rounds
+            N.call("dv_march_live", B, N.ptr(live), count, N.ptr(hits), N.ptr(resume), N.ptr(v), N.ptr(m8),
+                   n, st)
+            N.call("dv_mlp_eval_live", self.width, B, N.ptr(live), count, N.ptr(hits), N.ptr(self.features),
+                   N.ptr(self.voxel_map), self.voxel_map.shape[0], N.ptr(self.packed), N.ptr(blob), N.ptr(v),
+                   N.ptr(rgba), N.ptr(after), count + 4, N.ptr(self.tc_err), st)
             rounds += 1
             slot = rounds % 2
-            flags[slot:slot + 1].copy_(finish.all().reshape(1), non_blocking=True)
+            left[slot:slot + 1].copy_(counts[rounds:rounds + 1], non_blocking=True)
             events[slot].record()
             if rounds >= 2:
                 events[1 - slot].synchronize()
-                if bool(flags[1 - slot]):
+                if int(left[1 - slot]) == 0:
                     break
         return rgba[:, :3] + rgba[:, 3:], rounds
 

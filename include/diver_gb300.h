@@ -541,6 +541,28 @@ DV_API int dv_mlp_eval_tc(int width, int batch_size, const float* coords, const 
                           void* stream);
 
 /*
+ * The frame loop over its live pixels (no counterpart calls in the reference,
+ * whose rounds go over every pixel).  list holds the pixels still alive, in
+ * any order, and *count (device) how many; hits [8][capacity][6] are stored by
+ * list position, resume [batch][3] and rgba [batch][4] by pixel.
+ *   dv_realtime_begin  dv_aabb_intersect for every pixel: rgba = (0, 0, 0, 1),
+ *                      the first resume points, the first list (*count must be 0)
+ *   dv_march_live      dv_ray_march for the listed pixels: their next hits (x of
+ *                      the entry -1 after the last) and resume points
+ *   dv_mlp_eval_live   dv_mlp_eval_tc for the listed pixels; those not finished
+ *                      are appended to next (*next_count must be 0)
+ * A round changes a pixel exactly as dv_ray_march + dv_mlp_eval_tc do.
+ */
+DV_API int dv_realtime_begin(int batch_size, const float* v, const float* center, const uint8_t* octrees, int voxel_num,
+                             float* resume, float* rgba, int* list, int* count, void* stream);
+DV_API int dv_march_live(int capacity, const int* list, const int* count, float* hits, float* resume, const float* v,
+                         const uint8_t* mask, int voxel_num, void* stream);
+DV_API int dv_mlp_eval_live(int width, int capacity, const int* list, const int* count, const float* hits,
+                            const float* voxels, const int* voxel_map, int map_size, const float* packed_params,
+                            const void* tc_blob, const float* v, float* rgba, int* next, int* next_count, int* err,
+                            void* stream);
+
+/*
  * Whole real-time frame in one launch (no counterpart call in the reference,
  * whose eval_rt.py:115-122 loops on the host: dv_aabb_intersect, then rounds
  * of dv_ray_march + dv_mlp_eval until every pixel is finished).  Per pixel:
