@@ -217,30 +217,37 @@ __device__ __forceinline__ void integrate_tile(const Args& a, const float* sHit,
                                                uint32_t tstride) {
   const int t = threadIdx.x, q = t & 7, first = (t & ~31) + ((t & 31) >> 3);
 #pragma unroll 1
-  for (int p = 0; p < 8; ++p) {
-    const int row = first + 4 * p;
-    const float* h = sHit + row * HIT;
-    float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
-    const int4 ra = *reinterpret_cast<const int4*>(h + 8);
-    if (ra.x >= 0) {
-      const int4 rb = *reinterpret_cast<const int4*>(h + 12);
-      const int rows[8] = {ra.x, ra.y, ra.z, ra.w, rb.x, rb.y, rb.z, rb.w};
-      float4 v[8];
+  for (int p = 0; p < 8; p += 2) {  // two rows' loads in flight; a row without a hit reads the table's first
+    float4 v[2][8];
+    bool has[2];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = __ldg(reinterpret_cast<const float4*>(a.feats + (long long)rows[j] * 32) + q);
+    for (int u = 0; u < 2; ++u) {
+      const float* h = sHit + (first + 4 * (p + u)) * HIT;
+      const int4 ra = *reinterpret_cast<const int4*>(h + 8), rb = *reinterpret_cast<const int4*>(h + 12);
+      const int rows[8] = {ra.x, ra.y, ra.z, ra.w, rb.x, rb.y, rb.z, rb.w};
+      has[u] = ra.x >= 0;
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        v[u][j] = __ldg(reinterpret_cast<const float4*>(a.feats + (long long)(has[u] ? rows[j] : 0) * 32) + q);
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int row = first + 4 * (p + u);
+      const float* h = sHit + row * HIT;
       const float4 wa = *reinterpret_cast<const float4*>(h), wb = *reinterpret_cast<const float4*>(h + 4);
       const float w[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
-      if (FIRST) f = *reinterpret_cast<const float4*>(b_in + 4 * q);
+      float4 f = FIRST ? *reinterpret_cast<const float4*>(b_in + 4 * q) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) fma4(f, w[j], v[j]);
+      for (int j = 0; j < 8; ++j) fma4(f, w[j], v[u][j]);
       if (FIRST) f = make_float4(fmaxf(f.x, 0.f), fmaxf(f.y, 0.f), fmaxf(f.z, 0.f), fmaxf(f.w, 0.f));
-    }
-    uint32_t x[3], y[3];
-    tc::split_pair<3>(f.x, f.y, x);
-    tc::split_pair<3>(f.z, f.w, y);
-    uint8_t* dst = sA + tc::kmajor_offset(row, 4 * q, 32);
+      if (!has[u]) f = make_float4(0.f, 0.f, 0.f, 0.f);
+      uint32_t x[3], y[3];
+      tc::split_pair<3>(f.x, f.y, x);
+      tc::split_pair<3>(f.z, f.w, y);
+      uint8_t* dst = sA + tc::kmajor_offset(row, 4 * q, 32);
 #pragma unroll
-    for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(dst + i * tstride) = make_uint2(x[i], y[i]);
+      for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(dst + i * tstride) = make_uint2(x[i], y[i]);
+    }
   }
 }
 
@@ -264,6 +271,8 @@ __global__ void __launch_bounds__(128, W == 32 ? 4 : 1) mlp_eval_tc_kernel(const
   using Bi = Bias<W>;
   constexpr int KMAX = W > 32 ? W : 32;
   constexpr uint32_t TSTRIDE = 128 * KMAX * 2;
+  constexpr uint32_t PECOL = 2 * I::n1;
+  static_assert(PECOL + W <= NCOLS, "the pixel constants fit behind two blocks of the widest layer");
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sB = smem;
   uint8_t* sA = smem + 3 * I::TERM;
@@ -307,26 +316,36 @@ __global__ void __launch_bounds__(128, W == 32 ? 4 : 1) mlp_eval_tc_kernel(const
     if (!__syncthreads_or(start)) continue;
     bool alive = start, fin = false;
     float4 acc = make_float4(0.f, 0.f, 0.f, 1.f);
-    float pe2[W];  // bias + PE part of mlp2's first layer for this pixel's direction (FP32)
-#pragma unroll
-    for (int j = 0; j < W; ++j) pe2[j] = 0.f;
-    if (start) {
-      acc = reinterpret_cast<const float4*>(a.rgba)[px];
+    // bias + PE part of mlp2's first layer for this pixel's direction (FP32),
+    // kept in the TMEM columns behind the layers' two blocks
+    {
       float pe[PE_PAD];
-      pos_enc(__ldg(a.v + 3 * px), __ldg(a.v + 3 * px + 1), __ldg(a.v + 3 * px + 2), pe);
-#pragma unroll
-      for (int j = 0; j < W; ++j) pe2[j] = __ldg(a.params + L::l2_b + j);
-#pragma unroll
-      for (int k = 0; k < PE_DIM; ++k) {
-#pragma unroll
-        for (int j = 0; j < W; j += 4) {
-          const float4 w = __ldg(reinterpret_cast<const float4*>(a.params + L::l2_pe + k * W + j));
-          pe2[j] = fmaf(pe[k], w.x, pe2[j]);
-          pe2[j + 1] = fmaf(pe[k], w.y, pe2[j + 1]);
-          pe2[j + 2] = fmaf(pe[k], w.z, pe2[j + 2]);
-          pe2[j + 3] = fmaf(pe[k], w.w, pe2[j + 3]);
-        }
+      if (start) {
+        acc = reinterpret_cast<const float4*>(a.rgba)[px];
+        pos_enc(__ldg(a.v + 3 * px), __ldg(a.v + 3 * px + 1), __ldg(a.v + 3 * px + 2), pe);
       }
+#pragma unroll 1
+      for (int c0 = 0; c0 < W; c0 += 16) {
+        float e[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) e[j] = start ? __ldg(a.params + L::l2_b + c0 + j) : 0.f;
+        if (start) {
+#pragma unroll
+          for (int k = 0; k < PE_DIM; ++k) {
+#pragma unroll
+            for (int j = 0; j < 16; j += 4) {
+              const float4 w = __ldg(reinterpret_cast<const float4*>(a.params + L::l2_pe + k * W + c0 + j));
+              e[j] = fmaf(pe[k], w.x, e[j]);
+              e[j + 1] = fmaf(pe[k], w.y, e[j + 1]);
+              e[j + 2] = fmaf(pe[k], w.z, e[j + 2]);
+              e[j + 3] = fmaf(pe[k], w.w, e[j + 3]);
+            }
+          }
+        }
+        __syncwarp();
+        tc::st_32x32b_x16(trow + PECOL + c0, reinterpret_cast<const uint32_t*>(e));
+      }
+      tc::st_wait();
     }
     // A wait that gave up is seen by all at the tile's end.
 #pragma unroll 1
@@ -376,8 +395,11 @@ __global__ void __launch_bounds__(128, W == 32 ? 4 : 1) mlp_eval_tc_kernel(const
 #pragma unroll
         for (int c0 = 0; c0 < W; c0 += 16) {
           row16(trow + c0, I::n1, v);
+          float e[16];
+          tc::ld_32x32b_x16(trow + PECOL + c0, e);
+          tc::ld_wait();
 #pragma unroll
-          for (int i = 0; i < 16; ++i) v[i] = fmaxf(v[i] + pe2[c0 + i], 0.f);
+          for (int i = 0; i < 16; ++i) v[i] = fmaxf(v[i] + e[i], 0.f);
           put_row3<W, 16>(sA + tc::kmajor_offset(0, c0, W), TSTRIDE, t, v);
         }
       }
