@@ -191,6 +191,46 @@ __device__ __forceinline__ void load_segs(const float* p, float* v) {
   }
 }
 
+// Accumulators of two consecutive segments as one packed pair.  The products
+// below run on packed FMAs, both halves with the same weight: half the issue
+// slots for the same rounding (2035-ray DIVeR32 step: backward 358 -> 341 us,
+// forward 115 -> 108 us).
+template <int M, int SPT>
+struct AccPairs {
+  unsigned long long v[M][SPT / 2];
+  __device__ __forceinline__ explicit AccPairs(const float (&a)[M][SPT]) {
+#pragma unroll
+    for (int m = 0; m < M; ++m)
+#pragma unroll
+      for (int s = 0; s < SPT; s += 2) v[m][s / 2] = f32x2(a[m][s], a[m][s + 1]);
+  }
+  __device__ __forceinline__ void to(float (&a)[M][SPT]) const {
+#pragma unroll
+    for (int m = 0; m < M; ++m)
+#pragma unroll
+      for (int s = 0; s < SPT; s += 2) {
+        const float2 f = f32x2_get(v[m][s / 2]);
+        a[m][s] = f.x;
+        a[m][s + 1] = f.y;
+      }
+  }
+  __device__ __forceinline__ void fma(int m, const unsigned long long (&x)[SPT / 2], float w) {
+    const unsigned long long ww = f32x2(w, w);
+#pragma unroll
+    for (int s = 0; s < SPT / 2; ++s) v[m][s] = fma_f32x2(x[s], ww, v[m][s]);
+  }
+};
+
+template <int N>
+__device__ __forceinline__ void load_pairs(const float* p, unsigned long long (&v)[N / 2]) {
+#pragma unroll
+  for (int i = 0; i < N; i += 4) {
+    const float4 x = *reinterpret_cast<const float4*>(p + i);
+    v[i / 2] = f32x2(x.x, x.y);
+    v[i / 2 + 1] = f32x2(x.z, x.w);
+  }
+}
+
 // acc[m][s] += sum over k of X[k][segment s] * wl[k][output tx + 8 m].
 template <int K, int W, int SEGS>
 __device__ __forceinline__ void layer_fwd(const float* X, const float* wl, float (&acc)[W / 8][SEGS / 4]) {
@@ -198,22 +238,21 @@ __device__ __forceinline__ void layer_fwd(const float* X, const float* wl, float
   const int lane = threadIdx.x & 31, tx = lane & 7, ty = lane >> 3;
   const float* xp = X + SPT * ty;
   const float* wp = wl + 4 * tx;
+  AccPairs<W / 8, SPT> c(acc);
 #pragma unroll 4
   for (int k = 0; k < K; ++k) {
-    float x[SPT];
-    load_segs<SPT>(xp + k * LD, x);
+    unsigned long long x[SPT / 2];
+    load_pairs<SPT>(xp + k * LD, x);
 #pragma unroll
     for (int h = 0; h < W / 32; ++h) {
       const float4 w = *reinterpret_cast<const float4*>(wp + k * LDW + 32 * h);
-#pragma unroll
-      for (int s = 0; s < SPT; ++s) {
-        acc[4 * h][s] = fmaf(x[s], w.x, acc[4 * h][s]);
-        acc[4 * h + 1][s] = fmaf(x[s], w.y, acc[4 * h + 1][s]);
-        acc[4 * h + 2][s] = fmaf(x[s], w.z, acc[4 * h + 2][s]);
-        acc[4 * h + 3][s] = fmaf(x[s], w.w, acc[4 * h + 3][s]);
-      }
+      c.fma(4 * h, x, w.x);
+      c.fma(4 * h + 1, x, w.y);
+      c.fma(4 * h + 2, x, w.z);
+      c.fma(4 * h + 3, x, w.w);
     }
   }
+  c.to(acc);
 }
 
 template <int M, int SPT>
@@ -373,25 +412,24 @@ __device__ __forceinline__ void layer_bwd(const float* D, const float* wl, float
   const int lane = threadIdx.x & 31, tx = lane & 7, ty = lane >> 3;
   const float* dp = D + SPT * ty;
   const float* wp = wl + tx * LDW;
+  AccPairs<K / 8, SPT> c(acc);
 #pragma unroll
   for (int h = 0; h < W / 32; ++h)
 #pragma unroll 2
     for (int g = 0; g < 8; ++g) {  // outputs 32 h + g + 8 i: 4 consecutive weights
-      float d[4][SPT];
+      unsigned long long d[4][SPT / 2];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) load_segs<SPT>(dp + (32 * h + 8 * i + g) * LD, d[i]);
+      for (int i = 0; i < 4; ++i) load_pairs<SPT>(dp + (32 * h + 8 * i + g) * LD, d[i]);
 #pragma unroll
       for (int m = 0; m < K / 8; ++m) {
         const float4 w = *reinterpret_cast<const float4*>(wp + 8 * m * LDW + 32 * h + 4 * g);
-#pragma unroll
-        for (int s = 0; s < SPT; ++s) {
-          acc[m][s] = fmaf(w.x, d[0][s], acc[m][s]);
-          acc[m][s] = fmaf(w.y, d[1][s], acc[m][s]);
-          acc[m][s] = fmaf(w.z, d[2][s], acc[m][s]);
-          acc[m][s] = fmaf(w.w, d[3][s], acc[m][s]);
-        }
+        c.fma(m, d[0], w.x);
+        c.fma(m, d[1], w.y);
+        c.fma(m, d[2], w.z);
+        c.fma(m, d[3], w.w);
       }
     }
+  c.to(acc);
 }
 
 // Writes the input gradients over the activation they belong to, zero where
