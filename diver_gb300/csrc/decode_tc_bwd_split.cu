@@ -7,7 +7,7 @@
 //   - weight gradient    dW += delta^T @ activation: two terms each, all four
 //     products (FP32 accumulators resident in TMEM for the CTA's life);
 //   - bias gradient      dB += delta^T @ ones: the column sums of the two-term
-//     delta, also accumulated in TMEM (layer 3's from a column of ones in the
+//     delta, also accumulated in TMEM (the PE layer's from a column of ones in the
 //     PE tile, which the weight-gradient MMA already reads).
 // Products are accumulated in FP32 in TMEM, so the propagated deltas and the
 // gradients keep about 2^-24 (propagation) and 2^-16 (weight gradients) of
@@ -28,8 +28,9 @@
 //     side by side along N: per 16 columns of K, delta_0 x [W0|W1] and
 //     delta_1 x [W0|W1] (N = 64), delta_0 x W2 into columns 32..63 and
 //     delta_2 x W0 into columns 0..31; the epilogue adds the two column blocks.
-// Per 128-segment tile that is 40 propagation, 48 weight-gradient and 32
-// bias-gradient MMAs.
+// Per 128-segment tile that is 32 propagation, 40 weight-gradient and 24
+// bias-gradient MMAs with mlp1's output layer and mlp2's first taken as one
+// (40, 48 and 32 layer by layer: see Cfg).
 //
 // The forward is not recomputed: dv_decode_fwd_tc_split saved, per tile of 128
 // segments, every layer's input as a [128][2 x 32] two-term tile (X0, A1, A2,
@@ -48,7 +49,7 @@
 // the other of two delta tiles.  A propagation's commit also covers the
 // gradient MMAs queued before it, which is what frees the delta tile and the
 // record slot of the layer before.
-// Shared memory (226 KiB): the propagation images, the saved record in five
+// Shared memory (at most 226 KiB): the propagation images, the saved record in
 // per-layer slots, the PE tile, two delta tiles, a tile of ones, the FP32
 // staging rows of the feature gradient and the scatter's corners.  TMEM: all 512
 // columns (64 working, 384 weight-gradient and 64 bias-gradient columns).
@@ -56,7 +57,8 @@
 // with the chain doing the scatter in its waits and every MMA of a layer ahead
 // of its epilogue, 625 us in this form with one thread issuing and stepping
 // with the chain, 522 us with the issuer's warp running free of it, 513 us with
-// the layer loops rolled (instruction cache).
+// the layer loops rolled (instruction cache), 489 us folded.  What is left is
+// the scatter: the same kernel without its atomics takes 330 us.
 // Reference semantics: the autograd backward of model/diver.py:159-180.
 #include "common.cuh"
 #include "integrate.cuh"
@@ -69,7 +71,6 @@ namespace dv {
 namespace bws {
 
 constexpr int C = 32, W = 32;
-constexpr int NL = 5;
 constexpr int CHAIN = 256;             // the layer chain's threads: two per segment row (warps 1-8)
 constexpr int CHAIN_ALL = CHAIN + 32;  // chain and issuer warp
 constexpr int SCATTER = 256;           // warps 9-16
@@ -78,24 +79,43 @@ constexpr int FD = 48;              // delta columns per term (K of the widest p
 constexpr int DW = 3 * FD;          // delta tile columns: the three terms side by side
 constexpr int TILE = 128 * 32 * 2;  // one term of a [128][32] BF16 tile
 constexpr int DTILE = 128 * FD * 2; // one term's share of the delta tile
-constexpr int TMEM_COLS = 512;      // 64 working + 384 weight-gradient + 64 bias-gradient columns
-// layer: 0 (C->W), 1 (W->W), 2 (W->W+1: sigma, hidden), 3 (W+27->W), 4 (W->3)
-__host__ __device__ constexpr int IN(int l) { return l == 0 ? C : (l == 3 ? W + PE_DIM : W); }
-__host__ __device__ constexpr int OUT(int l) { return l == 2 ? W + 1 : (l == 4 ? 3 : W); }
-__host__ __device__ constexpr int OUT4(int l) { return pad4(OUT(l)); }
-__host__ __device__ constexpr int NBLK(int l) { return l == 3 ? 2 : 1; }  // 32-column input blocks (layer 3: + PE)
-// weight gradient of layer l: per input block, 64 columns (activation terms 0 and 1)
-__host__ __device__ constexpr int DWCOL(int l) { return 64 + 64 * l + (l > 3 ? 64 : 0); }
-// bias gradient of layer l != 3 (column 0 of 16); layer 3's is column 27 of its PE block
-__host__ __device__ constexpr int DBCOL(int l) { return 448 + 16 * (l < 3 ? l : l - 1); }
-constexpr int PE_ONES = 27;  // the PE tile's column of ones (PE_DIM = 27 values before it)
-__host__ __device__ constexpr int KPROP(int l) { return l == 4 ? 16 : (l == 2 ? W + 16 : W); }  // propagation K
-// propagation image of layer l in shared memory: [3 terms x 32 rows][KPROP(l)],
-// the three terms side by side along N, layers one after the other
-__host__ __device__ constexpr int PIMG(int l) { return 32 * KPROP(l) * 2; }  // one term's bytes
-__host__ __device__ constexpr int POFF(int l) { return 3 * 64 * (32 * l + (l > 2 ? 16 : 0) - (l > 4 ? 16 : 0)); }
-static_assert(POFF(3) == POFF(2) + 3 * PIMG(2) && POFF(5) == POFF(4) + 3 * PIMG(4), "images one after the other");
-static_assert(DWCOL(4) == DWCOL(3) + 64 * NBLK(3), "gradient blocks one after the other");
+constexpr int TMEM_COLS = 512;      // 64 working columns, the weight and the bias gradients
+constexpr int PE_ONES = 27;         // the PE tile's column of ones (PE_DIM = 27 values before it)
+
+// The layers that the chain steps through, last to first.
+//
+// Plain: the decoder's own five, 0 (C->W), 1 (W->W), 2 (W->W+1: sigma,
+// hidden), 3 (W+27->W), 4 (W->3).
+//
+// Folded: mlp1's output layer has no activation, so its hidden part WH and
+// mlp2's first layer W2 act as one matrix WF = WH W2, and the steps are
+// 0 (C->W), 1 (W->W), 2 (A2 and PE -> sigma and mlp2's hidden), 3 (W->3): a
+// fifth less of the MMAs, hand-overs and record bytes.  With delta the
+// gradient after WF and GF = A2^T delta,
+//   dL/dWH = GF W2^T,   dL/dW2 = WH^T GF + bh (sum delta)^T,   dL/dbh = W2 (sum delta),
+// once per CTA.  The forward keeps the two layers, so its ReLU decisions stand.
+template <bool FOLD>
+struct Cfg {
+  static constexpr int NL = FOLD ? 4 : 5;
+  static constexpr int PEL = FOLD ? 2 : 3;  // the layer with the PE rows; its bias gradient is column 27 of its PE block
+  __host__ __device__ static constexpr int REC(int l) { return FOLD && l == 3 ? 4 : l; }  // its input's tile in the record
+  __host__ __device__ static constexpr int IN(int l) { return l == 0 ? C : (l == PEL ? W + PE_DIM : W); }
+  __host__ __device__ static constexpr int OUT(int l) { return l == 2 ? W + 1 : (l == NL - 1 ? 3 : W); }
+  __host__ __device__ static constexpr int OUT4(int l) { return pad4(OUT(l)); }
+  __host__ __device__ static constexpr int NBLK(int l) { return l == PEL ? 2 : 1; }  // 32-column input blocks
+  // weight gradient of layer l: per input block, 64 columns (activation terms 0 and 1)
+  __host__ __device__ static constexpr int DWCOL(int l) { return 64 + 64 * l + (l > PEL ? 64 : 0); }
+  // bias gradient of layer l != PEL (column 0 of 16)
+  __host__ __device__ static constexpr int DBCOL(int l) { return 64 + 64 * (NL + 1) + 16 * (l < PEL ? l : l - 1); }
+  __host__ __device__ static constexpr int KPROP(int l) { return l == NL - 1 ? 16 : (l == 2 ? W + 16 : W); }  // propagation K
+  // propagation image of layer l in shared memory: [3 terms x 32 rows][KPROP(l)],
+  // the three terms side by side along N, layers one after the other
+  __host__ __device__ static constexpr int PIMG(int l) { return 32 * KPROP(l) * 2; }  // one term's bytes
+  __host__ __device__ static constexpr int POFF(int l) {
+    return 3 * 64 * (32 * l + (l > 2 ? 16 : 0) - (l >= NL ? 16 : 0));
+  }
+};
+
 constexpr uint32_t RECORD = 5 * 2 * TILE;  // saved record of one tile: 5 layer inputs, [128][2 x 32] each
 constexpr uint32_t ONES_BYTES = 128 * 16 * 2;  // a [128][16] BF16 tile of ones
 constexpr int COEF = 12;                       // floats per segment: 8 corner weights, lower corner's row, row steps
@@ -113,21 +133,24 @@ struct Args {
   float* grad_grid;
   float* grad_params;    // packed torch layout
   uint8_t* touched;      // optional: a byte per grid row, set at each segment's lower corner
-  int w_off[NL], b_off[NL];
+  int w_off[5], b_off[5];  // of the decoder's own layers
   const uint8_t* wb;     // transposed weight images, three terms of wterm bytes
   int wterm;
-  int b_img[NL];         // byte offset of layer l's image inside a term
+  int b_img[5];          // byte offset of layer l's image inside a term
+  const float* params;   // folded: the packed parameters
   int* err;
 };
 
-// Shared-memory layout (byte offsets; the propagation images take 3 x 10240 bytes).
+// Shared-memory layout (byte offsets).
+template <bool FOLD>
 struct Layout {
+  using P = Cfg<FOLD>;
   uint32_t bb, rec, pe, d, ones, stage, coef, bar;
   __host__ __device__ static Layout make() {
     Layout L;
     L.bb = 0;
-    L.rec = (uint32_t)(POFF(NL) + 1023) / 1024 * 1024;
-    L.pe = L.rec + RECORD;
+    L.rec = (uint32_t)(P::POFF(P::NL) + 1023) / 1024 * 1024;
+    L.pe = L.rec + P::NL * 2 * TILE;
     L.d = L.pe + 2 * TILE;
     L.ones = L.d + 2 * 3 * DTILE;
     L.stage = L.ones + ONES_BYTES;
@@ -136,7 +159,7 @@ struct Layout {
     return L;
   }
   // barriers: propagation, NL record slots, the last MMAs; then the TMEM address and the stop flag
-  __host__ __device__ uint32_t bytes() const { return bar + 8 * (2 + NL) + 16; }
+  __host__ __device__ uint32_t bytes() const { return bar + 8 * (2 + P::NL) + 16; }
 };
 
 // Writes n values (multiple of 8) of row r, columns c0.., as three BF16 terms
@@ -360,7 +383,7 @@ __device__ __forceinline__ void delta_ready() {
 }
 
 // PE tile row r, columns 16h..16h+15 (PE_DIM = 27 values, then a one in
-// column PE_ONES for layer 3's bias gradient, zeros after), two terms.
+// column PE_ONES for the layer's bias gradient, zeros after), two terms.
 __device__ __forceinline__ void load_pe(const Args& a, int ray, int h, float* v) {
   const float* pf = a.pe_feat + (long long)ray * PE_PAD + 16 * h;
 #pragma unroll
@@ -395,7 +418,7 @@ __device__ __forceinline__ void prop_row32(uint32_t taddr, float* v) {
   prop_row16(taddr + 16, v + 16);
 }
 
-// One tile per step of the persistent loop: the five layer steps, each the
+// One tile per step of the persistent loop: the layer steps, each the
 // propagation, its gradient MMAs and the epilogue that forms the next delta;
 // the last stages the tile's feature gradient (FP32) for the scatter group.
 // The saved record sits in five per-layer slots, each with its own mbarrier: a
@@ -404,9 +427,15 @@ __device__ __forceinline__ void prop_row32(uint32_t taddr, float* v) {
 // reads from global memory for the next tile (ray, PE row, the first delta's
 // inputs) is loaded before a wait and used after it.  Waits are bounded: a
 // thread whose wait gave up goes on through the tile, and all stop at its end.
+template <bool FOLD>
 __global__ void __launch_bounds__(THREADS, 1) decode_bwd_tc_split_kernel(const Args a) {
+  using P = Cfg<FOLD>;
+  constexpr int NL = P::NL, PEL = P::PEL;
+  static_assert(P::POFF(3) == P::POFF(2) + 3 * P::PIMG(2) && P::POFF(NL) == P::POFF(NL - 1) + 3 * P::PIMG(NL - 1),
+                "images one after the other");
+  static_assert(P::DBCOL(NL - 1) + 16 <= TMEM_COLS, "TMEM columns");
   extern __shared__ __align__(1024) uint8_t smem[];
-  const Layout lay = Layout::make();
+  const Layout<FOLD> lay = Layout<FOLD>::make();
   uint8_t* Bb = smem + lay.bb;
   uint8_t* REC = smem + lay.rec;
   uint8_t* PE = smem + lay.pe;
@@ -426,9 +455,9 @@ __global__ void __launch_bounds__(THREADS, 1) decode_bwd_tc_split_kernel(const A
   // propagation images, regrouped layer by layer with the three terms side by side
 #pragma unroll
   for (int l = 0; l < NL; ++l)
-    for (int i = t; i < 3 * PIMG(l) / 16; i += THREADS) {
-      const int j = i / (PIMG(l) / 16), o = i % (PIMG(l) / 16);
-      reinterpret_cast<uint4*>(Bb + POFF(l))[i] =
+    for (int i = t; i < 3 * P::PIMG(l) / 16; i += THREADS) {
+      const int j = i / (P::PIMG(l) / 16), o = i % (P::PIMG(l) / 16);
+      reinterpret_cast<uint4*>(Bb + P::POFF(l))[i] =
           __ldg(reinterpret_cast<const uint4*>(a.wb + j * a.wterm + a.b_img[l]) + o);
     }
   for (int i = t; i < 2 * 3 * DTILE / 16; i += THREADS) reinterpret_cast<uint4*>(smem + lay.d)[i] = make_uint4(0, 0, 0, 0);
@@ -461,7 +490,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_bwd_tc_split_kernel(const A
     auto load_slot = [&](int l, long long tile) {
       if (by) {
         tc::mbar_arrive_expect_tx(bar_rec + l, 2 * TILE);
-        tc::bulk_load(REC + l * 2 * TILE, a.saved + tile * (long long)RECORD + l * 2 * TILE, 2 * TILE, bar_rec + l);
+        tc::bulk_load(REC + l * 2 * TILE, a.saved + tile * (long long)RECORD + P::REC(l) * 2 * TILE, 2 * TILE, bar_rec + l);
       }
       pending |= 1u << l;
     };
@@ -474,7 +503,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_bwd_tc_split_kernel(const A
         const uint8_t* D = smem + lay.d + db * (3 * DTILE);
         named_sync(BAR_DELTA, CHAIN_ALL);  // this delta is in place; the previous propagation was waited for
         tc::fence_after_sync();
-        mma_prop(by, tmem, D, Bb + POFF(l), KPROP(l));
+        mma_prop(by, tmem, D, Bb + P::POFF(l), P::KPROP(l));
         tc::mma_commit_by(by, bar);
         // that propagation's commit covered the gradient MMAs of two steps ago: their slot takes
         // its next input (layers 0 and 1: this tile's)
@@ -485,11 +514,11 @@ __global__ void __launch_bounds__(THREADS, 1) decode_bwd_tc_split_kernel(const A
           phase_rec ^= 1u << l;
           pending &= ~(1u << l);
           const uint8_t* act = REC + l * 2 * TILE;  // this layer's input, two terms TILE apart
-          mma_dw(by, tmem + DWCOL(l), D, act, !first);
-          if (l == 3)
-            mma_dw(by, tmem + DWCOL(3) + 64, D, PE, !first);  // with layer 3's bias gradient (the ones column)
+          mma_dw(by, tmem + P::DWCOL(l), D, act, !first);
+          if (l == PEL)
+            mma_dw(by, tmem + P::DWCOL(PEL) + 64, D, PE, !first);  // with its bias gradient (the ones column)
           else
-            mma_db(by, tmem + DBCOL(l), D, ONES, !first);
+            mma_db(by, tmem + P::DBCOL(l), D, ONES, !first);
         }
         ok &= arrived;
         db ^= 1u;
@@ -554,7 +583,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_bwd_tc_split_kernel(const A
       for (int l = NL - 1; l >= 0; --l) {
         const uint8_t* act = REC + l * 2 * TILE;  // this layer's input, two terms TILE apart
         uint8_t* Dn = smem + lay.d + (db ^ 1u) * (3 * DTILE);
-        if (l == 2 && next < tiles) load_pe(a, ray_next, h, pe);
+        if (l == PEL - 1 && next < tiles) load_pe(a, ray_next, h, pe);
         if (l == 1 && valid_next && h == 0) {
           gn = a.d4[sn];
           on = a.out4[sn];
@@ -566,9 +595,10 @@ __global__ void __launch_bounds__(THREADS, 1) decode_bwd_tc_split_kernel(const A
         phase ^= 1u;
         tc::fence_after_sync();
         if (l == 3) {
-          // delta of layer 2: (dL/dsigma, d hidden[0..31]) in columns 0..32, zeros to 47;
-          // half 0 writes columns 0..23, half 1 columns 24..47
+          // delta of layer 2: (dL/dsigma, that of its other 32 outputs) in columns 0..32, zeros to
+          // 47; half 0 writes columns 0..23, half 1 columns 24..47
           prop_row32(trow, v);
+          if (FOLD) relu_mask(act, r, 0, v, 32);
           float w[24];
           if (h == 0) {
             w[0] = gx;
@@ -583,8 +613,8 @@ __global__ void __launch_bounds__(THREADS, 1) decode_bwd_tc_split_kernel(const A
           prop_row16(trow + 16 * h, v);
           relu_mask(act, r, 16 * h, v, 16);  // this layer's input is relu of the previous layer's output
           put3(Dn, r, 16 * h, v, 16);
-          // layer 3's gradient MMAs are done with this tile's PE: the next tile's goes in
-          if (l == 2 && next < tiles) put2(PE, r, 16 * h, pe, 16);
+          // layer PEL's gradient MMAs are done with this tile's PE: the next tile's goes in
+          if (l == PEL - 1 && next < tiles) put2(PE, r, 16 * h, pe, 16);
         } else {
           // the next tile's first delta; then dL/dfeature (FP32) to the staging rows, once the
           // scatter group has taken the last tile's
@@ -621,29 +651,84 @@ __global__ void __launch_bounds__(THREADS, 1) decode_bwd_tc_split_kernel(const A
     if (ok && !first) {
       const int o = r < FD ? r : r - FD;
       const bool row = r < 2 * FD;
+      // folded: GF (row o: output o, sigma first), W2 and WH in shared memory (the records' part)
+      constexpr int LD = W + 1;
+      float* G = reinterpret_cast<float*>(REC);  // [W + 1][LD]
+      float* W2 = G + LD * LD;                   // [h][j]
+      float* WH = W2 + W * LD;                   // [i][h]
+      float* DB = WH + W * LD;                   // sum of delta [W]
+      const int ct = t - 32;                     // this thread's number in the chain
+      if (FOLD) {
+        for (int i = ct; i < (W + 1) * LD; i += CHAIN) G[i] = 0.f;
+        for (int i = ct; i < W; i += CHAIN) DB[i] = 0.f;
+        for (int i = ct; i < W * W; i += CHAIN) {
+          const int x = i / W, y = i % W;
+          W2[x * LD + y] = __ldg(a.params + a.w_off[3] + i);
+          WH[x * LD + y] = __ldg(a.params + a.w_off[2] + x * (W + 4) + 1 + y);
+        }
+        named_sync(BAR_CHAIN, CHAIN);
+      }
 #pragma unroll
       for (int l = 0; l < NL; ++l) {
+        const int ol = FOLD && l == 3 ? 4 : l;  // the decoder's own layer (the folded one: see below)
 #pragma unroll
-        for (int b = 0; b < NBLK(l); ++b) {
+        for (int b = 0; b < P::NBLK(l); ++b) {
           float u[16];
-          tc::ld_32x32b_x16(tmem + lane + DWCOL(l) + 64 * b + 16 * h, v);
-          tc::ld_32x32b_x16(tmem + lane + DWCOL(l) + 64 * b + 32 + 16 * h, u);
+          tc::ld_32x32b_x16(tmem + lane + P::DWCOL(l) + 64 * b + 16 * h, v);
+          tc::ld_32x32b_x16(tmem + lane + P::DWCOL(l) + 64 * b + 32 + 16 * h, u);
           tc::ld_wait();
-          if (row && o < OUT(l)) {
+          if (row && o < P::OUT(l)) {
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
               const int c = 32 * b + 16 * h + i;
-              if (c < IN(l)) atomicAdd(a.grad_params + a.w_off[l] + c * OUT4(l) + o, v[i] + u[i]);
+              if (c >= P::IN(l)) continue;
+              if (!FOLD || l != 2) {
+                atomicAdd(a.grad_params + a.w_off[ol] + c * pad4(P::OUT(l)) + o, v[i] + u[i]);
+              } else if (b == 0) {
+                atomicAdd(G + o * LD + c, v[i] + u[i]);
+              } else if (o > 0) {  // PE rows of mlp2's first layer
+                atomicAdd(a.grad_params + a.w_off[3] + c * W + o - 1, v[i] + u[i]);
+              }
             }
-            // layer 3's bias gradient: the PE block's column of ones
-            if (l == 3 && b == 1 && h == 1)
-              atomicAdd(a.grad_params + a.b_off[l] + o, v[PE_ONES - 16] + u[PE_ONES - 16]);
+            // the PE block's column of ones
+            if (l == PEL && b == 1 && h == 1) {
+              const float sum = v[PE_ONES - 16] + u[PE_ONES - 16];
+              if (!FOLD) {
+                atomicAdd(a.grad_params + a.b_off[l] + o, sum);
+              } else if (o == 0) {
+                atomicAdd(a.grad_params + a.b_off[2], sum);
+              } else {
+                atomicAdd(a.grad_params + a.b_off[3] + o - 1, sum);
+                atomicAdd(DB + o - 1, sum);
+              }
+            }
           }
         }
-        if (l != 3 && h == 0) {
-          tc::ld_32x32b_x16(tmem + lane + DBCOL(l), v);
+        if (l != PEL && h == 0) {
+          tc::ld_32x32b_x16(tmem + lane + P::DBCOL(l), v);
           tc::ld_wait();
-          if (row && o < OUT(l)) atomicAdd(a.grad_params + a.b_off[l] + o, v[0]);
+          if (row && o < P::OUT(l)) atomicAdd(a.grad_params + a.b_off[ol] + o, v[0]);
+        }
+      }
+      if (FOLD) {
+        named_sync(BAR_CHAIN, CHAIN);
+        for (int e = ct; e < W * W; e += CHAIN) {
+          const int x = e / W, y = e % W;
+          // dL/dWH[i = x][h = y] and dL/dW2[h = x][j = y]
+          float wh = 0.f, w2 = __ldg(a.params + a.b_off[2] + 1 + x) * DB[y];
+#pragma unroll 4
+          for (int k = 0; k < W; ++k) {
+            wh = fmaf(G[(1 + k) * LD + x], W2[y * LD + k], wh);
+            w2 = fmaf(WH[k * LD + x], G[(1 + y) * LD + k], w2);
+          }
+          atomicAdd(a.grad_params + a.w_off[2] + x * (W + 4) + 1 + y, wh);
+          atomicAdd(a.grad_params + a.w_off[3] + e, w2);
+        }
+        if (ct < W) {
+          float bh = 0.f;
+          for (int j = 0; j < W; ++j) bh = fmaf(W2[ct * LD + j], DB[j], bh);
+          atomicAdd(a.grad_params + a.b_off[2] + 1 + ct, bh);
+          atomicAdd(a.grad_params + a.w_off[2] + ct * (W + 4), G[ct]);  // sigma's column
         }
       }
     }
@@ -654,24 +739,45 @@ __global__ void __launch_bounds__(THREADS, 1) decode_bwd_tc_split_kernel(const A
   if (warp == 0) tc::tmem_dealloc(tmem, TMEM_COLS);
 }
 
+// folded [n + W W]: the packed parameters, then WF[i][j] = sum_h WH[i][h] W2[h][j].
+__global__ void __launch_bounds__(256) fold_params_kernel(const float* __restrict__ params, int n,
+                                                          float* __restrict__ folded) {
+  constexpr int wh = C * W + W + W * W + W;                          // mlp1's output layer (rows of W + 4, sigma first)
+  constexpr int w2 = wh + W * (W + 4) + (W + 4);                     // mlp2's first layer
+  const int copies = (n + 255) / 256;
+  if ((int)blockIdx.x < copies) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i < n) folded[i] = __ldg(params + i);
+    return;
+  }
+  const int e = (blockIdx.x - copies) * 256 + threadIdx.x;  // four blocks
+  float f = 0.f;
+#pragma unroll 8
+  for (int h = 0; h < W; ++h)
+    f = fmaf(__ldg(params + wh + (e / W) * (W + 4) + 1 + h), __ldg(params + w2 + h * W + e % W), f);
+  folded[n + e] = f;
+}
+
 }  // namespace bws
 }  // namespace dv
 
 using namespace dv;
 
-extern "C" {
-
-int dv_decode_bwd_tc_split(int kind, int channels, const void* wb, int wb_term_bytes, const int* b_layers,
-                           int n_layers, int nvx, int nvy, int nvz, const float* seg, const int* seg_ray,
-                           long long n_seg, const int64_t* n_seg_dev, const float* pe_feat, const float* d4,
-                           const void* saved, long long saved_bytes, const float* out4, float* grad_voxels,
-                           float* grad_params, unsigned char* touched, int* err, void* stream) {
+// Checks the arguments of a split backward launch and starts it; params: folded.
+template <bool FOLD>
+static int bwd_split(int kind, int channels, const float* params, const void* wb, int wb_term_bytes, const int* b_layers,
+                     int n_layers, int nvx, int nvy, int nvz, const float* seg, const int* seg_ray, long long n_seg,
+                     const int64_t* n_seg_dev, const float* pe_feat, const float* d4, const void* saved,
+                     long long saved_bytes, const float* out4, float* grad_voxels, float* grad_params,
+                     unsigned char* touched, int* err, void* stream) {
   using namespace dv::bws;
+  using P = Cfg<FOLD>;
   DV_CHECK(n_seg >= 0, DV_ERR_ARG);
-  DV_CHECK(kind == 32 && channels == 32 && n_layers == NL, DV_ERR_UNSUPPORTED);
+  DV_CHECK(kind == 32 && channels == 32 && n_layers == P::NL, DV_ERR_UNSUPPORTED);
   if (n_seg == 0) return DV_OK;
   DV_CHECK(wb && b_layers && seg && seg_ray && pe_feat && d4 && saved && out4 && grad_voxels && grad_params,
            DV_ERR_ARG);
+  DV_CHECK(params || !FOLD, DV_ERR_ARG);
   DV_CHECK(nvx > 0 && nvy > 0 && nvz > 0 && wb_term_bytes > 0 && wb_term_bytes % 16 == 0, DV_ERR_ARG);
   DV_CHECK(((uintptr_t)wb & 15) == 0 && ((uintptr_t)saved & 15) == 0 && ((uintptr_t)out4 & 15) == 0 &&
                ((uintptr_t)grad_voxels & 15) == 0 && ((uintptr_t)d4 & 15) == 0,
@@ -695,27 +801,28 @@ int dv_decode_bwd_tc_split(int kind, int channels, const void* wb, int wb_term_b
   a.wb = reinterpret_cast<const uint8_t*>(wb);
   a.wterm = wb_term_bytes;
   a.err = err;
+  a.params = params;
   // packed torch layout offsets (same rule as dv_decoder_param_count)
   {
     int off = 0;
-    const int outs[NL] = {W, W, W + 1, W, 3};
-    for (int l = 0; l < NL; ++l) {
+    const int ins[5] = {C, W, W, W + PE_DIM, W}, outs[5] = {W, W, W + 1, W, 3};
+    for (int l = 0; l < 5; ++l) {
       a.w_off[l] = off;
-      a.b_off[l] = off + IN(l) * pad4(outs[l]);
+      a.b_off[l] = off + ins[l] * pad4(outs[l]);
       off = a.b_off[l] + pad4(outs[l]);
     }
   }
   // transposed images [N = in][K = out padded to 16], inside one term
-  const int bK[NL] = {W, W, W + 16, W, 16}, bN[NL] = {C, W, W, W, W};
-  for (int l = 0; l < NL; ++l) {
+  for (int l = 0; l < P::NL; ++l) {
+    const int n = l == 0 ? C : W;
     a.b_img[l] = b_layers[3 * l];
-    DV_CHECK(b_layers[3 * l + 1] == bK[l] && b_layers[3 * l + 2] == bN[l] && bK[l] == KPROP(l), DV_ERR_ARG);
+    DV_CHECK(b_layers[3 * l + 1] == P::KPROP(l) && b_layers[3 * l + 2] == n, DV_ERR_ARG);
     DV_CHECK(a.b_img[l] % 16 == 0 && a.b_img[l] >= 0, DV_ERR_ARG);
-    DV_CHECK((long long)a.b_img[l] + (long long)bK[l] * bN[l] * 2 <= wb_term_bytes, DV_ERR_ARG);
+    DV_CHECK((long long)a.b_img[l] + (long long)P::KPROP(l) * n * 2 <= wb_term_bytes, DV_ERR_ARG);
   }
-  const Layout lay = Layout::make();
+  const Layout<FOLD> lay = Layout<FOLD>::make();
   const size_t smem = lay.bytes();
-  auto k = decode_bwd_tc_split_kernel;
+  auto k = decode_bwd_tc_split_kernel<FOLD>;
   int dev = 0, sms = 0, smem_max = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -726,6 +833,37 @@ int dv_decode_bwd_tc_split(int kind, int channels, const void* wb, int wb_term_b
   const long long tiles = (n_seg + 127) / 128;
   const long long grid = std::min<long long>(tiles, (long long)sms);
   k<<<(unsigned)grid, THREADS, smem, (cudaStream_t)stream>>>(a);
+  DV_TRY_LAUNCH();
+  return DV_OK;
+}
+
+extern "C" {
+
+int dv_decode_bwd_tc_split(int kind, int channels, const void* wb, int wb_term_bytes, const int* b_layers,
+                           int n_layers, int nvx, int nvy, int nvz, const float* seg, const int* seg_ray,
+                           long long n_seg, const int64_t* n_seg_dev, const float* pe_feat, const float* d4,
+                           const void* saved, long long saved_bytes, const float* out4, float* grad_voxels,
+                           float* grad_params, unsigned char* touched, int* err, void* stream) {
+  return bwd_split<false>(kind, channels, nullptr, wb, wb_term_bytes, b_layers, n_layers, nvx, nvy, nvz, seg, seg_ray,
+                          n_seg, n_seg_dev, pe_feat, d4, saved, saved_bytes, out4, grad_voxels, grad_params, touched, err,
+                          stream);
+}
+
+int dv_decode_bwd_tc_folded(int kind, int channels, const float* params, const void* wb, int wb_term_bytes,
+                            const int* b_layers, int n_layers, int nvx, int nvy, int nvz, const float* seg,
+                            const int* seg_ray, long long n_seg, const int64_t* n_seg_dev, const float* pe_feat,
+                            const float* d4, const void* saved, long long saved_bytes, const float* out4,
+                            float* grad_voxels, float* grad_params, unsigned char* touched, int* err, void* stream) {
+  return bwd_split<true>(kind, channels, params, wb, wb_term_bytes, b_layers, n_layers, nvx, nvy, nvz, seg, seg_ray,
+                         n_seg, n_seg_dev, pe_feat, d4, saved, saved_bytes, out4, grad_voxels, grad_params, touched, err,
+                         stream);
+}
+
+int dv_fold_params(int kind, int channels, const float* params, float* folded, void* stream) {
+  DV_CHECK(kind == 32 && channels == 32, DV_ERR_UNSUPPORTED);
+  DV_CHECK(params && folded, DV_ERR_ARG);
+  const int n = dv_decoder_param_count(kind, channels);
+  bws::fold_params_kernel<<<(n + 255) / 256 + 4, 256, 0, (cudaStream_t)stream>>>(params, n, folded);
   DV_TRY_LAUNCH();
   return DV_OK;
 }

@@ -266,6 +266,19 @@ def tc_bwd_matrices(dec: Decoder):
     return [w0.t().contiguous(), w1.t().contiguous(), m2, w3[:, :W].t().contiguous(), m4]
 
 
+def tc_bwd_folded_matrices(dec: Decoder, wf: torch.Tensor | None = None):
+    """The same for the folded backward: mlp1's output layer and mlp2's first
+    layer as one, (sigma, the 32 outputs of WF = WH W2 [in][out]) from mlp1's
+    last activation.  wf: entries to take in place of that product."""
+    W = dec.width
+    m = tc_bwd_matrices(dec)
+    (w2, _), (w3, _) = dec.layers[dec.n_mlp1 - 1], dec.layers[dec.n_mlp1]
+    f = torch.zeros(W, W + 16)
+    f[:, 0] = w2.detach().float().cpu()[0]
+    f[:, 1:W + 1] = (w3.detach().float().cpu()[:, :W] @ w2.detach().float().cpu()[1:]).t() if wf is None else wf
+    return [m[0], m[1], f, m[4]]
+
+
 def pack_tc_bwd(dec: Decoder, bf16: bool = True):
     """(blob uint8, layers int32 [n, 3] = (byte offset, K, N)) of tc_bwd_matrices."""
     dt = torch.bfloat16 if bf16 else torch.float16
@@ -280,7 +293,8 @@ def tc_index_maps(kind: str, channels: int) -> dict:
     parameter vector rebuilds them on the device, e.g. after an optimizer step,
     without a host round trip.  Keys: 'fwd' (element indices of pack_tc's blob
     as 2-byte elements), 'bias', 'table' (pack_tc's layer rows), and for
-    DIVeR32 over 32 channels 'bwd' / 'bwd_table' (pack_tc_bwd)."""
+    DIVeR32 over 32 channels 'bwd' / 'bwd_table' (pack_tc_bwd) and 'folded' /
+    'folded_table' (tc_bwd_folded_matrices)."""
     n = plain_size(kind, channels)
     ids = torch.arange(1, n + 1, dtype=torch.float32)  # exact in float32 (n < 2^24)
     dec = Decoder(kind, channels, unpack_plain_grad(kind, channels, ids))
@@ -292,4 +306,9 @@ def tc_index_maps(kind: str, channels: int) -> dict:
         bim, btab = _kmajor_images(tc_bwd_matrices(dec), torch.float32)
         out["bwd"] = torch.cat(bim).long()
         out["bwd_table"] = torch.tensor(btab, dtype=torch.int32)
+        # the folded backward's, gathered from dv_fold_params' vector: the parameters, then WF
+        wf = torch.arange(n + 1, n + 1 + dec.width ** 2, dtype=torch.float32).reshape(dec.width, dec.width)
+        fim, ftab = _kmajor_images(tc_bwd_folded_matrices(dec, wf), torch.float32)
+        out["folded"] = torch.cat(fim).long()
+        out["folded_table"] = torch.tensor(ftab, dtype=torch.int32)
     return out

@@ -20,7 +20,7 @@ import torch
 from torch.autograd import Function
 
 from . import _native as N
-from .decoder import Decoder, pack_plain, tc_index_maps
+from .decoder import Decoder, pack_plain, plain_size, tc_index_maps
 from .ray_voxel_intersection import (Segments, dense_segments, masked_segments, masked_segments_begin,
                                      masked_segments_grid)
 
@@ -99,10 +99,16 @@ class TcWeights:
         self.err = torch.zeros(1, dtype=torch.int32, device=device)
         self.bwd = None
         self._i_bwd = None
+        self._folded = None
         if "bwd" in maps and self.bf16:
-            self._i_bwd = maps["bwd"].to(device)
+            # the split form's backward takes mlp1's output layer and mlp2's first
+            # layer as one: its images come from the folded parameter vector
+            name = "folded" if self.terms > 1 else "bwd"
+            self._i_bwd = maps[name].to(device)
             self.bwd = (torch.zeros(self.terms * self._i_bwd.numel() * 2, dtype=torch.uint8, device=device),
-                        maps["bwd_table"].contiguous())
+                        maps[name + "_table"].contiguous())
+            if self.terms > 1:
+                self._folded = torch.zeros(plain_size(kind, channels) + WIDTH[KIND_ID[kind]] ** 2, device=device)
         self.version = None
 
     @staticmethod
@@ -123,6 +129,9 @@ class TcWeights:
         form = 3 if self.terms > 1 else (2 if self.mode == "fp16" else 1)
         self._fill(self.blob, self._i_fwd, p, form)
         self._fill(self.bias, self._i_bias, p, 0)
+        if self._folded is not None:
+            _timed("dv_fold_params", KIND_ID[self.kind], self.channels, N.ptr(p), N.ptr(self._folded), N.stream(p.device))
+            p = self._folded
         if self.bwd is not None:
             self._fill(self.bwd[0], self._i_bwd, p, form)
 
@@ -152,8 +161,8 @@ class TcWeights:
         nx, ny, nz, c = _grid(voxels)
         wb, tb = self.bwd
         if self.terms > 1:
-            _timed("dv_decode_bwd_tc_split", kind, c, N.ptr(wb), wb.numel() // self.terms, tb.data_ptr(),
-                   tb.shape[0], nx, ny, nz, N.ptr(seg.seg), N.ptr(seg.ray), seg.total, seg.count_ptr,
+            _timed("dv_decode_bwd_tc_folded", kind, c, N.ptr(self._folded), N.ptr(wb), wb.numel() // self.terms,
+                   tb.data_ptr(), tb.shape[0], nx, ny, nz, N.ptr(seg.seg), N.ptr(seg.ray), seg.total, seg.count_ptr,
                    N.ptr(pe_feat), N.ptr(d4), N.ptr(saved), saved.numel(), N.ptr(out4), N.ptr(gv), N.ptr(gp),
                    N.ptr(touched), N.ptr(self.err), st)
             return True

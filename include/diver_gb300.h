@@ -437,6 +437,24 @@ DV_API int dv_decode_bwd_tc_split(int kind, int channels, const void* wb, int wb
                                   const void* saved, long long saved_bytes, const float* out4,
                                   float* grad_voxels, float* grad_params, unsigned char* touched, int* err, void* stream);
 
+/*
+ * dv_decode_bwd_tc_split with mlp1's output layer and mlp2's first layer taken
+ * as one matrix (no activation lies between them): a fifth less work, the same
+ * gradients to FP32 rounding.  folded: dv_fold_params of the parameters, the
+ * packed parameters followed by WF [in][out], the product of the two layers.
+ * wb / b_layers: the transposed images of four layers (mlp1's first two;
+ * [sigma | WF | zeros to 48]; mlp2's output), three terms each.  The rest as
+ * there.
+ */
+DV_API int dv_fold_params(int kind, int channels, const float* params, float* folded, void* stream);
+DV_API int dv_decode_bwd_tc_folded(int kind, int channels, const float* folded, const void* wb,
+                                   int wb_term_bytes, const int* b_layers, int n_layers, int nvx, int nvy,
+                                   int nvz, const float* seg, const int* seg_ray, long long n_seg,
+                                   const int64_t* n_seg_dev, const float* pe_feat, const float* d4,
+                                   const void* saved, long long saved_bytes, const float* out4,
+                                   float* grad_voxels, float* grad_params, unsigned char* touched, int* err,
+                                   void* stream);
+
 /* Clearing a grid gradient where a step wrote it (no counterpart in the
  * reference, whose optimizer zeroes the whole dense gradient every step).
  * touched: a byte per grid row (nvz * nvy * nvx, zero-initialised).
