@@ -57,8 +57,11 @@
 // with the chain doing the scatter in its waits and every MMA of a layer ahead
 // of its epilogue, 625 us in this form with one thread issuing and stepping
 // with the chain, 522 us with the issuer's warp running free of it, 513 us with
-// the layer loops rolled (instruction cache), 489 us folded.  What is left is
-// the scatter: the same kernel without its atomics takes 330 us.
+// the layer loops rolled (instruction cache), 490 us folded, 474 us with two
+// staging tiles and the scatter's segments fetched a tile ahead.  What is left
+// is the scatter: folded, without its atomics, the kernel takes 330 us, and the
+// atomics alone 290-310 us at any split of the segments (3.9 M distinct rows,
+// 1.0 GB read and written, at about half the copy rate).
 // Reference semantics: the autograd backward of model/diver.py:159-180.
 #include "common.cuh"
 #include "integrate.cuh"
@@ -97,6 +100,9 @@ constexpr int PE_ONES = 27;         // the PE tile's column of ones (PE_DIM = 27
 template <bool FOLD>
 struct Cfg {
   static constexpr int NL = FOLD ? 4 : 5;
+  // staging tiles, and whether the scatter group fetches the next tile's segments ahead (shared memory allows both folded)
+  static constexpr int NST = FOLD ? 2 : 1;
+  static constexpr bool AHEAD = FOLD;
   static constexpr int PEL = FOLD ? 2 : 3;  // the layer with the PE rows; its bias gradient is column 27 of its PE block
   __host__ __device__ static constexpr int REC(int l) { return FOLD && l == 3 ? 4 : l; }  // its input's tile in the record
   __host__ __device__ static constexpr int IN(int l) { return l == 0 ? C : (l == PEL ? W + PE_DIM : W); }
@@ -118,6 +124,7 @@ struct Cfg {
 
 constexpr uint32_t RECORD = 5 * 2 * TILE;  // saved record of one tile: 5 layer inputs, [128][2 x 32] each
 constexpr uint32_t ONES_BYTES = 128 * 16 * 2;  // a [128][16] BF16 tile of ones
+constexpr int STAGE = 128 * (C + 4);           // floats of a tile's staging rows
 constexpr int COEF = 12;                       // floats per segment: 8 corner weights, lower corner's row, row steps
 
 struct Args {
@@ -145,7 +152,7 @@ struct Args {
 template <bool FOLD>
 struct Layout {
   using P = Cfg<FOLD>;
-  uint32_t bb, rec, pe, d, ones, stage, coef, bar;
+  uint32_t bb, rec, pe, d, ones, stage, coef, seg, bar;
   __host__ __device__ static Layout make() {
     Layout L;
     L.bb = 0;
@@ -154,8 +161,9 @@ struct Layout {
     L.d = L.pe + 2 * TILE;
     L.ones = L.d + 2 * 3 * DTILE;
     L.stage = L.ones + ONES_BYTES;
-    L.coef = L.stage + 128 * (C + 4) * 4;
-    L.bar = L.coef + 128 * COEF * 4;
+    L.coef = L.stage + P::NST * STAGE * 4;
+    L.seg = L.coef + 128 * COEF * 4;
+    L.bar = L.seg + (P::AHEAD ? 128 * 6 * 4 : 0);
     return L;
   }
   // barriers: propagation, NL record slots, the last MMAs; then the TMEM address and the stop flag
@@ -268,7 +276,7 @@ __device__ __forceinline__ void mma_db(uint32_t by, uint32_t tmem, const uint8_t
 // issuer waits); the whole chain with the issuer; the scatter group; the
 // staging rows handed to it (the chain arrives, it waits) and taken by it (the
 // other way round).
-constexpr int BAR_DELTA = 1, BAR_CHAIN = 2, BAR_SCATTER = 3, BAR_STAGED = 4, BAR_TAKEN = 5;
+constexpr int BAR_DELTA = 1, BAR_CHAIN = 2, BAR_SCATTER = 3, BAR_STAGED = 4, BAR_STOP = 6, BAR_TAKEN = 7;  // STAGED and TAKEN: one per staging tile
 
 __device__ __forceinline__ void named_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 __device__ __forceinline__ void named_arrive(int id, int n) {
@@ -286,6 +294,12 @@ __device__ __forceinline__ bool named_and(int id, int n, bool v) {
   return r != 0;
 }
 
+// Asynchronous copy of one float into this thread's own shared memory, and the wait for all of this thread's.
+__device__ __forceinline__ void cp_async4(float* dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(tc::smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // Scatter of a finished tile's feature gradient into the corner rows of its
 // segments: thread i takes channel quad q = i % 8 of the HRUN consecutive
 // segments HRUN * (i / 8)...  Consecutive segments of a ray usually sit in
@@ -297,13 +311,11 @@ __device__ __forceinline__ bool named_and(int id, int n, bool v) {
 constexpr int HRUN = 4;
 static_assert((C / 4) * (128 / HRUN) == SCATTER, "one thread per (channel quad, run)");
 
-// Corner weights and rows of segment s (0 steps where the upper corner is
+// Corner weights and rows of the segment at sg (0 steps where the upper corner is
 // clamped; rows fit 32 bits, 2^32 rows are twice the device's memory), and its
 // row mark for the next step's sparse clear (dv_mark_corner_rows' rule).
-__device__ __forceinline__ void put_coefs(const Args& a, float* coef, long long s) {
-  const float* sg = a.seg + s * 6;
-  const SegCorner sc = segment_corners(__ldg(sg), __ldg(sg + 1), __ldg(sg + 2), __ldg(sg + 3), __ldg(sg + 4),
-                                       __ldg(sg + 5), a.nvx, a.nvy, a.nvz);
+__device__ __forceinline__ void put_coefs(const Args& a, float* coef, const float* sg) {
+  const SegCorner sc = segment_corners(sg[0], sg[1], sg[2], sg[3], sg[4], sg[5], a.nvx, a.nvy, a.nvz);
   const uint32_t row = ((uint32_t)sc.z * a.nvy + sc.y) * a.nvx + sc.x;
   float4* c = reinterpret_cast<float4*>(coef);
   c[0] = make_float4(sc.w[0], sc.w[1], sc.w[2], sc.w[3]);
@@ -319,7 +331,7 @@ __device__ __forceinline__ uint32_t coef_row(const uint4 m, int j) {
 
 // n: segments of this thread's run (0..HRUN); st: its quad in the run's first
 // staging row.
-__device__ __forceinline__ void scatter_run(const Args& a, const float* coef, int n, const float* st, int q) {
+__device__ __forceinline__ void scatter_run(const Args& a, const float* coef, int n, const float* st, int q, int taken) {
   float4 pend[8];  // contributions of the previous segment's corners not yet in memory
   uint4 pm = make_uint4(0u, 0u, 0u, 0u);
   bool pwhole = false;
@@ -366,7 +378,7 @@ __device__ __forceinline__ void scatter_run(const Args& a, const float* coef, in
     pm = m;
     pwhole = whole;
   }
-  named_arrive(BAR_TAKEN, CHAIN + SCATTER);
+  named_arrive(taken, CHAIN + SCATTER);
   if (n > 0) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) red_add4(grid + (long long)coef_row(pm, j) * C, pend[j]);
@@ -420,7 +432,9 @@ __device__ __forceinline__ void prop_row32(uint32_t taddr, float* v) {
 
 // One tile per step of the persistent loop: the layer steps, each the
 // propagation, its gradient MMAs and the epilogue that forms the next delta;
-// the last stages the tile's feature gradient (FP32) for the scatter group.
+// the last stages the tile's feature gradient (FP32) for the scatter group
+// (folded: in one of two staging tiles, so neither group waits for the other's
+// slow tile; and the group's segments come a tile ahead).
 // The saved record sits in five per-layer slots, each with its own mbarrier: a
 // slot is refilled with the next input of that layer once the MMAs that read
 // it are done, so the loads run behind the steps in between.  What the chain
@@ -539,22 +553,35 @@ __global__ void __launch_bounds__(THREADS, 1) decode_bwd_tc_split_kernel(const A
   } else if (warp > CHAIN / 32) {
     // ---- scatter group
     const int i = t - CHAIN_ALL, q = i % (C / 4), ls = (i / (C / 4)) * HRUN;
-    for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    float* ahead = reinterpret_cast<float*>(smem + lay.seg) + 6 * i;  // this thread's own segment of the next tile
+    auto fetch = [&](long long tile) {
+      if (P::AHEAD && i < 128 && tile < tiles && tile * 128 + i < S)
+#pragma unroll
+        for (int j = 0; j < 6; ++j) cp_async4(ahead + j, a.seg + (tile * 128 + i) * 6 + j);
+    };
+    fetch(blockIdx.x);
+    int p = 0;  // the staging tile
+    for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x, p = (p + 1) % P::NST) {
       const long long s0 = tile * 128;
-      if (i < 128 && s0 + i < S) put_coefs(a, coefs + i * COEF, s0 + i);
+      if (P::AHEAD) cp_async_wait();
+      if (i < 128 && s0 + i < S) put_coefs(a, coefs + i * COEF, P::AHEAD ? ahead : a.seg + (s0 + i) * 6);
+      fetch(tile + gridDim.x);
       named_sync(BAR_SCATTER, SCATTER);
-      named_sync(BAR_STAGED, CHAIN + SCATTER);
+      named_sync(BAR_STAGED + p, CHAIN + SCATTER);
       if (*stop) break;
       const long long left = S - (s0 + ls);
-      scatter_run(a, coefs + ls * COEF, left >= HRUN ? HRUN : (left > 0 ? (int)left : 0), stage + ls * (C + 4) + 4 * q, q);
+      scatter_run(a, coefs + ls * COEF, left >= HRUN ? HRUN : (left > 0 ? (int)left : 0),
+                  stage + p * STAGE + ls * (C + 4) + 4 * q, q, BAR_TAKEN + p);
       named_sync(BAR_SCATTER, SCATTER);  // the next tile's corners overwrite these
     }
+    if (P::AHEAD) cp_async_wait();  // none left in flight after a break
   } else {
     // ---- chain
     const uint32_t lane = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t trow = tmem + lane;
     const int r = 32 * (warp & 3) + (t & 31), h = warp > 4 ? 1 : 0;
     uint32_t phase = 0, phase_rec = 0, db = 0;
+    uint32_t done = 0;  // tiles staged
     float v[32];
     // the CTA's first tile: PE tile, first delta
     long long tile = blockIdx.x;
@@ -617,14 +644,14 @@ __global__ void __launch_bounds__(THREADS, 1) decode_bwd_tc_split_kernel(const A
           if (l == PEL - 1 && next < tiles) put2(PE, r, 16 * h, pe, 16);
         } else {
           // the next tile's first delta; then dL/dfeature (FP32) to the staging rows, once the
-          // scatter group has taken the last tile's
+          // scatter group has taken the rows before them
           prop_row16(trow + 16 * h, v);
           if (next < tiles) {
             if (h == 0) write_delta4(Dn, r, gn, on);
             delta_ready();
           }
-          if (!first) named_sync(BAR_TAKEN, CHAIN + SCATTER);
-          float* st = stage + r * (C + 4) + 16 * h;
+          if (done >= P::NST) named_sync(BAR_TAKEN + done % P::NST, CHAIN + SCATTER);
+          float* st = stage + (done % P::NST) * STAGE + r * (C + 4) + 16 * h;
 #pragma unroll
           for (int i = 0; i < 16; i += 4)
             *reinterpret_cast<float4*>(st + i) =
@@ -636,10 +663,12 @@ __global__ void __launch_bounds__(THREADS, 1) decode_bwd_tc_split_kernel(const A
       first = false;
       ok = named_and(BAR_CHAIN, CHAIN_ALL, ok);
       if (!ok && t == 32) *stop = 1;
-      if (!ok) named_sync(BAR_CHAIN + 4, CHAIN);
-      named_arrive(BAR_STAGED, CHAIN + SCATTER);
+      if (!ok) named_sync(BAR_STOP, CHAIN);
+      named_arrive(BAR_STAGED + done % P::NST, CHAIN + SCATTER);
+      ++done;
     }
-    if (!first && ok) named_sync(BAR_TAKEN, CHAIN + SCATTER);  // the last tile's
+    if (ok)  // the last tiles'
+      for (uint32_t u = done > P::NST ? done - P::NST : 0; u < done; ++u) named_sync(BAR_TAKEN + u % P::NST, CHAIN + SCATTER);
     if (!first) {
       tc::fence_before_sync();
       ok = named_and(BAR_CHAIN, CHAIN_ALL, ok);  // the issuer has seen the last MMAs end
