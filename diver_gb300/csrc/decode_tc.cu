@@ -66,7 +66,7 @@ struct TcArgs {
   int* err;    // set to 1 if an MMA completion wait timed out
   int steal;   // one CTA was launched per tile, and running ones take over those not yet started
   uint8_t* save;       // optional: every layer's input tile, per 128-segment tile (training)
-  int save_off[TC_MAX_LAYERS];  // byte offset of layer l's input tile inside a tile's record
+  int save_off[TC_MAX_LAYERS];  // byte offset of layer l's input tile inside a tile's record; negative: not saved
   int save_bytes;      // bytes per tile record (sum of 256 * K over the layers)
 };
 
@@ -541,9 +541,10 @@ __global__ void __launch_bounds__(128, TERMS == 1 ? (W == 32 ? 8 : 4) : ((C == 3
     if constexpr (TS) {                                                                                          \
       ok &= tc_layer_ts<first ? C : W, first>(a.L[l], sB, sA, tmem, ACOL, BF16, bar, phase);                     \
     } else {                                                                                                     \
+      const bool copy = saving && a.save_off[l] >= 0;                                                            \
       ok &= tc_layer<BF16, TERMS>(a.L[l], sB, wterm, sA, TSTRIDE, tmem, bar, phase,                              \
-                                  rec ? rec + a.save_off[l] : nullptr);                                          \
-      if (saving) __syncthreads();                                                                               \
+                                  copy ? rec + a.save_off[l] : nullptr);                                         \
+      if (copy) __syncthreads();                                                                                 \
     }                                                                                                            \
   } while (0)
     // Its output plus `bias`, through ReLU if asked, as the next layer's input.
@@ -798,6 +799,27 @@ static int decode_fwd_tc_args(TcArgs& a, int kind, int channels, int terms, cons
   return DV_OK;
 }
 
+// The split-operand forward; folded: its record leaves out the input of mlp2's
+// first layer, which the folded backward does not read (a fifth of the record:
+// captured 4096-ray step of the 256^3 scene, 322 -> 304 us).
+static int fwd_split(int kind, int channels, const void* wblob, int wbytes, const float* bias, int nbias,
+                     const int* layers, int n_layers, const float* voxels, int nvx, int nvy, int nvz, const float* seg,
+                     const int* seg_ray, long long n_seg, const int64_t* n_seg_dev, const float* pe_out, float* out4,
+                     void* save, long long save_capacity, bool folded, int* err, void* stream) {
+  DV_CHECK(n_seg >= 0, DV_ERR_ARG);
+  if (n_seg == 0) return DV_OK;
+  TcArgs a{};
+  const int rc = decode_fwd_tc_args(a, kind, channels, 3, wblob, wbytes, bias, nbias, layers, n_layers, voxels,
+                                    nullptr, nvx, nvy, nvz, seg, seg_ray, n_seg, n_seg_dev, pe_out, out4, save,
+                                    save_capacity, err);
+  if (rc != DV_OK) return rc;
+  if (folded) a.save_off[n_layers - 2] = -1;
+  cudaStream_t st = (cudaStream_t)stream;
+  if (kind == 32) return launch_decode_fwd_tc<32, 32, 2, 1, 3>(a, st);
+  if (channels == 32) return launch_decode_fwd_tc<32, 64, 1, 1, 3>(a, st);
+  return launch_decode_fwd_tc<64, 64, 1, 1, 3>(a, st);
+}
+
 extern "C" {
 
 int dv_decode_fwd_tc(int kind, int channels, int bf16, const void* wblob, int wbytes, const float* bias, int nbias,
@@ -824,17 +846,17 @@ int dv_decode_fwd_tc_split(int kind, int channels, const void* wblob, int wbytes
                            const float* seg, const int* seg_ray, long long n_seg, const int64_t* n_seg_dev,
                            const float* pe_out, float* out4, void* save, long long save_capacity, int* err,
                            void* stream) {
-  DV_CHECK(n_seg >= 0, DV_ERR_ARG);
-  if (n_seg == 0) return DV_OK;
-  TcArgs a{};
-  const int rc = decode_fwd_tc_args(a, kind, channels, 3, wblob, wbytes, bias, nbias, layers, n_layers, voxels,
-                                    nullptr, nvx, nvy, nvz, seg, seg_ray, n_seg, n_seg_dev, pe_out, out4, save,
-                                    save_capacity, err);
-  if (rc != DV_OK) return rc;
-  cudaStream_t st = (cudaStream_t)stream;
-  if (kind == 32) return launch_decode_fwd_tc<32, 32, 2, 1, 3>(a, st);
-  if (channels == 32) return launch_decode_fwd_tc<32, 64, 1, 1, 3>(a, st);
-  return launch_decode_fwd_tc<64, 64, 1, 1, 3>(a, st);
+  return fwd_split(kind, channels, wblob, wbytes, bias, nbias, layers, n_layers, voxels, nvx, nvy, nvz, seg, seg_ray, n_seg,
+                   n_seg_dev, pe_out, out4, save, save_capacity, false, err, stream);
+}
+
+int dv_decode_fwd_tc_folded(int kind, int channels, const void* wblob, int wbytes, const float* bias, int nbias,
+                            const int* layers, int n_layers, const float* voxels, int nvx, int nvy, int nvz,
+                            const float* seg, const int* seg_ray, long long n_seg, const int64_t* n_seg_dev,
+                            const float* pe_out, float* out4, void* save, long long save_capacity, int* err,
+                            void* stream) {
+  return fwd_split(kind, channels, wblob, wbytes, bias, nbias, layers, n_layers, voxels, nvx, nvy, nvz, seg, seg_ray, n_seg,
+                   n_seg_dev, pe_out, out4, save, save_capacity, true, err, stream);
 }
 
 long long dv_decode_tc_split_save_bytes(int kind, int channels, long long n_seg) {

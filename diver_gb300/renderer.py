@@ -176,8 +176,10 @@ class TcWeights:
     def decode(self, kind, channels, voxels, seg, pe_out, out4, st, voxels16=None, save=None):
         nx, ny, nz, c = _grid(voxels)
         if self.terms > 1:
-            _timed("dv_decode_fwd_tc_split", kind, c, N.ptr(self.blob), self.term_bytes, N.ptr(self.bias),
-                   self.bias.numel(), self.table.data_ptr(), self.table.shape[0], N.ptr(voxels), nx, ny, nz,
+            # a save record (save_buffer gives one where there is a backward to read it) is the folded backward's
+            _timed("dv_decode_fwd_tc_split" if save is None else "dv_decode_fwd_tc_folded", kind, c,
+                   N.ptr(self.blob), self.term_bytes, N.ptr(self.bias), self.bias.numel(),
+                   self.table.data_ptr(), self.table.shape[0], N.ptr(voxels), nx, ny, nz,
                    N.ptr(seg.seg), N.ptr(seg.ray), seg.total, seg.count_ptr, N.ptr(pe_out), N.ptr(out4),
                    N.ptr(save), 0 if save is None else save.numel(), N.ptr(self.err), st)
             return

@@ -362,6 +362,16 @@ DV_API int dv_decode_fwd_tc_split(int kind, int channels, const void* wblob, int
                                   const float* pe_out, float* out4, void* save,
                                   long long save_capacity, int* err, void* stream);
 
+/* dv_decode_fwd_tc_split whose record is for dv_decode_bwd_tc_folded only: the
+ * input tile of mlp2's first layer, which that backward does not read, keeps
+ * its place in the record but is not written. */
+DV_API int dv_decode_fwd_tc_folded(int kind, int channels, const void* wblob, int wbytes,
+                                   const float* bias, int nbias, const int* layers, int n_layers,
+                                   const float* voxels, int nvx, int nvy, int nvz, const float* seg,
+                                   const int* seg_ray, long long n_seg, const int64_t* n_seg_dev,
+                                   const float* pe_out, float* out4, void* save,
+                                   long long save_capacity, int* err, void* stream);
+
 /* Bytes of the `save` buffer of dv_decode_fwd_tc_split for n_seg segments:
  * per tile of 128 segments, every layer input tile as two BF16 terms. */
 DV_API long long dv_decode_tc_split_save_bytes(int kind, int channels, long long n_seg);

@@ -92,6 +92,9 @@ def test_split_backward_tile_edges(n):
     wb = torch.empty(3 * index.numel(), dtype=torch.bfloat16, device="cuda")
     N.call("dv_tc_image", N.ptr(dp), dp.numel(), N.ptr(index), index.numel(), 3, N.ptr(wb), st)
     assert torch.equal(wb[:index.numel()].cpu(), pack_tc_bwd(dec)[0].view(torch.bfloat16).reshape(-1))
+    N.call("dv_decode_fwd_tc_split", 32, 32, N.ptr(tw.blob), tw.term_bytes, N.ptr(tw.bias), tw.bias.numel(),
+           tw.table.data_ptr(), tw.table.shape[0], N.ptr(dv), *grid, N.ptr(pe[1]), N.ptr(out4), N.ptr(save), save.numel(),
+           N.ptr(tw.err), st)  # the record of every layer
     N.call("dv_decode_bwd_tc_split", 32, 32, N.ptr(wb), 2 * index.numel(), table.data_ptr(), table.shape[0], *grid,
            N.ptr(pe[0]), N.ptr(d4), N.ptr(save), save.numel(), N.ptr(out4), *(N.ptr(x) for x in grads[2]), None,
            N.ptr(tw.err), st)
