@@ -63,8 +63,8 @@ DTYPES = {"fp32": "f32", "bf16": "bf16", "fp16": "f16", "bf16s": "bf16x3 (split 
 #           intermediates are not compulsory
 ROW_BYTES = 32 * 4
 FLOP_FWD_SEG = 10176
-FWD_KERNELS = ("dv_decode_fwd", "dv_decode_fwd_tc", "dv_decode_fwd_tc_split", "dv_decode_fwd_tc_folded")
-BWD_KERNELS = ("dv_decode_bwd", "dv_decode_bwd_tc", "dv_decode_bwd_tc_split", "dv_decode_bwd_tc_folded")
+FWD_KERNELS = ("dv_decode_fwd", "dv_decode_fwd_save", "dv_decode_fwd_tc", "dv_decode_fwd_tc_split", "dv_decode_fwd_tc_folded")
+BWD_KERNELS = ("dv_decode_bwd", "dv_decode_bwd_saved", "dv_decode_bwd_tc", "dv_decode_bwd_tc_split", "dv_decode_bwd_tc_folded")
 
 
 def alg_work(kernel, S, U, R):

@@ -321,9 +321,17 @@ int dv_ray_pe(int kind, int channels, const float* params, int batch, const floa
   return DV_OK;
 }
 
-int dv_decode_fwd(int kind, int channels, const float* params, const float* voxels, int nvx, int nvy, int nvz,
-                  const float* seg, const int* seg_ray, long long n_seg, const int64_t* n_seg_dev,
-                  const float* pe_out, float* out4, void* stream) {
+long long dv_decode_save_bytes(int kind, int channels, long long n_seg) {
+  const int floats = kind == 32 && channels == 32 ? REC_FLOATS<32, 32, 2> : kind == 64 && channels == 32
+                     ? REC_FLOATS<32, 64, 1> : kind == 64 && channels == 64 ? REC_FLOATS<64, 64, 1> : 0;
+  if (n_seg < 0 || floats == 0) return -1;
+  return (n_seg + REC_SEGS - 1) / REC_SEGS * floats * (long long)sizeof(float);
+}
+
+int dv_decode_fwd_save(int kind, int channels, const float* params, const float* voxels, int nvx, int nvy, int nvz,
+                       const float* seg, const int* seg_ray, long long n_seg, const int64_t* n_seg_dev,
+                       const float* pe_out, float* out4, void* save, long long save_bytes,
+                       void* stream) {
   DecodeArgs a{};
   DV_CHECK(fill_layers(a, kind, channels) == DV_OK && n_seg >= 0, DV_ERR_ARG);
   if (n_seg == 0) return DV_OK;
@@ -340,12 +348,24 @@ int dv_decode_fwd(int kind, int channels, const float* params, const float* voxe
   a.params = params;
   a.pe_out = const_cast<float*>(pe_out);
   a.out4 = reinterpret_cast<float4*>(out4);
+  if (save) {
+    const long long need = dv_decode_save_bytes(kind, channels, n_seg);
+    DV_CHECK(((uintptr_t)save & 15) == 0 && need > 0 && need <= save_bytes, DV_ERR_ARG);
+    a.acts = static_cast<float*>(save);
+  }
   cudaStream_t st = (cudaStream_t)stream;
   const int sms = sm_count();
   if (kind == 32 && channels == 32) return decode_fwd_v32c32(a, st, sms);
   if (kind == 64 && channels == 32) return decode_fwd_v64c32(a, st, sms);
   if (kind == 64 && channels == 64) return decode_fwd_v64c64(a, st, sms);
   return DV_ERR_UNSUPPORTED;
+}
+
+int dv_decode_fwd(int kind, int channels, const float* params, const float* voxels, int nvx, int nvy, int nvz,
+                  const float* seg, const int* seg_ray, long long n_seg, const int64_t* n_seg_dev,
+                  const float* pe_out, float* out4, void* stream) {
+  return dv_decode_fwd_save(kind, channels, params, voxels, nvx, nvy, nvz, seg, seg_ray, n_seg, n_seg_dev, pe_out, out4,
+                            nullptr, 0, stream);
 }
 
 int dv_composite_fwd(int batch, const int64_t* offsets, const float* out4, int white_back, float* rgb, float* t_final,
@@ -403,10 +423,10 @@ int dv_composite_bwd(int batch, const int64_t* offsets, const float* out4, const
   return DV_OK;
 }
 
-int dv_decode_bwd(int kind, int channels, const float* params, const float* voxels, int nvx, int nvy, int nvz,
-                  const float* seg, const int* seg_ray, long long n_seg, const int64_t* n_seg_dev,
-                  const float* pe_feat, const float* pe_out, const float* d4, float* grad_voxels, float* grad_params,
-                  void* stream) {
+int dv_decode_bwd_saved(int kind, int channels, const float* params, const float* voxels, int nvx, int nvy, int nvz,
+                        const float* seg, const int* seg_ray, long long n_seg, const int64_t* n_seg_dev,
+                        const float* pe_feat, const float* pe_out, const float* d4, float* grad_voxels, float* grad_params,
+                        const void* saved, long long saved_bytes, void* stream) {
   DecodeArgs a{};
   DV_CHECK(fill_layers(a, kind, channels) == DV_OK && n_seg >= 0, DV_ERR_ARG);
   if (n_seg == 0) return DV_OK;
@@ -427,12 +447,25 @@ int dv_decode_bwd(int kind, int channels, const float* params, const float* voxe
   a.d4 = reinterpret_cast<const float4*>(d4);
   a.grad_grid = grad_voxels;
   a.grad_params = grad_params;
+  if (saved) {
+    const long long need = dv_decode_save_bytes(kind, channels, n_seg);
+    DV_CHECK(((uintptr_t)saved & 15) == 0 && need > 0 && need <= saved_bytes, DV_ERR_ARG);
+    a.acts = const_cast<float*>(static_cast<const float*>(saved));
+  }
   cudaStream_t st = (cudaStream_t)stream;
   const int sms = sm_count();
   if (kind == 32 && channels == 32) return decode_bwd_v32c32(a, st, sms);
   if (kind == 64 && channels == 32) return decode_bwd_v64c32(a, st, sms);
   if (kind == 64 && channels == 64) return decode_bwd_v64c64(a, st, sms);
   return DV_ERR_UNSUPPORTED;
+}
+
+int dv_decode_bwd(int kind, int channels, const float* params, const float* voxels, int nvx, int nvy, int nvz,
+                  const float* seg, const int* seg_ray, long long n_seg, const int64_t* n_seg_dev,
+                  const float* pe_feat, const float* pe_out, const float* d4, float* grad_voxels, float* grad_params,
+                  void* stream) {
+  return dv_decode_bwd_saved(kind, channels, params, voxels, nvx, nvy, nvz, seg, seg_ray, n_seg, n_seg_dev, pe_feat, pe_out,
+                             d4, grad_voxels, grad_params, nullptr, 0, stream);
 }
 
 int dv_reg_mean(int batch, const float* reg, const int* max_dev, float max_host, float* mean, float* inv_max,

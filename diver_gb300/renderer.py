@@ -68,6 +68,22 @@ def _check_params(kind: int, channels: int, params: torch.Tensor):
 FORMS = ("fp32", "bf16", "fp16", "bf16s")
 
 
+# Bytes up to which the plain FP32 form keeps its activations for the backward
+# (576 B a segment of DIVeR32, 864 of DIVeR64 over 64 channels).  Larger lists recompute them, and their
+# memory stays at the 60 B a segment of the lists and outputs.
+PLAIN_SAVE = 2 << 30
+
+
+def _plain_save(kind: int, channels: int, n_seg: int, device) -> torch.Tensor | None:
+    n = int(N.lib().dv_decode_save_bytes(kind, channels, n_seg))
+    if not 0 < n <= PLAIN_SAVE:
+        return None
+    try:
+        return torch.empty(n, dtype=torch.uint8, device=device)
+    except torch.cuda.OutOfMemoryError:  # the recomputing backward needs no record
+        return None
+
+
 # Rays up to which their directions' encoding runs on the calling stream (8 us
 # at this many, against about 25 us of host time for a side stream).
 PE_INLINE = 16384
@@ -209,8 +225,14 @@ class SegmentRender(Function):
         S = seg.total
         out4 = torch.empty(S, 4, device=dev)
         if tc is None:
-            _timed("dv_decode_fwd", kind, c, N.ptr(params), N.ptr(voxels), nx, ny, nz, N.ptr(seg.seg), N.ptr(seg.ray),
-                   S, seg.count_ptr, N.ptr(pe_out), N.ptr(out4), st)
+            save = _plain_save(kind, c, S, dev) if training else None
+            args = (kind, c, N.ptr(params), N.ptr(voxels), nx, ny, nz, N.ptr(seg.seg), N.ptr(seg.ray), S, seg.count_ptr,
+                    N.ptr(pe_out), N.ptr(out4))
+            if save is None:
+                _timed("dv_decode_fwd", *args, st)
+            else:
+                _timed("dv_decode_fwd_save", *args, N.ptr(save), save.numel(), st)
+            ctx.saved_layers = save
         else:
             # training: keep the layer inputs for the tensor-core backward
             save = tc.save_buffer(kind, c, S, dev) if training else None
@@ -266,8 +288,12 @@ class SegmentRender(Function):
         if ctx.tc is not None and ctx.tc.backward(ctx.kind, voxels, seg, pe_feat, pe_out, d4, gv, gp, st, saved, out4,
                                                   touched):
             return gv, gp, None, None, None, None, None, None, None, None, None
-        _timed("dv_decode_bwd", ctx.kind, c, N.ptr(params), N.ptr(voxels), nx, ny, nz, N.ptr(seg.seg), N.ptr(seg.ray),
-               seg.total, seg.count_ptr, N.ptr(pe_feat), N.ptr(pe_out), N.ptr(d4), N.ptr(gv), N.ptr(gp), st)
+        args = (ctx.kind, c, N.ptr(params), N.ptr(voxels), nx, ny, nz, N.ptr(seg.seg), N.ptr(seg.ray), seg.total,
+                seg.count_ptr, N.ptr(pe_feat), N.ptr(pe_out), N.ptr(d4), N.ptr(gv), N.ptr(gp))
+        if ctx.tc is None and saved is not None:
+            _timed("dv_decode_bwd_saved", *args, N.ptr(saved), saved.numel(), st)
+        else:
+            _timed("dv_decode_bwd", *args, st)
         return gv, gp, None, None, None, None, None, None, None, None, None
 
 

@@ -305,6 +305,25 @@ DV_API int dv_decode_bwd(int kind, int channels, const float* params, const floa
                          const float* d4, float* grad_voxels, float* grad_params, void* stream);
 
 /*
+ * The pair for a training step: the forward also writes its features and
+ * activations to `save` (FP32, dv_decode_save_bytes, 16-byte aligned), and the
+ * backward reads them (`saved`, the forward's buffer for the same segments,
+ * grid and parameters) where dv_decode_bwd gathers and recomputes them: the
+ * same values, so the same gradients.  save / saved null: as dv_decode_fwd /
+ * dv_decode_bwd.
+ */
+DV_API long long dv_decode_save_bytes(int kind, int channels, long long n_seg);
+DV_API int dv_decode_fwd_save(int kind, int channels, const float* params, const float* voxels, int nvx,
+                              int nvy, int nvz, const float* seg, const int* seg_ray, long long n_seg,
+                              const int64_t* n_seg_dev, const float* pe_out, float* out4, void* save,
+                              long long save_bytes, void* stream);
+DV_API int dv_decode_bwd_saved(int kind, int channels, const float* params, const float* voxels, int nvx,
+                               int nvy, int nvz, const float* seg, const int* seg_ray, long long n_seg,
+                               const int64_t* n_seg_dev, const float* pe_feat, const float* pe_out,
+                               const float* d4, float* grad_voxels, float* grad_params, const void* saved,
+                               long long saved_bytes, void* stream);
+
+/*
  * Tensor-core form of dv_decode_fwd: the same decoder with its matrix
  * products on tcgen05 (BF16 when bf16 = 1, FP16 when 0, FP32 accumulation in
  * TMEM).  The integral, biases, PE term (pe_out, FP32), ReLU and sigmoid stay

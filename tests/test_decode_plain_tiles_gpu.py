@@ -62,3 +62,42 @@ def test_plain_decoder_tile_edges(kind, channels, n):
     for (gw, gb), (w, b) in zip(unpack_plain_grad(kind, channels, gp.cpu().double()), layers):
         assert (gw - w.grad).norm() <= 1e-4 * w.grad.norm()
         assert (gb - b.grad).norm() <= 1e-4 * b.grad.norm()
+
+
+@pytest.mark.parametrize("kind,channels", [("diver32", 32), ("diver64", 32), ("diver64", 64)])
+@pytest.mark.parametrize("n", [1, 16, 17, 31, 32, 33, 1000, 40001])
+@pytest.mark.parametrize("held", [False, True])
+def test_plain_record_is_the_recompute(kind, channels, n, held):
+    """The forward's record gives the recomputing backward's gradients: the
+    same values in, so they differ by the order of their atomic sums only (1e-6
+    relative L2).  held: the count on the device, in lists with room to spare."""
+    from diver_gb300 import _native as N
+    from diver_gb300.decoder import pack_plain
+
+    base = min(n, 1000)
+    vox, seg, ray, dirs, dec, _ = case(base, channels, kind, 5 * base)
+    k, W = int(kind[5:]), dec.width
+    rep, room, B = -(-n // base), 100 if held else 0, dirs.shape[0]
+    ray = torch.cat([ray + i * B for i in range(rep)])[:n]
+    seg, dirs = seg.repeat(rep, 1)[:n], dirs.repeat(rep, 1)
+    seg, ray = torch.cat([seg, seg[:1].expand(room, 6)]), torch.cat([ray, ray[:1].expand(room)])
+    d4 = torch.randn(n + room, 4, generator=torch.Generator().manual_seed(n))
+    dv, ds, dr, dd, dp, dg = (x.cuda().contiguous() for x in (vox, seg, ray, dirs, pack_plain(dec), d4))
+    count = torch.tensor([n], device="cuda") if held else None
+    st, S = N.stream(dv.device), n + room
+    pe_feat, pe_out = torch.empty(len(dirs), 28, device="cuda"), torch.empty(len(dirs), W, device="cuda")
+    N.call("dv_ray_pe", k, channels, N.ptr(dp), len(dirs), N.ptr(dd), N.ptr(pe_feat), N.ptr(pe_out), st)
+    head = (k, channels, N.ptr(dp), N.ptr(dv), 10, 8, 6, N.ptr(ds), N.ptr(dr), S, N.ptr(count))
+    save = torch.empty(N.lib().dv_decode_save_bytes(k, channels, S), dtype=torch.uint8, device="cuda")
+    out, out2 = torch.zeros(S, 4, device="cuda"), torch.zeros(S, 4, device="cuda")
+    N.call("dv_decode_fwd", *head, N.ptr(pe_out), N.ptr(out), st)
+    N.call("dv_decode_fwd_save", *head, N.ptr(pe_out), N.ptr(out2), N.ptr(save), save.numel(), st)
+    assert torch.equal(out, out2)
+    grads = [(torch.zeros_like(dv), torch.zeros_like(dp)) for _ in range(2)]
+    tail = (N.ptr(pe_feat), N.ptr(pe_out), N.ptr(dg))
+    N.call("dv_decode_bwd", *head, *tail, *(N.ptr(x) for x in grads[0]), st)
+    N.call("dv_decode_bwd_saved", *head, *tail, *(N.ptr(x) for x in grads[1]), N.ptr(save), save.numel(), st)
+    for a, b in zip(*grads):
+        assert (a - b).norm() <= 1e-6 * b.norm()
+    with pytest.raises(RuntimeError):
+        N.call("dv_decode_fwd_save", *head, N.ptr(pe_out), N.ptr(out2), N.ptr(save), save.numel() - 1, st)
