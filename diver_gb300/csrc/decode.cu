@@ -322,8 +322,10 @@ int dv_ray_pe(int kind, int channels, const float* params, int batch, const floa
 }
 
 long long dv_decode_save_bytes(int kind, int channels, long long n_seg) {
-  const int floats = kind == 32 && channels == 32 ? REC_FLOATS<32, 32, 2> : kind == 64 && channels == 32
-                     ? REC_FLOATS<32, 64, 1> : kind == 64 && channels == 64 ? REC_FLOATS<64, 64, 1> : 0;
+  int floats = 0;
+  if (kind == 32 && channels == 32) floats = REC_FLOATS<32, 32, 2>;
+  if (kind == 64 && channels == 32) floats = REC_FLOATS<32, 64, 1>;
+  if (kind == 64 && channels == 64) floats = REC_FLOATS<64, 64, 1>;
   if (n_seg < 0 || floats == 0) return -1;
   return (n_seg + REC_SEGS - 1) / REC_SEGS * floats * (long long)sizeof(float);
 }

@@ -1,4 +1,5 @@
-"""GPU: the plain FP32 decoder, forward and backward, at the edges of its
+"""GPU: the per-ray encoding at the edges of its blocks' turns, and the plain
+FP32 decoder, forward and backward, at the edges of its
 16- and 32-segment warp tiles and of the backward's 128-segment steps, with
 rays that end inside tiles and segments on the grid's far faces, against the
 FP64 oracle.  Tolerances: forward 1e-5 abs, gradients 1e-4 relative L2, the
@@ -101,3 +102,26 @@ def test_plain_record_is_the_recompute(kind, channels, n, held):
         assert (a - b).norm() <= 1e-6 * b.norm()
     with pytest.raises(RuntimeError):
         N.call("dv_decode_fwd_save", *head, N.ptr(pe_out), N.ptr(out2), N.ptr(save), save.numel() - 1, st)
+
+
+@pytest.mark.parametrize("kind", ["diver32", "diver64"])
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 31, 32, 33, 304 * 16 + 1, 304 * 32 + 1, 30001])
+def test_ray_pe_edges(kind, n):
+    """Encoding and its mlp2 term against 64 bits: an angle of up to 8 pi is
+    off by 2^-24 of itself twice (FP32 pi, the product), 3e-6, and the term by
+    that over its 27 inputs (3e-5 for weights of up to 0.3)."""
+    from diver_gb300 import _native as N
+    from diver_gb300.decoder import pack_plain, random_decoder
+
+    dec = random_decoder(kind, 32, n)
+    d = torch.randn(n, 3, generator=torch.Generator().manual_seed(n))
+    d = d / d.norm(dim=-1, keepdim=True)
+    dd, dp = d.cuda().contiguous(), pack_plain(dec).cuda()
+    feat, out = torch.full((n + 1, 28), -7.0, device="cuda"), torch.full((n + 1, dec.width), -7.0, device="cuda")
+    N.call("dv_ray_pe", int(kind[5:]), 32, N.ptr(dp), n, N.ptr(dd), N.ptr(feat), N.ptr(out), N.stream(dd.device))
+    pe = torch_ref.pos_enc(d.double())
+    w, b = dec.layers[dec.n_mlp1]
+    ref = pe @ w.double()[:, dec.width:].t() + b.double()
+    assert (feat[:n, :27].cpu().double() - pe).abs().max() <= 5e-6
+    assert (out[:n].cpu().double() - ref).abs().max() <= 3e-5
+    assert bool((feat[n:] == -7.0).all()) and bool((out[n:] == -7.0).all())

@@ -70,3 +70,20 @@ def test_masked_walk_per_axis_extents():
                               torch.from_numpy(mask).cuda())
     assert np.array_equal(sg.counts.cpu().numpy(), num)
     assert same_bits(sg.seg.cpu().numpy(), orc.csr_from_padded(oi, num))
+
+
+@pytest.mark.parametrize("extra", [-1, 0, 33])
+def test_masked_count_of_large_batches(extra):
+    """Around 768 rays per SM, where a count goes from the ring to a thread per ray."""
+    from diver_gb300 import masked_segments
+
+    batch = 768 * torch.cuda.get_device_properties(0).multi_processor_count + extra
+    o, v = rays(batch, 11, True)
+    n, x0 = 12, -1.5
+    mask = np.random.default_rng(2).random((n, n, n)) < 0.5
+    wi, num, wt = orc.masked_walk(o, v, x0, n, 3.0 / n, mask, 1.0)
+    sg = masked_segments(torch.from_numpy(o).cuda(), torch.from_numpy(v).cuda(), x0, n, 3.0 / n,
+                         torch.from_numpy(mask).cuda(), 1.0)
+    assert np.array_equal(sg.counts.cpu().numpy(), num)
+    assert same_bits(sg.seg.cpu().numpy(), orc.csr_from_padded(wi, num))
+    assert same_bits(sg.t.cpu().numpy(), orc.csr_from_padded(wt, num))
