@@ -286,15 +286,15 @@ def pack_tc_bwd(dec: Decoder, bf16: bool = True):
     return torch.cat([i.view(torch.uint8) for i in images]), torch.tensor(table, dtype=torch.int32)
 
 
-def tc_index_maps(kind: str, channels: int) -> dict:
+def tc_index_maps(kind: str, channels: int, backward: tuple = ("bwd", "folded")) -> dict:
     """Where every element of the tensor-core images comes from in the packed
     plain parameter vector: index + 1, or 0 for padding.  The images are pure
     rearrangements of the parameters, so a gather of the (zero-prefixed)
     parameter vector rebuilds them on the device, e.g. after an optimizer step,
     without a host round trip.  Keys: 'fwd' (element indices of pack_tc's blob
     as 2-byte elements), 'bias', 'table' (pack_tc's layer rows), and for
-    DIVeR32 over 32 channels 'bwd' / 'bwd_table' (pack_tc_bwd) and 'folded' /
-    'folded_table' (tc_bwd_folded_matrices)."""
+    DIVeR32 over 32 channels those of `backward`: 'bwd' / 'bwd_table'
+    (pack_tc_bwd), 'folded' / 'folded_table' (tc_bwd_folded_matrices)."""
     n = plain_size(kind, channels)
     ids = torch.arange(1, n + 1, dtype=torch.float32)  # exact in float32 (n < 2^24)
     dec = Decoder(kind, channels, unpack_plain_grad(kind, channels, ids))
@@ -303,12 +303,13 @@ def tc_index_maps(kind: str, channels: int) -> dict:
     _, _, table = pack_tc(dec, True)
     out = {"fwd": torch.cat(images).long(), "bias": torch.cat([b for _, b in mats]).long(), "table": table}
     if kind == "diver32" and channels == 32:
-        bim, btab = _kmajor_images(tc_bwd_matrices(dec), torch.float32)
-        out["bwd"] = torch.cat(bim).long()
-        out["bwd_table"] = torch.tensor(btab, dtype=torch.int32)
-        # the folded backward's, gathered from dv_fold_params' vector: the parameters, then WF
-        wf = torch.arange(n + 1, n + 1 + dec.width ** 2, dtype=torch.float32).reshape(dec.width, dec.width)
-        fim, ftab = _kmajor_images(tc_bwd_folded_matrices(dec, wf), torch.float32)
-        out["folded"] = torch.cat(fim).long()
-        out["folded_table"] = torch.tensor(ftab, dtype=torch.int32)
+        for name in backward:
+            if name == "folded":  # gathered from dv_fold_params' vector: the parameters, then WF
+                wf = torch.arange(n + 1, n + 1 + dec.width ** 2, dtype=torch.float32).reshape(dec.width, dec.width)
+                mats = tc_bwd_folded_matrices(dec, wf)
+            else:
+                mats = tc_bwd_matrices(dec)
+            images, btab = _kmajor_images(mats, torch.float32)
+            out[name] = torch.cat(images).long()
+            out[name + "_table"] = torch.tensor(btab, dtype=torch.int32)
     return out

@@ -101,7 +101,10 @@ class TcWeights:
         mode = mode or ("bf16" if bf16 else "fp16")
         if mode not in ("bf16", "fp16", "bf16s"):
             raise ValueError(f"unknown tensor-core form {mode!r}")
-        maps = tc_index_maps(kind, channels)
+        # the split form's backward takes mlp1's output layer and mlp2's first
+        # layer as one: its images come from the folded parameter vector
+        name = {"bf16": "bwd", "bf16s": "folded", "fp16": None}[mode]
+        maps = tc_index_maps(kind, channels, (name,) if name else ())
         self.kind, self.channels, self.mode = kind, channels, mode
         self.bf16 = mode != "fp16"
         self.terms = 3 if mode == "bf16s" else 1
@@ -116,10 +119,7 @@ class TcWeights:
         self.bwd = None
         self._i_bwd = None
         self._folded = None
-        if "bwd" in maps and self.bf16:
-            # the split form's backward takes mlp1's output layer and mlp2's first
-            # layer as one: its images come from the folded parameter vector
-            name = "folded" if self.terms > 1 else "bwd"
+        if name in maps:
             self._i_bwd = maps[name].to(device)
             self.bwd = (torch.zeros(self.terms * self._i_bwd.numel() * 2, dtype=torch.uint8, device=device),
                         maps[name + "_table"].contiguous())
