@@ -83,6 +83,19 @@ __device__ __forceinline__ float4 integrate4(const float* __restrict__ grid, con
   return acc;
 }
 
+// Asks L2 for the 8 corner rows (BYTES each) of a segment: lower corner's row,
+// row steps to the upper corners.
+template <int BYTES>
+__device__ __forceinline__ void prefetch_rows(const void* grid, uint32_t row, uint32_t dx, uint32_t dy, uint32_t dz) {
+  const uint8_t* p = static_cast<const uint8_t*>(grid) + (unsigned long long)row * BYTES;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const unsigned long long rows = (unsigned long long)((j & 1) ? dx : 0u) + ((j & 2) ? dy : 0u) + ((j & 4) ? dz : 0u);
+#pragma unroll
+    for (int b = 0; b < BYTES; b += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + rows * BYTES + b));
+  }
+}
+
 // Vector atomic add of 4 floats (sm_90+ global float4 atomics).
 __device__ __forceinline__ void red_add4(float* dst, float4 v) {
   atomicAdd(reinterpret_cast<float4*>(dst), v);
