@@ -28,7 +28,7 @@
 // shared memory): a 2035-ray DIVeR32 training step on a 160^3 grid, backward
 // 1068 -> 362 us, forward 196 -> 115 us; a 1024-ray DIVeR64 step over 64
 // channels on a 192^3 grid, backward 2853 -> 600 us.  Packed FMAs since: 338
-// and 107 us; with the forward's record (REC_SEGS) 247 and 124.
+// and 107 us; with the forward's record (REC_SEGS) 237 and 124.
 #pragma once
 #include "common.cuh"
 #include "integrate.cuh"
@@ -353,7 +353,7 @@ __device__ __forceinline__ float3 colour(const float* w3, const float* b3, const
 // the features and every relu activation as they lie in a warp's shared memory,
 // rows of REC_LD.  The backward reads it in place of gathering and recomputing
 // (a third of its FMAs, and the gather's latency).  Measured, a 2035-ray DIVeR32
-// step on a 160^3 grid: backward 338 -> 247 us, forward 107 -> 124 us.
+// step on a 160^3 grid: backward 338 -> 237 us, forward 107 -> 124 us.
 constexpr int REC_SEGS = 32, REC_LD = REC_SEGS + 4;
 template <int C, int W, int D1>
 constexpr int REC_FLOATS = (C + (D1 + 1) * W) * REC_LD;
@@ -729,6 +729,13 @@ __global__ void __launch_bounds__(32 * WARPS, 1) decode_bwd_plain(const DecodeAr
     if constexpr (SAVED) {
       static_assert(L::A1 == C * LD && L::DS == (C + (D1 + 1) * W) * LD && REC_SEGS % SEGS == 0, "the record's rows");
       load_record<C + (D1 + 1) * W, SEGS>(mine, a.acts, s0, S);
+      // the next step's record on its way to L2 (DIVeR32: 247 -> 237 us)
+      const long long sn = s0 + step * span;
+      if (sn < S) {
+        const float* rec = a.acts + sn / REC_SEGS * REC_FLOATS<C, W, D1>;
+        for (int i = 32 * lane; i < REC_FLOATS<C, W, D1>; i += 32 * 32)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(rec + i));
+      }
     } else {
       gather_warp<C, SEGS>(a, S, s0, coef, X0);
       __syncwarp();
