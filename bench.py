@@ -85,12 +85,13 @@ def alg_work(kernel, S, U, R):
 # is this times the segments of a launch.  The split backward has no entry:
 # its current form has no ncu section capture (the roofline reports null).
 TRAFFIC_PER_SEG = {"dv_decode_bwd_tc": 1302.35, "dv_decode_fwd_tc": 810.52, "dv_decode_fwd_tc_split": 997.2}
-# Kernels of this library per captured training step: row clear, three weight
-# image gathers, ray PE, slot walk, 3 scan kernels, slot compaction, decoder
+# Kernels of this library per captured training step: row clear, weight image
+# gathers (forward, biases, backward; the split form's after the folded
+# product), ray PE, slot walk, 3 scan kernels, slot compaction, decoder
 # forward, compositing forward, sparsity mean, loss, loss gradients,
-# compositing backward, decoder backward (which also marks the rows the next
-# step's clear zeroes).
-OUR_LAUNCHES_PER_STEP = 17
+# compositing backward, row marks (the split backward sets them itself),
+# decoder backward.
+OUR_LAUNCHES_PER_STEP = {"fp32": 15, "fp16": 17, "bf16": 18, "bf16s": 18}
 
 
 def parse():
@@ -478,7 +479,7 @@ def run_ours(args, rank, world, local):
                 "captured once in a CUDA graph and replayed (diver_gb300.graphs)",
         "timed_region": regions,
         "e2e": e2e[tform],
-        "gpu_launches": OUR_LAUNCHES_PER_STEP * args.steps,
+        "gpu_launches": OUR_LAUNCHES_PER_STEP[tform] * args.steps,
         "roofline": roofline,
         "train_forms": train_forms,
         "configs": extra,

@@ -271,8 +271,8 @@ __device__ __forceinline__ void gather_tile_split(const TcArgs& a, long long S, 
 // bulk async copy and, before the caller's barrier lets anyone overwrite A,
 // waits until that copy has read it.
 template <int BF16, int TERMS>
-__device__ __forceinline__ bool tc_layer(const TcLayer& L, const uint8_t* sB, uint32_t wterm, const uint8_t* sA,
-                                         uint32_t tstride, uint32_t tmem, uint64_t* bar, uint32_t& phase,
+__device__ __forceinline__ bool tc_layer(const TcLayer& L, const uint8_t* sB, const uint8_t* sA, uint32_t tstride,
+                                         uint32_t tmem, uint64_t* bar, uint32_t& phase,
                                          uint8_t* save = nullptr) {
   if (threadIdx.x == 0) {
     tc::fence_after_sync();
@@ -507,7 +507,6 @@ __global__ void __launch_bounds__(128, TERMS == 1 ? (W == 32 ? 8 : 4) : ((C == 3
   tc::fence_after_sync();
   const uint32_t tmem = *tslot;
   const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);  // this warp's TMEM lanes
-  const uint32_t wterm = (uint32_t)a.wbytes;
   uint32_t phase = 0;
   bool ok = true;
   const bool saving = a.save != nullptr;
@@ -542,7 +541,7 @@ __global__ void __launch_bounds__(128, TERMS == 1 ? (W == 32 ? 8 : 4) : ((C == 3
       ok &= tc_layer_ts<first ? C : W, first>(a.L[l], sB, sA, tmem, ACOL, BF16, bar, phase);                     \
     } else {                                                                                                     \
       const bool copy = saving && a.save_off[l] >= 0;                                                            \
-      ok &= tc_layer<BF16, TERMS>(a.L[l], sB, wterm, sA, TSTRIDE, tmem, bar, phase,                              \
+      ok &= tc_layer<BF16, TERMS>(a.L[l], sB, sA, TSTRIDE, tmem, bar, phase,                                     \
                                   copy ? rec + a.save_off[l] : nullptr);                                         \
       if (copy) __syncthreads();                                                                                 \
     }                                                                                                            \

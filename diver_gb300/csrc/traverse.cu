@@ -2,9 +2,10 @@
 // the octree first-hit search and the 8-hit ray march (real-time path), and
 // the prefix sum that turns per-ray counts into CSR segment offsets.
 //
-// One thread walks one ray; the walk itself is inherently sequential (each
-// crossing is computed from the previous, rounded point), so bit-exactness
-// with the reference fixes the per-ray order of operations.  What changes
+// One thread steps one ray (the masked walk's occupancy and output are other
+// warps' work); the walk itself is inherently sequential (each crossing is
+// computed from the previous, rounded point), so bit-exactness with the
+// reference fixes the per-ray order of operations.  What changes
 // against the reference is around the walk: outputs are either counted only,
 // written to caller-sized padded rows, or written compacted (CSR) so that the
 // segment-parallel decoder never touches padding; max(count) is reduced per
