@@ -309,11 +309,15 @@ int dv_clear_marked_rows(float* grid, int channels, int nvx, int nvy, int nvz, u
   DV_CHECK(grid && touched && ((uintptr_t)grid & 15) == 0, DV_ERR_ARG);
   DV_CHECK((long long)nvy * nvz < (1ll << 31), DV_ERR_ARG);
   const long long rows = (long long)nvx * nvy * nvz;
-  // 4 blocks per SM: the clear runs beside the step's traversal on another
-  // stream.  The traversal's blocks still fit beside them, and the clear is
-  // over before the decode, whose persistent blocks want the whole SM (a block
-  // that starts late has its full share of tiles left).  Captured 4096-ray
-  // step at 1 / 2 / 4 / 8 blocks: 1443 / 1360 / 1330 / 1326 us.
+  // 4 blocks per SM: the clear runs on a stream of its own and is over before
+  // the decode, whose persistent blocks want the whole SM (a block that starts
+  // late has its full share of tiles left).  Captured 4096-ray step at 1 / 2 /
+  // 4 / 8 blocks: 1443 / 1360 / 1330 / 1326 us.  The traversal's blocks, which
+  // need shared memory, mostly wait for it: an SM changes its split between
+  // shared memory and L1 only when it is empty.  Asking for the traversal's
+  // split here, with 2 blocks, lets both run (step of 4096 rays through a 256^3
+  // grid 927 -> 906 us), but the clear's writes then slow a larger batch's walk
+  // by more than that (8192 rays of a 320 x 320 x 160 grid 960 -> 982 us).
   const unsigned need = ceil_div((long long)nvy * nvz, 8);  // 8 warps (lines) per block
   const unsigned blocks = need < 152u * 4u ? need : 152u * 4u;
   float4* g = reinterpret_cast<float4*>(grid);
