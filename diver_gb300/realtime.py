@@ -161,6 +161,8 @@ class RealtimeModel:
         # (a round over an empty list changes nothing; the frame is the same, the
         # round count at most one higher)
         n = self.voxel_num
+        if v.shape[-1] != 3 or v.numel() != 3 * B:  # the kernels read (x, y, z) at v + 3 b
+            raise ValueError(f"dirs must hold one (x, y, z) per ray, [B, 3], got {tuple(v.shape)}")
         N.need_cuda("dirs", v, torch.float32)
         N.need_cuda("center", center, torch.float32)
         m8, o8 = _u8("mask", self.voxel_masks), _u8("octrees", self.octrees)
