@@ -128,10 +128,13 @@ def ptr(t: torch.Tensor | None) -> int | None:
 
 def stream(device: torch.device | str | int | None = None) -> int:
     """The current stream's handle (a stream object per launch costs more than
-    the launch)."""
+    the launch); ValueError for another device than a CUDA one."""
     index = device
     if index is not None and not isinstance(index, int):  # a torch.device, or its name
-        index = (index if isinstance(index, torch.device) else torch.device(index)).index
+        d = index if isinstance(index, torch.device) else torch.device(index)
+        if d.type != "cuda":
+            raise ValueError(f"expected a cuda device, got {d}")
+        index = d.index
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
