@@ -36,7 +36,7 @@ def _check_rays(o: torch.Tensor, v: torch.Tensor) -> int:
 def mask_side(voxel_num: float, mask_scale: float) -> int:
     """int(voxel_num * mask_scale) with the product rounded to float32, as the reference computes it."""
     f32 = ctypes.c_float  # the product of two FP32 values is exact in double, so this rounds once
-    return int(f32(f32(voxel_num).value * f32(mask_scale).value).value)
+    return int(f32(f32(float(voxel_num)).value * f32(float(mask_scale)).value).value)
 
 
 def _check_mask(mask: torch.Tensor, voxel_num: float, mask_scale: float) -> torch.Tensor:
