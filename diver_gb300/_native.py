@@ -138,6 +138,30 @@ def stream(device: torch.device | str | int | None = None) -> int:
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
+class LastWrite:
+    """Puts the readers of a buffer that is kept from call to call behind its last
+    write, whatever streams the two run on: done() after the write's launches,
+    wait() before a reader's, both on the current stream of `device`.  While that
+    stream is being captured neither does anything: no event crosses a capture's
+    boundary, torch.cuda.graph starts one on a device that is idle, and what a
+    graph writes itself it orders itself."""
+
+    __slots__ = ("event",)
+
+    def __init__(self):
+        self.event = None
+
+    def done(self, device: torch.device) -> None:
+        if not torch.cuda.is_current_stream_capturing():
+            event = torch.cuda.Event()  # a new one: a wait on the last one may be queued at this moment
+            event.record(torch.cuda.current_stream(device))
+            self.event = event
+
+    def wait(self, device: torch.device) -> None:
+        if self.event is not None and not torch.cuda.is_current_stream_capturing():
+            torch.cuda.current_stream(device).wait_event(self.event)
+
+
 def need_cuda(name: str, t: torch.Tensor, dtype: torch.dtype | None = None) -> None:
     if not isinstance(t, torch.Tensor):
         raise TypeError(f"{name} must be a torch.Tensor")

@@ -126,6 +126,7 @@ class TcWeights:
             if self.terms > 1:
                 self._folded = torch.zeros(plain_size(kind, channels) + WIDTH[KIND_ID[kind]] ** 2, device=device)
         self.version = None
+        self.written = N.LastWrite()  # of the images
 
     @staticmethod
     def from_decoder(decoder: Decoder, device, bf16: bool = True, mode: str | None = None) -> "TcWeights":
@@ -150,6 +151,7 @@ class TcWeights:
             p = self._folded
         if self.bwd is not None:
             self._fill(self.bwd[0], self._i_bwd, p, form)
+        self.written.done(p.device)
 
     def save_buffer(self, kind: int, channels: int, n_seg: int, device) -> torch.Tensor | None:
         """Buffer for the forward's layer inputs, read back by the tensor-core
@@ -191,6 +193,7 @@ class TcWeights:
 
     def decode(self, kind, channels, voxels, seg, pe_out, out4, st, voxels16=None, save=None):
         nx, ny, nz, c = _grid(voxels)
+        self.written.wait(voxels.device)  # a refresh may have run on another stream than this call's
         if self.terms > 1:
             # a save record (save_buffer gives one where there is a backward to read it) is the folded backward's
             _timed("dv_decode_fwd_tc_split" if save is None else "dv_decode_fwd_tc_folded", kind, c,
@@ -387,10 +390,11 @@ class DIVeRField(torch.nn.Module):
             return None
         tw = self._tc.get(form)
         if tw is None:
-            tw = self._tc[form] = TcWeights(self.kind, self.voxels.shape[-1], self.voxels.device, mode=form)
+            tw = TcWeights(self.kind, self.voxels.shape[-1], self.voxels.device, mode=form)
         if self.refresh_always or tw.version != self.params._version:
             tw.refresh(self.params)
             tw.version = self.params._version
+        self._tc[form] = tw  # other threads find it with its images queued and their event set
         return tw
 
     def _refreshes(self, form: str) -> bool:

@@ -1,0 +1,53 @@
+"""GPU: one field or model used from several streams.  What a call keeps for the
+next ones is written on the stream (or side stream) of the call that needed it
+first; a call on another stream that finds it must wait for that write.  The
+write is held back for about a tenth of a second by torch's bounded spin, so an
+unordered reader would read what was there before."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+HOLD = 200_000_000  # clocks
+
+
+def rays(n, seed=3):
+    from diver_gb300 import scenes
+
+    c2w = scenes.sphere_cameras(1, 4.0, seed)[0]
+    o, d = scenes.camera_rays(c2w, 40, 40, 50.0, "cuda")
+    return o[:n].contiguous(), d[:n].contiguous()
+
+
+def small_field():
+    from diver_gb300 import scenes
+    from diver_gb300.renderer import DIVeRField
+
+    return DIVeRField.from_scene(scenes.small_scene("cpu"), "cuda")
+
+
+@pytest.mark.parametrize("form", ["bf16", "fp16", "bf16s"])
+@pytest.mark.parametrize("grad", [False, True])
+@pytest.mark.parametrize("capacity", [False, True])
+def test_images_refreshed_on_another_stream(form, grad, capacity):
+    """The first call after a change of the decoder refreshes its images on the
+    field's side stream; a second one, on another stream and small enough to
+    stay on it, decodes with the new images."""
+    field, want = small_field(), small_field()
+    o, d = rays(1500)
+    cap = field.segment_capacity(o.shape[0]) if capacity else None
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.set_grad_enabled(grad):
+        field(o, d, form=form, capacity=cap)  # images of the first decoder
+        with torch.no_grad():
+            for f in (field, want):
+                f.params.mul_(0.5)
+        ref = want(o, d, form=form, capacity=cap)[0].detach()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(field._side_stream(field.voxels.device)):
+            torch.cuda._sleep(HOLD)
+        got = []
+        for s in (a, b):
+            with torch.cuda.stream(s):
+                got.append(field(o, d, form=form, capacity=cap)[0].detach())
+    torch.cuda.synchronize()
+    assert torch.equal(got[0], ref) and torch.equal(got[1], ref)
