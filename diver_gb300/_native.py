@@ -151,6 +151,9 @@ class LastWrite:
     def __init__(self):
         self.event = None
 
+    def __reduce__(self):
+        return LastWrite, ()  # a copied or loaded buffer has been written by other work than this one's
+
     def done(self, device: torch.device) -> None:
         if not torch.cuda.is_current_stream_capturing():
             event = torch.cuda.Event()  # a new one: a wait on the last one may be queued at this moment

@@ -443,11 +443,14 @@ class DIVeRField(torch.nn.Module):
         if form in ("fp32", "bf16s"):
             return None
         key = ("grid16", form, self.voxels._version)
-        if getattr(self, "_g16key", None) != key:
+        kept = getattr(self, "_g16", None)
+        if kept is None or kept[0] != key:
             dt = torch.bfloat16 if form == "bf16" else torch.float16
-            self._g16 = self.voxels.detach().to(dt).contiguous()
-            self._g16key = key
-        return self._g16
+            copy, written = self.voxels.detach().to(dt).contiguous(), N.LastWrite()
+            written.done(copy.device)
+            kept = self._g16 = (key, copy, written)  # one object: another thread sees all of it
+        kept[2].wait(kept[1].device)  # the copy may have been made on another stream than this call's
+        return kept[1]
 
     @torch.no_grad()
     def accumulate_alpha(self, os: torch.Tensor, ds: torch.Tensor, alpha_map: torch.Tensor, pad: int = 0,

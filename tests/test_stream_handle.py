@@ -35,3 +35,13 @@ def test_device_rays_refuse_a_host_device(monkeypatch):
     monkeypatch.setattr(N, "call", call)
     with pytest.raises(ValueError, match="cuda device"):
         scenes.camera_rays_device(torch.eye(3, 4), 4, 4, 5.0, device="cpu")
+
+
+def test_last_write_is_not_copied():
+    """A field's copy (copy.deepcopy) holds no event of the original's."""
+    import copy
+    import pickle
+
+    w = N.LastWrite()
+    w.event = object()
+    assert copy.deepcopy(w).event is None and pickle.loads(pickle.dumps(w)).event is None

@@ -51,3 +51,26 @@ def test_images_refreshed_on_another_stream(form, grad, capacity):
                 got.append(field(o, d, form=form, capacity=cap)[0].detach())
     torch.cuda.synchronize()
     assert torch.equal(got[0], ref) and torch.equal(got[1], ref)
+
+
+@pytest.mark.parametrize("form", ["bf16", "fp16"])
+def test_grid_copy_made_on_another_stream(form):
+    """A render on another stream than the one that makes the 16-bit copy of the grid."""
+    field, want = small_field(), small_field()
+    o, d = rays(1500)
+    cap = field.segment_capacity(o.shape[0])
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.no_grad():
+        field(o, d, form=form, capacity=cap)
+        for f in (field, want):
+            f.voxels.mul_(0.5)
+        ref = want(o, d, form=form, capacity=cap)[0]
+        torch.cuda.synchronize()
+        got = []
+        for s in (a, b):
+            with torch.cuda.stream(s):
+                if s is a:
+                    torch.cuda._sleep(HOLD)
+                got.append(field(o, d, form=form, capacity=cap)[0])
+    torch.cuda.synchronize()
+    assert torch.equal(got[0], ref) and torch.equal(got[1], ref)
