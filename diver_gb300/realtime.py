@@ -89,13 +89,17 @@ class RealtimeModel:
     def tc_blob(self) -> torch.Tensor:
         """Tensor-core images of the folded layers (three BF16 terms), made once
         per model from the aligned params on the device."""
-        blob = getattr(self, "_tc_blob", None)
+        blob, written = getattr(self, "_tc_blob", None), getattr(self, "_tc_written", None)
+        dev = self.packed.device
         if blob is None:
-            dev = self.packed.device
             blob = torch.empty(N.lib().dv_realtime_tc_bytes(self.width), dtype=torch.uint8, device=dev)
             N.call("dv_realtime_tc_pack", self.width, N.ptr(self.packed), N.ptr(blob), N.stream(dev))
-            self._tc_blob = blob
             self.tc_err = torch.zeros(1, dtype=torch.int32, device=dev)
+            written = self._tc_written = N.LastWrite()
+            written.done(dev)
+            self._tc_blob = blob  # last: another thread finds the rest with it
+        if written is not None:  # None: loaded, finished
+            written.wait(dev)  # the images may have been made on another stream than this call's
         return blob
 
     def mlp_eval(self, rgba, coords, v, finish, tensor_cores: bool = False):

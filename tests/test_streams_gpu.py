@@ -74,3 +74,28 @@ def test_grid_copy_made_on_another_stream(form):
                 got.append(field(o, d, form=form, capacity=cap)[0])
     torch.cuda.synchronize()
     assert torch.equal(got[0], ref) and torch.equal(got[1], ref)
+
+
+def realtime_model():
+    from tests.test_realtime import small_realtime
+
+    return small_realtime("diver32", "cuda", bias=0.2)[2]
+
+
+def test_realtime_images_made_on_another_stream():
+    """A frame on another stream than the one that makes the model's tensor-core images."""
+    from diver_gb300 import scenes
+
+    c2w = scenes.sphere_cameras(1, 4.0, 3)[0]
+    _, v = scenes.camera_rays(c2w, 40, 40, 50.0, "cuda")
+    want = realtime_model().render_frame(c2w[:, 3], v)[0]
+    model = realtime_model()
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(a):
+        torch.cuda._sleep(HOLD)
+        model.tc_blob()
+    with torch.cuda.stream(b):
+        got = model.render_frame(c2w[:, 3], v)[0]
+    torch.cuda.synchronize()
+    assert torch.equal(got, want) and int(model.tc_err.item()) == 0
