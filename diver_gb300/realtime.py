@@ -184,9 +184,10 @@ class RealtimeModel:
         st = N.stream(dev)
         N.call("dv_realtime_begin", B, N.ptr(v), N.ptr(center), N.ptr(o8), n, N.ptr(resume), N.ptr(rgba),
                N.ptr(lists[0]), N.ptr(counts), st)
-        if getattr(self, "_flags", None) is None:
-            self._flags = (torch.zeros(2, dtype=torch.int32, pin_memory=True), [torch.cuda.Event(), torch.cuda.Event()])
-        left, events = self._flags
+        # of this call alone: its last round's copy is still under way when it returns, and another
+        # frame of the model, on another stream or thread, waits for its own (torch's pinned pool
+        # holds a freed buffer back until the copies into it have run)
+        left, events = torch.zeros(2, dtype=torch.int32, pin_memory=True), (torch.cuda.Event(), torch.cuda.Event())
         while rounds < limit:
             live, after = lists[rounds % 2], lists[1 - rounds % 2]
             count = counts.data_ptr() + 4 * rounds

@@ -99,3 +99,41 @@ def test_realtime_images_made_on_another_stream():
         got = model.render_frame(c2w[:, 3], v)[0]
     torch.cuda.synchronize()
     assert torch.equal(got, want) and int(model.tc_err.item()) == 0
+
+
+def test_frames_of_one_model_on_several_threads():
+    """Each thread renders its own view on its own stream; a frame's round counts
+    come back to that frame alone, so every one equals the frame rendered by
+    itself.  Frames one after the other on two streams share nothing either."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    from diver_gb300 import scenes
+
+    model = realtime_model()
+    eyes, dirs, want = [], [], []
+    for seed in range(4):
+        c2w = scenes.sphere_cameras(1, 4.0, seed)[0]
+        eyes.append(c2w[:, 3])
+        dirs.append(scenes.camera_rays(c2w, 20 * (seed + 1), 30, 45.0, "cuda")[1])
+        want.append(model.render_frame(eyes[-1], dirs[-1])[0])
+    torch.cuda.synchronize()
+
+    def frames(i):
+        s, out = torch.cuda.Stream(), []
+        with torch.cuda.stream(s):
+            for _ in range(10):
+                out.append(model.render_frame(eyes[i], dirs[i])[0])
+        s.synchronize()
+        return out
+
+    with ThreadPoolExecutor(4) as pool:
+        for i, out in enumerate(pool.map(frames, range(4))):
+            assert all(torch.equal(x, want[i]) for x in out)
+    streams, got = [torch.cuda.Stream() for _ in range(2)], []
+    for k in range(20):
+        with torch.cuda.stream(streams[k % 2]):
+            got.append(model.render_frame(eyes[k % 4], dirs[k % 4])[0])
+    torch.cuda.synchronize()
+    assert all(torch.equal(x, want[k % 4]) for k, x in enumerate(got))
+    held = [k for k, x in vars(model).items() if isinstance(x, torch.Tensor) and x.is_pinned()]
+    assert not held and int(model.tc_err.item()) == 0
