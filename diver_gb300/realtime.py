@@ -18,6 +18,8 @@ here DIVeR64 over 32 channels packs to the layout its kernel reads
 """
 from __future__ import annotations
 
+import math
+
 import torch
 
 from . import _native as N
@@ -175,7 +177,7 @@ class RealtimeModel:
         rgba = torch.empty(B, 4, device=dev)
         if B == 0:
             return rgba[:, :3] + rgba[:, 3:], 0
-        limit = max(0, min(limit, 3 * n + 4))  # a round takes at least one grid plane per live pixel
+        limit = max(0, math.ceil(min(limit, 3 * n + 4)))  # a round takes at least one grid plane per live pixel
         hits = torch.empty(8, B, 6, device=dev)
         resume = torch.empty(B, 3, device=dev)
         lists = torch.empty(2, B, dtype=torch.int32, device=dev)

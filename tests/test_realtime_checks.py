@@ -43,3 +43,10 @@ def test_frame_refuses_directions_of_another_shape(model, shape):
 def test_frame_takes_one_direction_per_ray(model, shape):
     with pytest.raises(Launched, match="dv_realtime_begin"):
         model.render_frame(EYE, torch.ones(shape))
+
+
+@pytest.mark.parametrize("rounds", [0, 1, 2.0, 2.5, 1e9, float("inf"), torch.tensor(3), -1, True])
+def test_frame_takes_any_number_of_rounds(model, rounds):
+    """max_rounds is compared with the rounds done, so any number will do."""
+    with pytest.raises(Launched, match="dv_realtime_begin"):
+        model.render_frame(EYE, torch.ones(5, 3), max_rounds=rounds)
