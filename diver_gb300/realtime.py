@@ -141,7 +141,11 @@ class RealtimeModel:
         B = dirs.shape[0]
         v = dirs.contiguous()
         center = ((eye.float().cpu() - self.xyzmin) / self.voxel_size).to(dev).contiguous()
+        if center.numel() < 3:
+            raise ValueError(f"eye must hold 3 coordinates, got {tuple(eye.shape)}")
         if mode == "fused":
+            if v.numel() * v.element_size() < 12 * B:  # the kernel reads three floats at v + 3 b
+                raise ValueError(f"dirs must hold one (x, y, z) in FP32 per ray, [B, 3], got {tuple(v.shape)} {v.dtype}")
             rgba = torch.empty(B, 4, device=dev)
             m8 = self.voxel_masks.view(torch.uint8) if self.voxel_masks.dtype == torch.bool else self.voxel_masks
             o8 = self.octrees.view(torch.uint8) if self.octrees.dtype == torch.bool else self.octrees

@@ -50,3 +50,22 @@ def test_frame_takes_any_number_of_rounds(model, rounds):
     """max_rounds is compared with the rounds done, so any number will do."""
     with pytest.raises(Launched, match="dv_realtime_begin"):
         model.render_frame(EYE, torch.ones(5, 3), max_rounds=rounds)
+
+
+@pytest.mark.parametrize("mode", ["tc", "fused", "loop"])
+@pytest.mark.parametrize("eye,shape", [((3,), (5, 2)), ((3,), (6,)), ((2,), (5, 3)), ((0,), (5, 3))])
+def test_no_mode_reads_past_its_inputs(model, mode, eye, shape):
+    """A camera centre or directions with less than the kernels read, in any mode."""
+    with pytest.raises(ValueError, match="eye|dirs|v must"):
+        model.render_frame(torch.ones(eye), torch.ones(shape), mode=mode)
+
+
+def test_one_launch_frame_refuses_short_types(model):
+    with pytest.raises(ValueError, match="dirs"):
+        model.render_frame(EYE, torch.ones(5, 3, dtype=torch.float16), mode="fused")
+
+
+@pytest.mark.parametrize("shape", [(5, 3), (4, 5, 3), (5, 1, 3)])  # (rays in the first dimension)
+def test_one_launch_frame_takes_what_it_took(model, shape):
+    with pytest.raises(Launched, match="dv_realtime_frame"):
+        model.render_frame(EYE, torch.ones(shape), mode="fused")
