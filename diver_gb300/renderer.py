@@ -2,8 +2,9 @@
 
 `render_segments` is a torch.autograd.Function over the CUDA pipeline:
   forward   dv_ray_pe, dv_decode_fwd, dv_composite_fwd
-  backward  dv_composite_bwd, dv_decode_bwd (recomputes each segment's decode
-            instead of storing activations; grid gradient by vector atomics)
+  backward  dv_composite_bwd, dv_decode_bwd_saved (reads the activations that
+            dv_decode_fwd_save kept; dv_decode_bwd recomputes them where they
+            were not: see PLAIN_SAVE; grid gradient by vector atomics)
 It returns per-ray rgb and the reference's sparsity term
 mean(log(1 + sigma^2 / 0.5)) over the padded [B, M] sigma (train.py:84-85),
 so `mse(rgb, target) + l_s * reg` is the reference's training loss
@@ -15,6 +16,9 @@ reference's DIVeR module does (model/diver.py:16-207) for callers that want a
 module.
 """
 from __future__ import annotations
+
+import threading
+import weakref
 
 import torch
 from torch.autograd import Function
@@ -68,20 +72,46 @@ def _check_params(kind: int, channels: int, params: torch.Tensor):
 FORMS = ("fp32", "bf16", "fp16", "bf16s")
 
 
-# Bytes up to which the plain FP32 form keeps its activations for the backward
-# (576 B a segment of DIVeR32, 864 of DIVeR64 over 64 channels).  Larger lists recompute them, and their
-# memory stays at the 60 B a segment of the lists and outputs.
+# Bytes of activations that plain FP32 forwards keep for backwards yet to run, all
+# together on a device (576 B a segment of DIVeR32, 864 of DIVeR64 over 64
+# channels; a list of fixed capacity counts by its capacity, 1.8 GB for 4096 rays
+# of a 256^3 grid).  A forward beyond that leaves its backward to recompute, with
+# the 60 B a segment of the lists and outputs.
 PLAIN_SAVE = 2 << 30
 
 
-def _plain_save(kind: int, channels: int, n_seg: int, device) -> torch.Tensor | None:
+class PlainRecord:
+    """A forward's activations; counted for as long as the object lives, which is
+    until its backward has read it (SegmentRender)."""
+
+    __slots__ = ("data", "__weakref__")
+
+    def __init__(self, data: torch.Tensor):
+        self.data = data
+
+
+_records = weakref.WeakSet()
+_records_lock = threading.Lock()
+
+
+def _plain_save(kind: int, channels: int, n_seg: int, device: torch.device) -> PlainRecord | None:
+    """Room for n_seg segments' activations, or None: recompute."""
     n = int(N.lib().dv_decode_save_bytes(kind, channels, n_seg))
     if not 0 < n <= PLAIN_SAVE:
         return None
-    try:
-        return torch.empty(n, dtype=torch.uint8, device=device)
-    except torch.cuda.OutOfMemoryError:  # the recomputing backward needs no record
+    # A graph keeps its record's memory for good, and cannot make up for an
+    # allocation that fails: it takes no more than an eighth of what is free.
+    if torch.cuda.is_current_stream_capturing() and 8 * n > torch.cuda.mem_get_info(device)[0]:
         return None
+    with _records_lock:
+        if sum(r.data.numel() for r in list(_records) if r.data.device == device) + n > PLAIN_SAVE:
+            return None
+        try:
+            record = PlainRecord(torch.empty(n, dtype=torch.uint8, device=device))
+        except torch.cuda.OutOfMemoryError:
+            return None
+        _records.add(record)
+    return record
 
 
 # Rays up to which their directions' encoding runs on the calling stream (8 us
@@ -227,28 +257,29 @@ class SegmentRender(Function):
             pe_feat, pe_out = pe
         S = seg.total
         out4 = torch.empty(S, 4, device=dev)
+        rgb = torch.empty(B, 3, device=dev)
+        reg = torch.empty(B, device=dev)
+        reg_mean = torch.empty((), device=dev)
+        inv_m = torch.empty(1, device=dev)
+        ctx.record = ctx.saved_layers = None
         if tc is None:
-            save = _plain_save(kind, c, S, dev) if training else None
+            # last of the allocations: what it takes is missing nowhere in here
+            ctx.record = record = _plain_save(kind, c, S, dev) if training else None
             args = (kind, c, N.ptr(params), N.ptr(voxels), nx, ny, nz, N.ptr(seg.seg), N.ptr(seg.ray), S, seg.count_ptr,
                     N.ptr(pe_out), N.ptr(out4))
-            if save is None:
+            if record is None:
                 _timed("dv_decode_fwd", *args, st)
             else:
-                _timed("dv_decode_fwd_save", *args, N.ptr(save), save.numel(), st)
-            ctx.saved_layers = save
+                _timed("dv_decode_fwd_save", *args, N.ptr(record.data), record.data.numel(), st)
         else:
             # training: keep the layer inputs for the tensor-core backward
             save = tc.save_buffer(kind, c, S, dev) if training else None
             tc.decode(kind, c, voxels, seg, pe_out, out4, st, voxels16, save)
             ctx.saved_layers = save
-        rgb = torch.empty(B, 3, device=dev)
-        reg = torch.empty(B, device=dev)
         _timed("dv_composite_fwd", B, N.ptr(seg.offsets), N.ptr(out4), int(bool(white_back)), N.ptr(rgb), None,
                N.ptr(reg), st)
         # mean over the padded [B, M]; M (max segments per ray) stays on the
         # device when the segments were built without a host read
-        reg_mean = torch.empty((), device=dev)
-        inv_m = torch.empty(1, device=dev)
         on_dev = seg.max_count is None
         _timed("dv_reg_mean", B, N.ptr(reg), N.ptr(seg.max_dev) if on_dev else None,
                0.0 if on_dev else float(seg.max_count), N.ptr(reg_mean), N.ptr(inv_m), st)
@@ -270,7 +301,18 @@ class SegmentRender(Function):
         scale = None
         if g_reg is not None:
             scale = (g_reg.detach().float().reshape(1) * ctx.inv_m).contiguous()
-        d4 = torch.empty_like(out4)
+
+        def room(make, like):
+            """make(like); where the device is full, without the plain form's record."""
+            try:
+                return make(like)
+            except torch.cuda.OutOfMemoryError:
+                if ctx.record is None:
+                    raise
+                ctx.record = None
+                return make(like)
+
+        d4 = room(torch.empty_like, out4)
         _timed("dv_composite_bwd", B, N.ptr(seg.offsets), N.ptr(out4), N.ptr(rgb), N.ptr(g_rgb),
                1.0 / B if scale is not None else 0.0, N.ptr(scale), N.ptr(d4), st)
         if ctx.grad_voxels is not None:
@@ -281,20 +323,21 @@ class SegmentRender(Function):
             touched = touched[0] if touched else None
             torch.cuda.current_stream(dev).wait_event(filled)
         else:
-            gv, touched = torch.zeros_like(voxels), None
-        saved = getattr(ctx, "saved_layers", None)
+            gv, touched = room(torch.zeros_like, voxels), None
+        saved = ctx.saved_layers
         # the split tensor-core backward sets the row marks in its scatter
         if touched is not None and not (ctx.tc is not None and ctx.tc.marks_rows(saved)):
             N.call("dv_mark_corner_rows", N.ptr(seg.seg), seg.total, seg.count_ptr, nx, ny, nz, N.ptr(touched), st)
             touched = None
-        gp = torch.zeros_like(params)
+        gp = room(torch.zeros_like, params)
         if ctx.tc is not None and ctx.tc.backward(ctx.kind, voxels, seg, pe_feat, pe_out, d4, gv, gp, st, saved, out4,
                                                   touched):
             return gv, gp, None, None, None, None, None, None, None, None, None
         args = (ctx.kind, c, N.ptr(params), N.ptr(voxels), nx, ny, nz, N.ptr(seg.seg), N.ptr(seg.ray), seg.total,
                 seg.count_ptr, N.ptr(pe_feat), N.ptr(pe_out), N.ptr(d4), N.ptr(gv), N.ptr(gp))
-        if ctx.tc is None and saved is not None:
-            _timed("dv_decode_bwd_saved", *args, N.ptr(saved), saved.numel(), st)
+        record, ctx.record = ctx.record, None  # given back: a second backward of a retained graph recomputes
+        if record is not None:
+            _timed("dv_decode_bwd_saved", *args, N.ptr(record.data), record.data.numel(), st)
         else:
             _timed("dv_decode_bwd", *args, st)
         return gv, gp, None, None, None, None, None, None, None, None, None
