@@ -469,7 +469,9 @@ DV_API int dv_decode_bwd_tc_split(int kind, int channels, const void* wb, int wb
 /*
  * dv_decode_bwd_tc_split with mlp1's output layer and mlp2's first layer taken
  * as one matrix (no activation lies between them): a fifth less work, the same
- * gradients to FP32 rounding.  folded: dv_fold_params of the parameters, the
+ * gradients to FP32 rounding, but for that of mlp2's first layer where the
+ * hidden layer is far smaller than its own product and bias (26 times: 1.7e-4
+ * relative against 9e-6 of dv_decode_bwd_tc_split).  folded: dv_fold_params of the parameters, the
  * packed parameters followed by WF [in][out], the product of the two layers.
  * wb / b_layers: the transposed images of four layers (mlp1's first two;
  * [sigma | WF | zeros to 48]; mlp2's output), three terms each.  The rest as
