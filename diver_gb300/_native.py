@@ -141,15 +141,24 @@ def stream(device: torch.device | str | int | None = None) -> int:
 class LastWrite:
     """Puts the readers of a buffer that is kept from call to call behind its last
     write, whatever streams the two run on: done() after the write's launches,
-    wait() before a reader's, both on the current stream of `device`.  While that
-    stream is being captured neither does anything: no event crosses a capture's
-    boundary, torch.cuda.graph starts one on a device that is idle, and what a
-    graph writes itself it orders itself."""
+    wait() before a reader's, both on the current stream of `device`.
 
-    __slots__ = ("event",)
+    A stream waits for a write's event once (a wait costs a small call 7 to 10 us,
+    also on an event long past) and is in `behind` from then on, by its handle.  A
+    handle cannot come back for another stream before the write has run: a
+    destroyed stream's handle goes when the stream's work is done, which the
+    write, or the wait for it, is part of.  (The per-thread default stream's
+    handle stands for many streams and is never put there.)
+
+    While the current stream is being captured nothing is recorded or waited for:
+    no event crosses a capture's boundary, torch.cuda.graph starts one on a device
+    that is idle, and what a graph writes itself it orders itself."""
+
+    __slots__ = ("state",)
+    PER_THREAD = 2  # cudaStreamPerThread
 
     def __init__(self):
-        self.event = None
+        self.state = (None, set())  # event of the last write, handles of the streams behind it
 
     def __reduce__(self):
         return LastWrite, ()  # a copied or loaded buffer has been written by other work than this one's
@@ -158,11 +167,25 @@ class LastWrite:
         if not torch.cuda.is_current_stream_capturing():
             event = torch.cuda.Event()  # a new one: a wait on the last one may be queued at this moment
             event.record(torch.cuda.current_stream(device))
-            self.event = event
+            self.state = (event, {stream(device)} - {self.PER_THREAD})
 
     def wait(self, device: torch.device) -> None:
-        if self.event is not None and not torch.cuda.is_current_stream_capturing():
-            torch.cuda.current_stream(device).wait_event(self.event)
+        event, behind = self.state
+        if event is None:
+            return
+        handle = stream(device)
+        if handle in behind or torch.cuda.is_current_stream_capturing():
+            return
+        torch.cuda.current_stream(device).wait_event(event)
+        if handle != self.PER_THREAD:
+            behind.add(handle)
+
+    def join(self, main: torch.cuda.Stream, side: torch.cuda.Stream) -> None:
+        """main.wait_stream(side), which puts main behind the write where side is."""
+        behind = self.state[1]  # of the write that the wait covers
+        main.wait_stream(side)
+        if side.cuda_stream in behind and main.cuda_stream != self.PER_THREAD:
+            behind.add(main.cuda_stream)
 
 
 def need_cuda(name: str, t: torch.Tensor, dtype: torch.dtype | None = None) -> None:

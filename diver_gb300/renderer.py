@@ -562,7 +562,10 @@ class DIVeRField(torch.nn.Module):
             with torch.cuda.stream(side):
                 tc = prepare()
             seg = segments if segments is not None else self.segments(os, ds, capacity)
-            main.wait_stream(side)
+            if tc is None:
+                main.wait_stream(side)
+            else:
+                tc.written.join(main, side)
         g16 = self.grid16(form) if not torch.is_grad_enabled() else None
         return render_segments(self.voxels, self.params, seg, ds, self.kind, self.white_back, tc, g16, grad_voxels,
                                pe)
