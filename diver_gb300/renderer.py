@@ -104,7 +104,7 @@ def _plain_save(kind: int, channels: int, n_seg: int, device: torch.device) -> P
     if torch.cuda.is_current_stream_capturing() and 8 * n > torch.cuda.mem_get_info(device)[0]:
         return None
     with _records_lock:
-        if sum(r.data.numel() for r in list(_records) if r.data.device == device) + n > PLAIN_SAVE:
+        if len(_records) and sum(r.data.numel() for r in list(_records) if r.data.device == device) + n > PLAIN_SAVE:
             return None
         try:
             record = PlainRecord(torch.empty(n, dtype=torch.uint8, device=device))
