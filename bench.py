@@ -76,15 +76,6 @@ def alg_work(kernel, S, U, R):
     return 0, 0
 
 
-# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per segment of the
-# decode kernels in the captured 4096-ray training step, from ncu captures of
-# `python bench.py --profile train --form <form>`: the single-term BF16 kernels
-# on the 256^3 grid, the split-operand forward on the 128^3 grid of the same
-# scene family (557,787 segments; its traffic is per-segment: the rays'
-# segments, the corner rows and the saved record); the roofline's `traffic`
-# is this times the segments of a launch.  The split backward has no entry:
-# its current form has no ncu section capture (the roofline reports null).
-TRAFFIC_PER_SEG = {"dv_decode_bwd_tc": 1302.35, "dv_decode_fwd_tc": 810.52, "dv_decode_fwd_tc_split": 997.2}
 # Kernels of this library per captured training step: row clear, weight image
 # gathers (forward, biases, backward; the split form's after the folded
 # product), ray PE, slot walk, 3 scan kernels, slot compaction, decoder
@@ -462,7 +453,7 @@ def run_ours(args, rank, world, local):
                     "unit": "TFLOP/s", "frac": flops / sec / 1e12 / tensor,
                     "peak_source": "MEASURED_PEAKS.json bf16_tflops_sustained (of measured)" if peaks else "fallback"}
     roofline.update({
-        "traffic": TRAFFIC_PER_SEG[dom] * S_mean if dom in TRAFFIC_PER_SEG else None,
+        "traffic": None,  # no DRAM-byte capture of the present kernels
         "algorithmic_bytes": nbytes, "algorithmic_flops": flops,
         "tensor_frac": flops / sec / 1e12 / tensor, "hbm_frac": nbytes / sec / 1e9 / hbm,
         "avg_launch_ms": avg_ms, "segments_per_launch": S_mean, "corner_rows_per_launch": U_mean,
