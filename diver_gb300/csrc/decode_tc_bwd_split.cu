@@ -52,7 +52,8 @@
 // Shared memory (at most 226 KiB): the propagation images, the saved record in
 // per-layer slots, the PE tile, two delta tiles, a tile of ones, the FP32
 // staging rows of the feature gradient and the scatter's corners.  TMEM: all 512
-// columns (64 working, 384 weight-gradient and 64 bias-gradient columns).
+// columns are allocated (64 working; folded 320 weight-gradient and 48
+// bias-gradient columns, layer by layer 384 and 64: Cfg::DWCOL, Cfg::DBCOL).
 // Measured, captured 4096-ray step of the 256^3 scene (1.26 M segments): 733 us
 // with the chain doing the scatter in its waits and every MMA of a layer ahead
 // of its epilogue, 625 us in this form with one thread issuing and stepping
@@ -444,7 +445,8 @@ __device__ __forceinline__ void prop_row32(uint32_t taddr, float* v) {
 // the last stages the tile's feature gradient (FP32) for the scatter group
 // (folded: in one of two staging tiles, so neither group waits for the other's
 // slow tile; and the group's segments come a tile ahead).
-// The saved record sits in five per-layer slots, each with its own mbarrier: a
+// The saved record sits in a slot per layer step (four folded, five layer by
+// layer), each with its own mbarrier: a
 // slot is refilled with the next input of that layer once the MMAs that read
 // it are done, so the loads run behind the steps in between.  What the chain
 // reads from global memory for the next tile (ray, PE row, the first delta's

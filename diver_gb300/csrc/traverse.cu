@@ -1069,8 +1069,10 @@ static int walk_block(int batch) { return batch < sm_count() * 256 ? 32 : 256; }
 
 static bool aligned_to(const void* p, uintptr_t n) { return ((uintptr_t)p % n) == 0; }
 
-// The segment writers store seg with 16-byte (masked) or 8-byte (dense)
-// vector stores and seg_t / seg_ray in 8-byte pairs.
+// What the segment lists' entry points take.  The walks need 8 bytes for seg
+// (8-byte stores) and 4 for the others; the entry points have asked for more
+// (masked lists: seg on 16 bytes; seg_t and seg_ray on 8) since their earlier
+// writers' vector stores, and go on refusing what they refused.
 static bool segment_buffers_aligned(const float* seg, const float* seg_t, const int* seg_ray, uintptr_t seg_align) {
   return aligned_to(seg, seg_align) && aligned_to(seg_t, 8) && aligned_to(seg_ray, 8);
 }

@@ -123,10 +123,11 @@ class RealtimeModel:
         """rgb [B,3] of B rays from camera centre `eye` (world) with unit
         directions `dirs` [B,3] (eval_rt.py:106-122); also returns the number of
         host rounds.  mode:
-          "tc"     (default) the reference's loop of aabb_intersect, then rounds
-                   of ray_march + the tensor-core decoder (FP32-grade) until every
-                   pixel is finished, each over the pixels still alive
-                   (dv_realtime_begin, dv_march_live, dv_mlp_eval_live)
+          "tc"     (default) the reference's loop with the tensor-core decoder
+                   (FP32-grade) over the pixels still alive: dv_realtime_begin,
+                   then rounds of dv_march_live + dv_mlp_eval_live until none is
+                   left; a pixel gets what aabb_intersect, ray_march and
+                   dv_mlp_eval_tc give it
           "fused"  the whole frame in one launch with the FP32 decoder
                    (dv_realtime_frame)
           "loop"   the reference's loop with the FP32 decoder (dv_mlp_eval);

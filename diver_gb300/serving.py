@@ -222,8 +222,9 @@ class GpuRenderer:
         """Launches one batch per scene ([(model, work), ...]), each on its scene's
         stream, in two passes: first every batch's rays and traversal count walk,
         then, scene by scene, the total's host read, the emission walk, decode and
-        compositing.  The count walks of all scenes run together, and the host reads a total only once its walk has had the time
-        of the others' launches.  Returns [(event, [(request, first, count)])]."""
+        compositing.  The count walks of all scenes run together, and the host reads
+        a total only once its walk has had the time of the others' launches.
+        Returns [(event, [(request, first, count)])]."""
         began = []
         for field_model, work in batches:
             dev = field_model.voxels.device
