@@ -421,24 +421,25 @@ class DIVeRField(torch.nn.Module):
         self._tc = {}
         self.refresh_always = False
 
-    def tc_weights(self, form: str) -> TcWeights | None:
+    def tc_weights(self, form: str, made: TcWeights | None = None) -> TcWeights | None:
         """Tensor-core weights for form 'bf16' / 'fp16' / 'bf16s' (None for
         'fp32'), refreshed on the device whenever the decoder parameters
         changed (or on every call while `refresh_always` is set, as inside a
         captured graph, so that each replay packs the parameters of that
-        moment)."""
+        moment).  made: what to fill where the field has none yet."""
         if form not in FORMS:
             raise ValueError(f"unknown decoder form {form!r} (one of {FORMS})")
         if form == "fp32":
             return None
-        tw = self._tc.get(form)
-        if tw is None:
-            tw = TcWeights(self.kind, self.voxels.shape[-1], self.voxels.device, mode=form)
+        tw = self._tc.get(form) or made or self._new_weights(form)
         if self.refresh_always or tw.version != self.params._version:
             tw.refresh(self.params)
             tw.version = self.params._version
         self._tc[form] = tw  # other threads find it with its images queued and their event set
         return tw
+
+    def _new_weights(self, form: str) -> TcWeights:
+        return TcWeights(self.kind, self.voxels.shape[-1], self.voxels.device, mode=form)
 
     def _refreshes(self, form: str) -> bool:
         """Whether tc_weights(form) would rebuild its images."""
@@ -539,8 +540,8 @@ class DIVeRField(torch.nn.Module):
         kind = KIND_ID[self.kind]
         pe = (torch.empty(ds.shape[0], 28, device=dev), torch.empty(ds.shape[0], WIDTH[kind], device=dev))
 
-        def prepare():
-            tc = self.tc_weights(form)
+        def prepare(made=None):
+            tc = self.tc_weights(form, made)
             if ds.shape[0]:
                 _check_params(kind, self.voxels.shape[-1], self.params)
                 _timed("dv_ray_pe", kind, self.voxels.shape[-1], N.ptr(self.params), ds.shape[0], N.ptr(ds),
@@ -555,12 +556,14 @@ class DIVeRField(torch.nn.Module):
             # the tensor-core weight images and the directions' encoding do not
             # depend on the segments: they run on a side stream beside the
             # traversal (the outputs are allocated on the calling stream, which
-            # waits for the side stream)
+            # waits for the side stream; new images too, so that their memory
+            # goes back, when the field goes, to the stream that decodes with them)
+            made = self._new_weights(form) if form in FORMS and form != "fp32" and form not in self._tc else None
             main = torch.cuda.current_stream(dev)
             side = self._side_stream(dev)
             side.wait_stream(main)
             with torch.cuda.stream(side):
-                tc = prepare()
+                tc = prepare(made)
             seg = segments if segments is not None else self.segments(os, ds, capacity)
             if tc is None:
                 main.wait_stream(side)

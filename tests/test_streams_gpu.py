@@ -139,3 +139,20 @@ def test_frames_of_one_model_on_several_threads():
     kept = [y for x in vars(model).values() for y in (x if isinstance(x, (tuple, list)) else [x])]
     assert not any(isinstance(y, torch.Tensor) and y.is_pinned() for y in kept)
     assert int(model.tc_err.item()) == 0
+
+
+@pytest.mark.parametrize("form", ["bf16", "fp16", "bf16s"])
+def test_images_belong_to_the_calling_stream(form):
+    """The refresh runs on the side stream, but the images' memory is the calling
+    stream's: freed there, it is used again behind the decode that read it."""
+    field = small_field()
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s), torch.no_grad():
+        field(*rays(1500), form=form)
+    torch.cuda.synchronize()
+    tw = field.tc_weights(form)
+    kept = [tw.blob, tw.bias, tw.err] + ([tw.bwd[0]] if tw.bwd else []) + ([tw._folded] if tw._folded is not None else [])
+    for t in kept:
+        owner = [g["stream"] for g in torch.cuda.memory_snapshot()
+                 if g["address"] <= t.data_ptr() < g["address"] + g["total_size"]]
+        assert owner == [s.cuda_stream]
