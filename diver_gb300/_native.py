@@ -126,15 +126,21 @@ def ptr(t: torch.Tensor | None) -> int | None:
     return None if t is None else t.data_ptr()
 
 
+_cuda_index: dict = {}  # CUDA device, or its name -> its index (None: the current device)
+
+
 def stream(device: torch.device | str | int | None = None) -> int:
     """The current stream's handle (a stream object per launch costs more than
     the launch); ValueError for another device than a CUDA one."""
     index = device
     if index is not None and not isinstance(index, int):  # a torch.device, or its name
-        d = index if isinstance(index, torch.device) else torch.device(index)
-        if d.type != "cuda":
-            raise ValueError(f"expected a cuda device, got {d}")
-        index = d.index
+        try:
+            index = _cuda_index[device]  # (reading a device's type makes a string every time)
+        except KeyError:
+            d = torch.device(device)
+            if d.type != "cuda":
+                raise ValueError(f"expected a cuda device, got {d}") from None
+            index = _cuda_index[device] = d.index
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
